@@ -172,12 +172,13 @@ __global__ void k_field64(const double4* __restrict__ pos, const int4* __restric
 }
 
 // Walk records for projection axis `axis`: positions and gradient permuted
-// cyclically, the neighbour links copied.  The FP64 record carries rho_A and
-// the gradient (the reference's field form); the FP32 record carries the four
-// vertex densities (the mixed walk's barycentric form of the same field).
+// cyclically.  The FP64 record carries rho_A, the gradient and the neighbour
+// links; the mixed walk's are one TetGeo32 per (tet, entry face) and, in
+// `link`, the three rotations of its links (walk32.cuh).
 __global__ void k_records(const double4* __restrict__ pos, const int4* __restrict__ rows,
                           const double* __restrict__ grad, int nt, int axis,
-                          TetRec64* __restrict__ r64, TetRot32* __restrict__ rot) {
+                          TetRec64* __restrict__ r64, TetGeo32* __restrict__ geo,
+                          uint4* __restrict__ link) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   const int4 v = rows[2 * (size_t)t];
@@ -201,33 +202,20 @@ __global__ void k_records(const double4* __restrict__ pos, const int4* __restric
     r.vid = v;
     r64[t] = r;
   }
-  if (rot) {
-    // the record of each neighbour as entered from this tet
-    const int nbo[4] = {nb.x, nb.y, nb.z, nb.w};
-    int nxt[4];
+  if (geo) {
     float zmin = (float)q[0][2], zmax = zmin;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      zmin = fminf(zmin, (float)q[s][2]);
-      zmax = fmaxf(zmax, (float)q[s][2]);
-      const int n = nbo[s];
-      if (n < 0) {
-        nxt[s] = -1;
-        continue;
-      }
-      const int4 m = rows[2 * (size_t)n + 1];
-      const int f = m.x == t ? 0 : (m.y == t ? 1 : (m.z == t ? 2 : (m.w == t ? 3 : -1)));
-      nxt[s] = f >= 0 ? 4 * n + f : INT_MIN;
-    }
     // extent of the projection, over the float coordinates the walk reads
     float lo[2] = {(float)q[0][0], (float)q[0][1]}, hi[2] = {lo[0], lo[1]};
 #pragma unroll
-    for (int s = 1; s < 4; ++s)
+    for (int s = 1; s < 4; ++s) {
+      zmin = fminf(zmin, (float)q[s][2]);
+      zmax = fmaxf(zmax, (float)q[s][2]);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         lo[c] = fminf(lo[c], (float)q[s][c]);
         hi[c] = fmaxf(hi[c], (float)q[s][c]);
       }
+    }
     const float ext = __fmul_ru(fmaxf(__fsub_ru(hi[0], lo[0]), __fsub_ru(hi[1], lo[1])), 1.0000010f);
     // Condition of the FP32 field value rho3 + grad . (p - v3) at a point p
     // of the tet: the magnitudes summed over the least vertex value, a bound
@@ -243,18 +231,53 @@ __global__ void k_records(const double4* __restrict__ pos, const int4* __restric
     }
     const double cond = (rmax + (fabs(g[0]) + fabs(g[1])) * (double)ext +
                          fabs(g[2]) * (double)(zmax - zmin)) / rmin;
-    const int fp64_field = (cond <= kFieldCond) ? 0 : (int)0x80000000u;  // also NaN, rmin = 0
+    const bool trusted = cond <= kFieldCond;  // false also for NaN and rmin = 0
 #pragma unroll
     for (int F = 0; F < 4; ++F) {
-      const int s0 = rot_slot(F, 0), s1 = rot_slot(F, 1), s2 = rot_slot(F, 2), s3 = rot_slot(F, 3);
-      TetRot32 r;
-      r.xy01 = make_float4((float)q[s0][0], (float)q[s0][1], (float)q[s1][0], (float)q[s1][1]);
-      r.xy23 = make_float4((float)q[s2][0], (float)q[s2][1], (float)q[s3][0], (float)q[s3][1]);
-      r.z = make_float4((float)q[s0][2], (float)q[s1][2], (float)q[s2][2], (float)q[s3][2]);
-      r.fld = make_float4((float)p[s3].w, (float)g[0], (float)g[1], (float)g[2]);
-      r.nb = make_int4(nxt[s0], nxt[s1], nxt[s2], __float_as_int(ext) | fp64_field);
-      rot[4 * (size_t)t + F] = r;
+      float4* o = reinterpret_cast<float4*>(geo + 4 * (size_t)t + F);
+      o[0] = make_float4((float)q[F][0], (float)q[F][1], (float)q[F][2], (float)p[F].w);
+      o[1] = make_float4((float)g[0], (float)g[1], (float)g[2], trusted ? ext : INFINITY);
     }
+  }
+  if (link) {
+    const int vid[4] = {v.x, v.y, v.z, v.w}, nbo[4] = {nb.x, nb.y, nb.z, nb.w};
+    uint4* o = link + 12 * (size_t)t;
+    uint32_t lk[4][3];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {  // exit through face m, into neighbour n
+      const int n = nbo[m];
+      int4 w = make_int4(-1, -1, -1, -1);
+      int f = -1;
+      if (n >= 0) {
+        w = rows[2 * (size_t)n];
+        const int4 b = rows[2 * (size_t)n + 1];
+        f = b.x == t ? 0 : (b.y == t ? 1 : (b.z == t ? 2 : (b.w == t ? 3 : -1)));
+      }
+      const int wid[4] = {w.x, w.y, w.z, w.w};
+      int ws[3];  // the neighbour's entry face in its listed order
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int sl = f >= 0 ? rot_slot(f, k) : 0;
+        ws[k] = sl == 0 ? wid[0] : (sl == 1 ? wid[1] : (sl == 2 ? wid[2] : wid[3]));
+      }
+#pragma unroll
+      for (int F = 0; F < 4; ++F) {  // entered through face F
+        if (F == m) continue;
+        const int k = rot_inv(F, m);  // record slot of the vertex left behind
+        const int u[3] = {vid[rot_slot(F, (k + 1) % 3)], vid[rot_slot(F, (k + 2) % 3)], vid[F]};
+        uint32_t L = n < 0 ? kLinkHull : kLinkGeneral;
+        if (f >= 0) {
+          const int r = link_rotation(u, ws);
+          if (r >= 0) L = 3u * (4u * (uint32_t)n + (uint32_t)f) + (uint32_t)r;
+        }
+        lk[F][k] = L;
+      }
+    }
+#pragma unroll
+    for (int F = 0; F < 4; ++F)
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+        o[3 * F + r] = make_uint4(lk[F][r], lk[F][(r + 1) % 3], lk[F][(r + 2) % 3], 0u);
   }
 }
 
@@ -581,13 +604,19 @@ dtfe_status_t mesh_field64(Mesh* m) {
   return DTFE_OK;
 }
 
+static void drop_mixed_records(AxisData& A, Mesh* m) {
+  dfree_async(A.geo32, 4 * (size_t)m->nt, m);
+  dfree_async(A.link32, 12 * (size_t)m->nt, m);
+}
+
 dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32) {
   if (axis < 0 || axis > 2) return set_error(DTFE_ERR_INVALID, "axis %d not in 0..2", axis);
   if (!m->grad) return set_error(DTFE_ERR_INVALID, "mesh_records before mesh_gradients");
   AxisData& A = m->ax[axis];
-  const bool need64 = want64 && !A.rec64, need32 = want32 && !A.rot32;
+  const bool need64 = want64 && !A.rec64, need32 = want32 && !A.geo32;
   if (!need64 && !need32) return DTFE_OK;
   // the mixed walk's records address 4*t + F in an int: up to 2^29 - 1 tets
+  const bool links = need32 && m->nt <= kMaxLinkedTets;
   if (need32 && m->nt >= (1 << 29))
     return set_error(DTFE_ERR_UNSUPPORTED, "mixed maps of %d tets (at most 2^29 - 1)", m->nt);
   // all or nothing: a record array that exists has been built; stream-ordered
@@ -595,11 +624,13 @@ dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32) {
   // device (the serving loop builds and drops them while maps run)
   dtfe_status_t st = DTFE_OK;
   if (need64) st = dmalloc_async(&A.rec64, m->nt, m);
-  if (st == DTFE_OK && need32) st = dmalloc_async(&A.rot32, 4 * (size_t)m->nt, m);
+  if (st == DTFE_OK && need32) st = dmalloc_async(&A.geo32, 4 * (size_t)m->nt, m);
+  if (st == DTFE_OK && links) st = dmalloc_async(&A.link32, 12 * (size_t)m->nt, m);
   if (st == DTFE_OK && m->nt) {
     k_records<<<grid_for(m->nt), kBlock, 0, m->stream>>>(m->pos, m->rows, m->grad, m->nt, axis,
                                                          need64 ? A.rec64 : nullptr,
-                                                         need32 ? A.rot32 : nullptr);
+                                                         need32 ? A.geo32 : nullptr,
+                                                         links ? A.link32 : nullptr);
     count_launch();
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
@@ -607,7 +638,7 @@ dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32) {
   }
   if (st != DTFE_OK) {
     if (need64) dfree_async(A.rec64, m->nt, m);
-    if (need32) dfree_async(A.rot32, 4 * (size_t)m->nt, m);
+    if (need32) drop_mixed_records(A, m);
     return st;
   }
   return DTFE_OK;
@@ -616,14 +647,14 @@ dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32) {
 size_t mesh_record_bytes(const Mesh& m, int axis) {
   const AxisData& A = m.ax[axis];
   const size_t nt = (size_t)m.nt;
-  return (A.rot32 ? 4 * sizeof(TetRot32) * nt : 0) + (A.rec64 ? sizeof(TetRec64) * nt : 0);
+  return (A.geo32 ? mixed_record_bytes(m.nt) : 0) + (A.rec64 ? sizeof(TetRec64) * nt : 0);
 }
 
 size_t mesh_missing_record_bytes(const Mesh& m, int axis, int precision) {
   const AxisData& A = m.ax[axis];
   const size_t nt = (size_t)m.nt;
   size_t b = 0;
-  if (precision == DTFE_MIXED && !A.rot32) b += 4 * sizeof(TetRot32) * nt;
+  if (precision == DTFE_MIXED && !A.geo32) b += mixed_record_bytes(m.nt);
   // the mixed walk reads FP64 records only when the coordinates are not floats
   const bool want64 = precision == DTFE_FP64 ||
                       (!m.fp32_exact && !(m.flags & DTFE_MESH_NO_FP64_REC));
@@ -636,7 +667,7 @@ size_t mesh_missing_record_bytes(const Mesh& m, int axis, int precision) {
 void mesh_drop_records(Mesh* m, int axis) {
   if (axis < 0 || axis > 2) return;
   dfree_async(m->ax[axis].rec64, m->nt, m);
-  dfree_async(m->ax[axis].rot32, 4 * (size_t)m->nt, m);
+  drop_mixed_records(m->ax[axis], m);
 }
 
 dtfe_status_t mesh_hull_mask(Mesh* m, int axis, uint32_t* host_mask_out, int* count_out) {
@@ -740,7 +771,7 @@ void mesh_free(Mesh* m) {
   // is then synchronised (the caller's own streams are done with the mesh)
   for (auto& A : m->ax) {
     dfree_async(A.rec64, m->nt, m);
-    dfree_async(A.rot32, 4 * (size_t)m->nt, m);
+    drop_mixed_records(A, m);
   }
   dfree_async(m->fld64, m->nt, m);
   dfree_async(m->pos, m->n, m);

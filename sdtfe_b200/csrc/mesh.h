@@ -54,7 +54,8 @@ struct AxisData {
   signed char* tri_face = nullptr;  // device, n_tri: the tet face (0..3) under each triangle
   // walk records in this axis' projected frame (built on demand, per precision)
   TetRec64* rec64 = nullptr;
-  TetRot32* rot32 = nullptr;  // 4 per tet (one per entry face): the mixed walk's records
+  TetGeo32* geo32 = nullptr;  // 4 per tet (one per entry face): the mixed walk's records
+  uint4* link32 = nullptr;    // 12 per tet: their links (none beyond kMaxLinkedTets)
 };
 
 struct Mesh {

@@ -433,7 +433,7 @@ dtfe_status_t launch_grid64(Mesh& m, int G, double box_len, const double center[
   WalkConf64 w{box_len, (dxy / 2.0) / kPerturbMax, seed, max_visits};
   SDTFE_CUDA(cudaMemsetAsync(m.stats, 0, sizeof(unsigned long long) * kStatCount, s));
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
-  k_grid64<<<grid_blocks(G), 128, 0, s>>>(A.rec64, A.tri, A.n_tri, G, dxy, offx, offy, offz,
+  k_grid64<<<grid_warps(G) / 4, 128, 0, s>>>(A.rec64, A.tri, A.n_tri, G, dxy, offx, offy, offz,
                                           box_len, (int)ss, w, 4 * A.n_tri + 64, d_grid, m.stats);
   count_launch();
   SDTFE_CUDA(cudaGetLastError());

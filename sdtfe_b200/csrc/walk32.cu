@@ -14,16 +14,16 @@
 // Every ray therefore visits the FP64 path's tets in the FP64 path's order.
 //
 // Two kinds of step.  A tet entered through a face shared with the previous
-// tet takes the fast step on its record for that entry face (TetRot32): the
-// entry face's vertices sit in fixed slots, so the six products, the exit
-// face (closed form, proven equal to the reference's rule by static_assert),
-// the exit crossing and the chord need no table and no data-dependent
-// indexing beyond picking one of three exit faces.  Anything the fast step
-// cannot decide exactly - an uncertain sign, a rule that does not enter
-// through the known face, an ill-conditioned or hull crossing whose error
+// tet takes the fast step (FastStep): the ray carries the face's triangle, so
+// the step reads one vertex (the record of that entry face, TetGeo32) and the
+// links behind it, and needs no table and no data-dependent indexing beyond
+// picking one of three exit faces (closed form, proven equal to the
+// reference's rule by static_assert).  Anything the fast step
+// cannot decide exactly - an uncertain sign, a face that is not shared vertex
+// by vertex, an ill-conditioned or hull crossing whose error
 // would matter, a midpoint in the slab's guard band, a tet whose FP32 field
-// value is not trusted - goes to the general step (mesh-order record, FP64
-// where needed), which also takes the first tet of every ray.
+// value is not trusted - goes to the general step (mesh vertex order, FP64
+// where needed).
 //
 // What is FP32.  The crossings and the field value.  The exit crossing's z is
 // the apex z plus a barycentric offset (weights = the exit face's signed edge
@@ -78,7 +78,8 @@ struct MixConf {
   int max_visits;
   const TetRec64* __restrict__ rec64;  // exact coordinates when the floats are not
   int exact32;                         // the float coordinates are the doubles
-  const TetRot32* __restrict__ rot;    // records per entry face (NULL: general steps only)
+  const TetGeo32* __restrict__ geo;    // records per entry face
+  const uint4* __restrict__ link;      // their links (NULL: general steps only)
   const signed char* __restrict__ tri_face;  // the tet face under each hull triangle
   const int4* __restrict__ rows;       // the mesh's tetra_data rows (vertex ids, neighbours)
   const double4* __restrict__ pos;     // vertices and their densities, original frame
@@ -86,7 +87,9 @@ struct MixConf {
   int axis;                            // projection axis (frame permutation)
   // Chord midpoints inside (zlo_in, zhi_in) are surely inside the slab for
   // every tet of the mesh; others are tested against their own error bound.
+  // The fast step tests it in float as |z - zc| < zh, which is stricter.
   double zlo_in, zhi_in;
+  float zc, zh;
 };
 
 struct RayState {
@@ -121,43 +124,41 @@ struct Verts32 {
   float z[4];
 };
 
-// The general step sees a tet in the mesh's own vertex order A..D: its record
-// for entry face 3 (ABC) has exactly that slot order (rot_slot(3, k) = k), and
-// the neighbours come from the mesh's tetra_data rows.
-__device__ __forceinline__ const TetRot32* mesh_order(const TetRot32* __restrict__ R, int t) {
-  return R + 4 * (size_t)t + 3;
+// The general step sees a tet in the mesh's own vertex order A..D: vertex k is
+// the apex of its record for entry face k, and the neighbours come from the
+// mesh's tetra_data rows.
+__device__ __forceinline__ float4 vertex32(const TetGeo32* __restrict__ R, int t, int k) {
+  return __ldg(reinterpret_cast<const float4*>(R + 4 * (size_t)t + k));
 }
 
-__device__ __forceinline__ void load32(const TetRot32* __restrict__ R, const int4* __restrict__ rows,
+__device__ __forceinline__ void load32(const TetGeo32* __restrict__ R, const int4* __restrict__ rows,
                                        int t, Verts32& v, int4& nb) {
-  const TetRot32* p = mesh_order(R, t);
-  const float4 a = __ldg(&p->xy01), b = __ldg(&p->xy23), z = __ldg(&p->z);
   nb = __ldg(&rows[2 * (size_t)t + 1]);
-  v.x[0] = a.x; v.y[0] = a.y; v.x[1] = a.z; v.y[1] = a.w;
-  v.x[2] = b.x; v.y[2] = b.y; v.x[3] = b.z; v.y[3] = b.w;
-  v.z[0] = z.x; v.z[1] = z.y; v.z[2] = z.z; v.z[3] = z.w;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float4 a = vertex32(R, t, k);
+    v.x[k] = a.x;
+    v.y[k] = a.y;
+    v.z[k] = a.z;
+  }
 }
 
 // Exact double coordinates of vertex k of tet t, fetched from memory (the
 // float record when its floats are the doubles, else the FP64 record).
-__device__ __forceinline__ double2 xy64_at(const TetRot32* __restrict__ R32,
+__device__ __forceinline__ double2 xy64_at(const TetGeo32* __restrict__ R32,
                                            const TetRec64* __restrict__ R64, int exact32, int t,
                                            int k) {
   if (exact32) {
-    const TetRot32* p = mesh_order(R32, t);
-    const float4 q = __ldg(k < 2 ? &p->xy01 : &p->xy23);
-    return (k & 1) ? make_double2(q.z, q.w) : make_double2(q.x, q.y);
+    const float4 a = vertex32(R32, t, k);
+    return make_double2(a.x, a.y);
   }
   return __ldg(&R64[t].xy[k]);
 }
 
-__device__ __forceinline__ double z64_at(const TetRot32* __restrict__ R32,
+__device__ __forceinline__ double z64_at(const TetGeo32* __restrict__ R32,
                                          const TetRec64* __restrict__ R64, int exact32, int t,
                                          int k) {
-  if (exact32) {
-    const float4 z = __ldg(&mesh_order(R32, t)->z);
-    return (double)sel4(k, z.x, z.y, z.z, z.w);
-  }
+  if (exact32) return (double)vertex32(R32, t, k).z;
   const double2 zz = __ldg(k < 2 ? &R64[t].zab : &R64[t].zcd);
   return (k & 1) ? zz.y : zz.x;
 }
@@ -181,7 +182,7 @@ __device__ __forceinline__ double edge_u64_exact(double lz, double ox, double oy
 
 // Slow path: the reference's six signs for tet t, packed 2 bits per edge
 // (0: zero, 1: positive, 2: negative).
-__device__ __noinline__ unsigned exact_signs(const TetRot32* __restrict__ R32,
+__device__ __noinline__ unsigned exact_signs(const TetGeo32* __restrict__ R32,
                                              const TetRec64* __restrict__ R64, int exact32,
                                              double lz, int t, double ox, double oy) {
   SDTFE_EDGE_TABLES
@@ -217,10 +218,9 @@ struct Hit32 {
 };
 
 // The filtered test of one tet.  u[] receives the FP32 products (units of lz).
-__device__ __forceinline__ Hit32 tet_test(const TetRot32* __restrict__ R32, const MixConf& C,
+__device__ __forceinline__ Hit32 tet_test(const TetGeo32* __restrict__ R32, const MixConf& C,
                                           const RayState& r, int t, const Verts32& v, float u[6],
-                                          float* bmax, const unsigned char* __restrict__ lut,
-                                          int* fallbacks) {
+                                          float* bmax, int* fallbacks) {
   SDTFE_EDGE_TABLES
   float dx[4], dy[4];
   float dmax = 0.f;
@@ -246,7 +246,7 @@ __device__ __forceinline__ Hit32 tet_test(const TetRot32* __restrict__ R32, cons
   *bmax = bound;
   Hit32 h;
   if (unc == 0) {
-    const unsigned ent = lut[neg];
+    const unsigned ent = face_lut_entry(neg);
     h.enter = (int)(ent & 3u);
     h.leave = (int)((ent >> 2) & 3u);
     h.ok = (ent & 16u) != 0;
@@ -294,7 +294,7 @@ __device__ __forceinline__ float crossing(int f, const float u[6], float bmax, c
 // Used where a crossing is not shared with a neighbouring chord (the ray's
 // entry into and exit from the mesh, a re-entry after a perturbation or a
 // turn-around) and where the FP32 weights are ill-conditioned.
-__device__ __noinline__ double exact_crossing(const TetRot32* __restrict__ R32,
+__device__ __noinline__ double exact_crossing(const TetGeo32* __restrict__ R32,
                                                const TetRec64* __restrict__ R64, int exact32,
                                                double lz, int t, int f, double ox, double oy) {
   SDTFE_EDGE_TABLES
@@ -326,7 +326,7 @@ __device__ __noinline__ double exact_crossing(const TetRot32* __restrict__ R32,
 constexpr float kCrossingTol = 9.765625e-4f;
 
 // The reference's FP64 chord midpoint for the chosen faces (slab-test guard).
-__device__ __noinline__ double midpoint64(const TetRot32* __restrict__ R32,
+__device__ __noinline__ double midpoint64(const TetGeo32* __restrict__ R32,
                                           const TetRec64* __restrict__ R64, int exact32, double lz,
                                           int t, int enter, int leave, double ox, double oy) {
   SDTFE_EDGE_TABLES
@@ -364,7 +364,7 @@ __device__ __noinline__ double field64(const MixConf& C, int t, double ox, doubl
 // of one chord is bit-for-bit the entry of the next and the chord lengths
 // telescope.  The slab test compares the float midpoint with a guard band;
 // inside the band the reference's FP64 midpoint decides.
-__device__ __forceinline__ double chord32(const TetRot32* __restrict__ R, const MixConf& C,
+__device__ __forceinline__ double chord32(const TetGeo32* __restrict__ R, const MixConf& C,
                                           const RayState& r, int t, int enter, int leave,
                                           double z_in, double z_out, float hz, float e_inout,
                                           int* fallbacks) {
@@ -443,16 +443,19 @@ __device__ __forceinline__ T sel3(int k, T a, T b, T c) {
   return k == 0 ? a : (k == 1 ? b : c);
 }
 
-struct FastStep {
-  double z_out;    // exit crossing
-  float e_out;     // bound on the exit crossing's z error
-  int next;        // record of the next tet; -1: the ray left the mesh here
-};
-
 // ---------------------------------------------------------------------------
-// What a walk does with each crossed tet.  An accumulator provides
-//   fast(...)        the fast step's chord, from the FP32 exit crossing and the
-//                    record's field; false declines the step (nothing committed)
+// What a walk does with each crossed tet.  The fast step's part of an
+// accumulator:
+//   clear(...)       from the chord's ends: true when the FP32 exit crossing
+//                    decides all there is to decide (the common case)
+//   add(...)         takes the chord that clear() looked at
+//   settle(...)      a chord that is not clear, or ends at the hull: taken
+//                    after all (true), or left to the general step (false,
+//                    nothing committed)
+//   kHullLast        every exit through the hull takes the general step: a ray
+//                    waits for it until the warp's others have come there too,
+//                    instead of holding them up in mid-walk one by one
+// and the general step's:
 //   exact_exit(...)  whether the general step must recompute an FP32 exit
 //                    crossing exactly before its chord
 //   enter(z)         a ray's entry crossing was computed exactly
@@ -460,50 +463,78 @@ struct FastStep {
 //   carry(leave)     the next tet is entered through this tet's leave face
 //                    (true) or, after a turn-around, its enter face (false)
 
+// What the fast step knows of the tet it crosses: the apex relative to the
+// origin, the record's field, and the crossings' error bounds.
+struct FastTet {
+  uint32_t L;          // the tet's link (record and rotation)
+  float X, Y;          // apex - origin
+  float4 a, b;         // the record: (x, y, z, rho), (gx, gy, gz, ext)
+  double zw;           // apex z
+  float c_in, h_in, c_out, h_out;
+  // z error of a crossing: the weights' error c over the face's height h above
+  // the apex, plus the rounding of the offset (the double sum with the apex z
+  // is exact).  The weights' error enters the offset's numerator and its
+  // denominator, so the crossing is within 5/3 of this (and the rounding) of
+  // the exact one.
+  __device__ __forceinline__ static float err(float c, float h) { return (c + 8.f * kEps) * h; }
+  __device__ __forceinline__ float e_in() const { return err(c_in, h_in); }
+  __device__ __forceinline__ float e_out() const { return err(c_out, h_out); }
+};
+
 // Surface density (src/dtfe.c:356-369): the chord's value at its midpoint
 // times its length, when the midpoint lies strictly inside the slab.
 struct SurfaceAcc32 {
+  static constexpr bool kHullLast = false;
   double sum = 0.0;
+  struct Chord {
+    double d;  // length
+    float zr;  // midpoint above the apex
+  };
 
-  // The slab test compares the midpoint with a guard band (the crossings'
-  // error bounds); inside the band the step declines and the reference's FP64
-  // midpoint decides.  The chord value is the reference's own formula
-  // (src/dtfe.c:363-368) from the apex: the tet's linear field
-  // rho3 + grad . (p - v3) at the point p of the ray line at the chord's
-  // midpoint.  p lies on the line, so errors of the crossings only move chord
-  // ends, shared with the neighbours: they cancel to first order.
-  // fld = (rho3, grad_x, grad_y, grad_z); (x3, y3) = v3 - origin.  An exit
-  // through the hull (next == -1) is declined unless the error its FP32
-  // crossing can add to the chord is below 1e-7 of the ray's integral: such a
-  // crossing is not shared with a neighbouring chord, so its error does not
-  // cancel.
-  __device__ __forceinline__ bool fast(const MixConf& C, const RayState&, int, double z_in,
-                                       float e_in, double z_out, float e_out, int next,
-                                       const float4& f, float x3, float y3, float zw) {
-    const double d = z_out - z_in;
-    const double zm = z_in + 0.5 * d;
+  // The chord value is the reference's own formula (src/dtfe.c:363-368) from
+  // the apex: the tet's linear field rho3 + grad . (p - v3) at the point p of
+  // the ray line at the chord's midpoint.  p lies on the line, so errors of
+  // the crossings only move chord ends, shared with the neighbours: they
+  // cancel to first order.
+  __device__ __forceinline__ bool clear(const MixConf& C, const FastTet& t, double z_in,
+                                        double z_out, Chord* ch) const {
+    ch->d = z_out - z_in;
+    ch->zr = (float)(__fma_rn(0.5, ch->d, z_in) - t.zw);
+    return fabsf((t.a.z - C.zc) + ch->zr) < C.zh;
+  }
+  __device__ __forceinline__ double value(const FastTet& t, const Chord& ch) const {
+    return (double)__fmaf_rn(t.b.z, ch.zr, __fmaf_rn(-t.b.y, t.Y, __fmaf_rn(-t.b.x, t.X, t.a.w)));
+  }
+  __device__ __forceinline__ void add(const FastTet& t, const Chord& ch, double, double) {
+    sum = __fma_rn(value(t, ch), ch.d, sum);
+  }
+  // The slab test compares the midpoint, whose error is at most half of e_in +
+  // e_out times 5/3, with a guard band of the whole of e_in + e_out; inside
+  // the band the step declines and the reference's FP64 midpoint decides.
+  // An exit through the hull is declined unless the error its FP32 crossing
+  // can add to the chord is below 1e-7 of the ray's integral (at most about
+  // 1.7e-7, 5/3 e_out): such a crossing is not shared with a neighbouring
+  // chord, so its error does not cancel.
+  __device__ __forceinline__ bool settle(const MixConf& C, const FastTet& t, bool hull, double z_in,
+                                         double z_out, const Chord& ch) {
+    const double zm = __fma_rn(0.5, ch.d, z_in);
     bool inside = true;
     if (!(zm > C.zlo_in && zm < C.zhi_in)) {  // near a slab bound: this chord's own guard
-      const float g = 64.f * kEps * fabsf((float)zm) + e_in + e_out;
+      const float g = 64.f * kEps * fabsf((float)zm) + t.e_in() + t.e_out();
       const float d0 = (float)(zm - C.z0d), d1 = (float)(zm - C.z1d);
       if (!(fabsf(d0) > g && fabsf(d1) > g)) return false;  // the reference's midpoint decides
       inside = d0 > 0.f && d1 < 0.f;
     }
-    const float zr = (float)(zm - (double)zw);
-    const float g = __fmaf_rn(f.w, zr, __fmaf_rn(-f.z, y3, __fmaf_rn(-f.y, x3, f.x)));
-    const double contrib = inside ? (double)g * d : 0.0;
-    if (next == -1 && inside) {
-      // the exit crossing's z error times the field is not cancelled: at most
-      // about 1.7e-7 of the ray's integral (5/3 e_out)
-      if (!(fabsf(g) * e_out <= 1e-7f * (float)fabs(sum + contrib))) return false;
-    }
-    sum += contrib;
+    if (!inside) return true;
+    const double g = value(t, ch), s = __fma_rn(g, ch.d, sum);
+    if (hull && !(fabsf((float)g) * t.e_out() <= 1e-7f * (float)fabs(s))) return false;
+    sum = s;
     return true;
   }
   __device__ __forceinline__ bool exact_exit(double, float) const { return false; }
   __device__ __forceinline__ void enter(double) {}
   __device__ __forceinline__ void carry(bool) {}
-  __device__ __forceinline__ void general(const TetRot32* __restrict__ R, const MixConf& C,
+  __device__ __forceinline__ void general(const TetGeo32* __restrict__ R, const MixConf& C,
                                           const RayState& r, int t, int enter, int leave,
                                           double z_in, double z_out, float hz, float e_inout,
                                           int* fallbacks) {
@@ -511,90 +542,13 @@ struct SurfaceAcc32 {
   }
 };
 
-// One walk step on the record of (tet, entry face), for a ray whose entry
-// crossing (z_in, f_in) was carried over from the previous tet.  Succeeds
-// when the FP32 products decide all six reference signs, the reference's rule
-// enters through the known face and the accumulator takes the chord
-// (SurfaceAcc32: the midpoint is clear of the slab bounds); otherwise nothing
-// is committed and the general step takes the tet.  The step also declines an
-// ill-conditioned exit crossing; the general step computes it exactly.
-template <class Acc>
-__device__ __forceinline__ bool fast_step(const MixConf& C, const RayState& r, int ri,
-                                          double z_in, float e_in, Acc& acc, FastStep* o) {
-  const TetRot32* p = C.rot + ri;
-  const float4 a = __ldg(&p->xy01), b = __ldg(&p->xy23), z = __ldg(&p->z), f = __ldg(&p->fld);
-  const int4 nb = __ldg(&p->nb);
-  const float x0 = __fsub_rn(__fsub_rn(a.x, r.oxh), r.oxl), y0 = __fsub_rn(__fsub_rn(a.y, r.oyh), r.oyl);
-  const float x1 = __fsub_rn(__fsub_rn(a.z, r.oxh), r.oxl), y1 = __fsub_rn(__fsub_rn(a.w, r.oyh), r.oyl);
-  const float x2 = __fsub_rn(__fsub_rn(b.x, r.oxh), r.oxl), y2 = __fsub_rn(__fsub_rn(b.y, r.oyh), r.oyl);
-  const float x3 = __fsub_rn(__fsub_rn(b.z, r.oxh), r.oxl), y3 = __fsub_rn(__fsub_rn(b.w, r.oyh), r.oyl);
-  // The line crossed the entry face (the previous step decided its signs), so
-  // the origin lies in the tet's projection and no |relative coordinate|
-  // exceeds the record's extent: the bound of tet_test with that for dmax.
-  const float dmax = __int_as_float(nb.w & 0x7fffffff);
-  const float bound = __fmaf_ru(kProdErr * kEps * dmax, dmax, __fmaf_ru(r.e_coef, dmax, r.thr_hi));
-  const float e01 = __fmaf_rn(x0, y1, -__fmul_rn(y0, x1));
-  const float e12 = __fmaf_rn(x1, y2, -__fmul_rn(y1, x2));
-  const float e20 = __fmaf_rn(x2, y0, -__fmul_rn(y2, x0));
-  const float a0 = __fmaf_rn(x3, y0, -__fmul_rn(y3, x0));
-  const float a1 = __fmaf_rn(x3, y1, -__fmul_rn(y3, x1));
-  const float a2 = __fmaf_rn(x3, y2, -__fmul_rn(y3, x2));
-  const float umin = fminf(fminf(fminf(fabsf(e01), fabsf(e12)), fminf(fabsf(e20), fabsf(a0))),
-                           fminf(fabsf(a1), fabsf(a2)));
-  // every sign certain, and the reference's rule (rot_exit_rule) enters here;
-  // sign-bit arithmetic, so that the only branch is the decline
-  const unsigned n0 = __float_as_uint(a0) >> 31, n1 = __float_as_uint(a1) >> 31,
-                 n2 = __float_as_uint(a2) >> 31;
-  const unsigned k0 = n1 & ~n2, k1 = n2 & ~n0, k2 = n0 & ~n1;
-  // (sign bit of nb.w: the tet's FP32 field value is not trusted)
-  const unsigned ok = (__float_as_uint(e01) & __float_as_uint(e12) & __float_as_uint(e20) &
-                       ~(unsigned)nb.w) >> 31 &
-                      (k0 | k1 | k2) & (umin > bound ? 1u : 0u);
-  if (!ok) return false;
-  // The exit slot k is one-hot in (k0, k1, k2) (exactly one is set once ok
-  // holds); every choice below picks by those bits with masks, so that lanes
-  // leaving through different faces stay on one instruction stream.
-  const unsigned m0 = 0u - k0, m1 = 0u - k1, m2 = 0u - k2;
-  const auto pick = [m0, m1, m2](float a, float b, float c) {
-    return __uint_as_float((__float_as_uint(a) & m0) | (__float_as_uint(b) & m1) |
-                           (__float_as_uint(c) & m2));
-  };
-  const int next = (int)(((unsigned)nb.x & m0) | ((unsigned)nb.y & m1) | ((unsigned)nb.z & m2));
-  if (next < -1) return false;  // a neighbour that does not list this tet
-  // exit face: apex (slot 3) and slots i = k+1, j = k+2 (mod 3); the weight of
-  // each corner is the product of the face edge opposite it
-  const float w3 = pick(e12, e20, e01);
-  const float wi = -pick(a2, a0, a1);
-  const float wj = pick(a1, a2, a0);
-  const float zi = pick(z.y, z.z, z.x), zj = pick(z.z, z.x, z.y);
-  const float den = w3 + wi + wj;
-  const float rr = __fdividef(1.f, den);
-  const float cond = 3.f * bound * fabsf(rr);  // relative error of the weights
-  const float hi = zi - z.w, hj = zj - z.w;
-  if (!(cond <= kCrossingTol)) return false;  // ill-conditioned
-  const float dzr = rr * __fmaf_rn(wj, hj, wi * hi);
-  // z error: the weights' error over the face's height above the apex, plus
-  // the rounding of the offset (the double sum with the apex z is exact).
-  // The weights' error enters the offset's numerator and its denominator, so
-  // the crossing is within 5/3 e_out (and the rounding) of the exact one; the
-  // slab test compares the midpoint, whose error is at most half of
-  // e_in + e_out times 5/3, with the whole of e_in + e_out.
-  const float e_out = (cond + 8.f * kEps) * fmaxf(fabsf(hi), fabsf(hj));
-  const double z_out = (double)z.w + (double)dzr;
-  if (!acc.fast(C, r, ri >> 2, z_in, e_in, z_out, e_out, next, f, x3, y3, z.w)) return false;
-  o->z_out = z_out;
-  o->e_out = e_out;
-  o->next = next;
-  return true;
-}
-
 // Record of the neighbour across face m of tet t, as entered from t (-1: none).
-__device__ __forceinline__ int rot_next(const MixConf& C, int t, int m) {
-  if (!C.rot) return -1;
+__device__ __forceinline__ int rec_next(const MixConf& C, int t, int m) {
+  if (!C.link) return -1;
   const int G = m == 0 ? 1 : 0;  // a record of t whose entry face is not m
-  const int4 nb = __ldg(&C.rot[4 * (size_t)t + G].nb);
-  const int v = sel3(rot_inv(G, m), nb.x, nb.y, nb.z);
-  return v >= 0 ? v : -1;
+  const uint4 lk = __ldg(C.link + 3 * (4 * (size_t)t + G));
+  const uint32_t L = sel3(rot_inv(G, m), lk.x, lk.y, lk.z);
+  return L <= kLinkLast ? (int)(L / 3u) : -1;
 }
 
 // 3-D grid column (src/dtfe.c:465-513): the tet's linear field is sampled at
@@ -613,6 +567,7 @@ __device__ __forceinline__ int rot_next(const MixConf& C, int t, int m) {
 // built (k + gx x + gy y + gz z) and the general step the reference's own
 // expression from vertex A.
 struct ColumnAcc32 {
+  static constexpr bool kHullLast = true;
   double* col;          // the column's cells (z fastest)
   const double4* __restrict__ fld;  // per-tet FP64 field (mesh_field64)
   double z0, dzs, inv_dzs, w;
@@ -634,27 +589,35 @@ struct ColumnAcc32 {
     const double band = (2.0 * (double)e + 64.0 * DBL_EPSILON * (fabs(z) + fabs(z0) + dzs)) * inv_dzs;
     return fl >= -1.0 && fl < (double)nzs && (*t - fl <= band || fl + 1.0 - *t <= band);
   }
-  __device__ __forceinline__ bool fast(const MixConf&, const RayState& r, int t, double,
-                                       float, double z_out, float e_out, int next, const float4&,
-                                       float, float, float) {
-    if (next < 0) return false;  // the hull exit: its crossing is computed exactly
+  struct Chord {
+    int i1;  // index of the exit crossing's node
+  };
+  __device__ __forceinline__ bool clear(const MixConf&, const FastTet& t, double, double z_out,
+                                        Chord* ch) const {
     double tz;
-    if (near_node(z_out, e_out, &tz)) return false;
+    const bool near = near_node(z_out, t.e_out(), &tz);
     // away from the band tz's ceiling is the reference's index of z_out
-    const int i1u = (int)fmin(fmax(ceil(tz), -1.0), (double)nzs + 1.0);
-    const int i0 = i_in < 0 ? 0 : i_in, i1 = i1u > nzs ? nzs : i1u;
+    ch->i1 = (int)fmin(fmax(ceil(tz), -1.0), (double)nzs + 1.0);
+    return !near;
+  }
+  __device__ __forceinline__ void add(const FastTet& t, const Chord& ch, double ox, double oy) {
+    const int i0 = i_in < 0 ? 0 : i_in, i1 = ch.i1 > nzs ? nzs : ch.i1;
     if (i1 > i0) {
-      const double2 kx = __ldg(reinterpret_cast<const double2*>(fld + t));
-      const double2 yz = __ldg(reinterpret_cast<const double2*>(fld + t) + 1);
-      const double base = kx.x + kx.y * r.ox + yz.x * r.oy;
+      const double2* f = reinterpret_cast<const double2*>(fld + t.L / 12u);
+      const double2 kx = __ldg(f), yz = __ldg(f + 1);
+      const double base = kx.x + kx.y * ox + yz.x * oy;
       for (int is = i0; is < i1; ++is) {
         const int iz = (int)((unsigned)is / (unsigned)ss);
         const double zi = z0 + dzs * is + dzs / 2.;
         cell_add(col + iz, (base + yz.y * zi) * w);
       }
     }
-    i_in = i1u;
-    return true;
+    i_in = ch.i1;
+  }
+  // a crossing near a node, or the hull exit: computed exactly
+  __device__ __forceinline__ bool settle(const MixConf&, const FastTet&, bool, double, double,
+                                         const Chord&) {
+    return false;
   }
   __device__ __forceinline__ bool exact_exit(double z_out, float e_out) const {
     double t;
@@ -664,7 +627,7 @@ struct ColumnAcc32 {
   __device__ __forceinline__ void carry(bool through_leave) {
     if (through_leave) i_in = i_out;  // else the enter face's index, already in i_in
   }
-  __device__ __forceinline__ void general(const TetRot32* __restrict__, const MixConf& C,
+  __device__ __forceinline__ void general(const TetGeo32* __restrict__, const MixConf& C,
                                           const RayState& r, int t, int, int, double, double z_out,
                                           float, float, int* fallbacks) {
     i_out = node_index(z_out);
@@ -692,12 +655,14 @@ struct WalkState {
   Acc acc;
   double z_in;
   float e_in;        // bound on z_in's error
+  uint64_t ray;      // keys the perturbation draws
   uint64_t ctr;      // perturbation draws so far
   int crossed, fallbacks, cur, prev, ri;
   bool carried;      // z_in holds the crossing of the face shared with prev
 };
 
-constexpr int kWalkOn = -1;  // general_step: the walk continues
+constexpr int kWalkOn = -1;    // the walk continues
+constexpr int kWalkHull = -2;  // the fast walk has come to an exit through the hull
 
 // The general step on tet w.cur (src/dtfe.c:300-372): the mesh-order record,
 // the filtered test with the reference's FP64 signs as fallback, perturbation,
@@ -708,8 +673,7 @@ constexpr int kWalkOn = -1;  // general_step: the walk continues
 // about one step in a hundred and would otherwise crowd the fast loop's
 // registers.
 template <class Acc>
-__device__ __noinline__ int general_step(const TetRot32* __restrict__ R, const MixConf& C,
-                                         uint64_t ray, const unsigned char* __restrict__ lut,
+__device__ __noinline__ int general_step(const TetGeo32* __restrict__ R, const MixConf& C,
                                          WalkState<Acc>& w, int* visits, int max_record) {
   RayState& r = w.r;
   const int cur = w.cur;
@@ -717,11 +681,11 @@ __device__ __noinline__ int general_step(const TetRot32* __restrict__ R, const M
   Verts32 v;
   load32(R, C.rows, cur, v, nb);
   float u[6], bmax;
-  Hit32 h = tet_test(R, C, r, cur, v, u, &bmax, lut, &w.fallbacks);
+  Hit32 h = tet_test(R, C, r, cur, v, u, &bmax, &w.fallbacks);
   if (!h.ok) return kRayNoExit;
   int np = 0;
   while (h.special) {  // FP64 perturbation, exactly as the reference (src/dtfe.c:219-245)
-    const int k = sdtfe_rand31(C.seed, ray, w.ctr++) % 4;
+    const int k = sdtfe_rand31(C.seed, w.ray, w.ctr++) % 4;
     const double2 vk = xy64_at(R, C.rec64, C.exact32, cur, k);
     double dx = __dsub_rn(vk.x, r.ox);
     double dy = __dsub_rn(vk.y, r.oy);
@@ -737,7 +701,7 @@ __device__ __noinline__ int general_step(const TetRot32* __restrict__ R, const M
     ray_setup(r, C);
     w.carried = false;  // the ray moved: this tet computes its own entry
     if (++np > kPerturbMax) return kRayPerturbMax;
-    h = tet_test(R, C, r, cur, v, u, &bmax, lut, &w.fallbacks);
+    h = tet_test(R, C, r, cur, v, u, &bmax, &w.fallbacks);
     if (!h.ok) return kRayNoExit;
   }
   const int enter = h.enter, leave = h.leave;
@@ -787,127 +751,349 @@ __device__ __noinline__ int general_step(const TetRot32* __restrict__ R, const M
   }  // else the enter face's crossing, already in z_in
   w.acc.carry(m == leave);
   w.carried = true;
-  w.ri = rot_next(C, cur, m);
+  w.ri = rec_next(C, cur, m);
   w.prev = cur;
   w.cur = nx;
+  return kWalkOn;
+}
+
+// The triangle a fast walk carries: the face the ray last crossed, its
+// vertices relative to the ray origin (z absolute), and their cyclic products
+// u(0,1), u(1,2), u(2,0), all negative.
+struct Tri32 {
+  float x0, y0, z0, x1, y1, z1, x2, y2, z2;
+  float e01, e12, e20;
+};
+
+// u(p, q) = px*qy - py*qx, rounded as one product and one fused multiply-add
+__device__ __forceinline__ float prod32(float px, float py, float qx, float qy) {
+  return __fmaf_rn(px, qy, -__fmul_rn(py, qx));
+}
+
+// What the fast step reads of a RayState.
+struct Origin32 {
+  float oxh, oxl, oyh, oyl, thr_hi, e_coef;
+  __device__ __forceinline__ explicit Origin32(const RayState& r)
+      : oxh(r.oxh), oxl(r.oxl), oyh(r.oyh), oyl(r.oyl), thr_hi(r.thr_hi), e_coef(r.e_coef) {}
+};
+
+// The bound of tet_test for a ray that crossed a face of the tet: the origin
+// then lies in the tet's projection, and no |relative coordinate| exceeds the
+// record's extent.
+__device__ __forceinline__ float product_bound(const Origin32& r, float ext) {
+  return __fmaf_ru(__fmaf_ru(kProdErr * kEps, ext, r.e_coef), ext, r.thr_hi);
+}
+
+// The triangle of record rec's entry face, in the record's order.  False when
+// its products are not all certain and negative (the general step takes the
+// tet), as for a tet whose field is not trusted.
+__device__ __forceinline__ bool entry_triangle(const MixConf& C, const RayState& r, int rec,
+                                               Tri32* s) {
+  const int t = rec >> 2, F = rec & 3;
+  const float4 a = vertex32(C.geo, t, rot_slot(F, 0)), b = vertex32(C.geo, t, rot_slot(F, 1)),
+               c = vertex32(C.geo, t, rot_slot(F, 2));
+  s->x0 = __fsub_rn(__fsub_rn(a.x, r.oxh), r.oxl);
+  s->y0 = __fsub_rn(__fsub_rn(a.y, r.oyh), r.oyl);
+  s->x1 = __fsub_rn(__fsub_rn(b.x, r.oxh), r.oxl);
+  s->y1 = __fsub_rn(__fsub_rn(b.y, r.oyh), r.oyl);
+  s->x2 = __fsub_rn(__fsub_rn(c.x, r.oxh), r.oxl);
+  s->y2 = __fsub_rn(__fsub_rn(c.y, r.oyh), r.oyl);
+  s->z0 = a.z;
+  s->z1 = b.z;
+  s->z2 = c.z;
+  s->e01 = prod32(s->x0, s->y0, s->x1, s->y1);
+  s->e12 = prod32(s->x1, s->y1, s->x2, s->y2);
+  s->e20 = prod32(s->x2, s->y2, s->x0, s->y0);
+  const float bound = product_bound(Origin32(r), __ldg(&C.geo[rec].ext));
+  return s->e01 < -bound && s->e12 < -bound && s->e20 < -bound;
+}
+
+// A record in one 256-bit load.
+__device__ __forceinline__ void load_record(const TetGeo32* p, float4* a, float4* b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a->x), "=f"(a->y), "=f"(a->z), "=f"(a->w), "=f"(b->x), "=f"(b->y), "=f"(b->z),
+        "=f"(b->w)
+      : "l"(p));
+}
+
+// 1/x by the reciprocal instruction alone (x normal wherever the result is used)
+__device__ __forceinline__ float rcp32(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// The fast step.  The ray carries the triangle it last crossed (Tri32), with
+// the origin strictly inside it: its three products are negative, and certain,
+// because each was decided by the step that first met its edge.  The tet adds
+// one vertex, the apex V.  Of a_k = u(V, P_k) two have one sign and one the
+// other (the P_k surround the origin), and the reference's rule
+// (rot_exit_rule) leaves through the face without P_k, a_{k+1} < 0 < a_{k+2}.
+// The triangle of that face is (P_{k+1}, P_{k+2}, V): two vertices stay, and
+// of its products u(k+1, k+2) is carried, u(V, P_{k+1}) = a_{k+1} is known and
+// u(P_{k+2}, V) is formed anew (its rounding is not that of -a_{k+2}).  So a
+// step reads and transforms one vertex and forms four products, with the bits
+// that a record holding all four vertices would give (every product is formed
+// from the same operands in the same cyclic direction).
+// All that can go wrong is gathered in one condition (clear), so that the
+// common step has one branch.
+//
+// What bounds it: instruction issue (73 % of the cycles of 32 warps per SM;
+// 104 thread instructions a visit, 56 of them on the FMA and ALU pipes' FP32)
+// together with the L1's load return (30 wavefronts a warp's visit, 60 % of
+// its cycles: 48 B a lane, lanes of one warp in six to eight tets).  Records
+// of all four vertices (80 B, five 16-byte loads, eight relative coordinates,
+// nine products) took 154 instructions and 41 wavefronts.  131k clustered
+// points, 1024^2 x 16 map: 18.3 -> 13.3 ms; 512^3 grid over the 83k lattice:
+// 3.04 -> 2.37 ms.  Measured and not kept: two steps a loop turn (2 % fewer
+// instructions, 3 to 8 % slower), the next record fetched a step ahead (20 to
+// 70 % slower: 12 registers more), the warp's rays dealt out along a Z-curve
+// (5 % fewer wavefronts, no faster).
+template <class Acc>
+struct FastStep {
+  FastTet t;
+  typename Acc::Chord ch;
+  double z_out;
+  float w3, ai;   // u(i, j) and u(V, P_i) of the exit face (P_i, P_j, V)
+  float zi, zj;
+  uint32_t next;
+  bool k0, k1;    // which vertex is left behind (else the third)
+  bool decided;   // the signs and the exit crossing are good enough
+  bool clear;     // and nothing else needs a closer look
+
+  template <class T>
+  __device__ __forceinline__ T pick(T a, T b, T c) const { return k0 ? a : (k1 ? b : c); }
+
+  __device__ __forceinline__ FastStep(const MixConf& C, const Origin32& r, const Acc& acc,
+                                      const Tri32& s, uint32_t L, double z_in, float c_in,
+                                      float h_in) {
+    load_record(C.geo + L / 3u, &t.a, &t.b);
+    const uint4 lk = __ldg(C.link + L);
+    t.L = L;
+    t.X = __fsub_rn(__fsub_rn(t.a.x, r.oxh), r.oxl);
+    t.Y = __fsub_rn(__fsub_rn(t.a.y, r.oyh), r.oyl);
+    t.zw = (double)t.a.z;
+    const float a0 = prod32(t.X, t.Y, s.x0, s.y0);
+    const float a1 = prod32(t.X, t.Y, s.x1, s.y1);
+    const float a2 = prod32(t.X, t.Y, s.x2, s.y2);
+    const float bound = product_bound(r, t.b.w);
+    const float umin = fminf(fminf(fminf(fabsf(s.e01), fabsf(s.e12)), fminf(fabsf(s.e20), fabsf(a0))),
+                             fminf(fabsf(a1), fabsf(a2)));
+    // (a_0, a_1, a_2 are not all of one sign)
+    const bool p2 = a2 > 0.f;
+    k0 = p2 & (a1 < 0.f);
+    k1 = !p2 & (a0 > 0.f);
+    next = pick(lk.x, lk.y, lk.z);
+    // exit face: apex and slots i = k+1, j = k+2 (mod 3); the weight of each
+    // corner is the product of the face edge opposite it: w_j = a_i, w_i = -a_j
+    w3 = pick(s.e12, s.e20, s.e01);
+    ai = pick(a1, a2, a0);
+    const float aj = pick(a2, a0, a1);
+    zi = pick(s.z1, s.z2, s.z0);
+    zj = pick(s.z2, s.z0, s.z1);
+    const float rr = rcp32(__fadd_rn(__fsub_rn(w3, aj), ai));
+    const float hi = zi - t.a.z, hj = zj - t.a.z;
+    const float dzr = rr * __fmaf_rn(ai, hj, -aj * hi);
+    z_out = t.zw + (double)dzr;
+    t.c_in = c_in;
+    t.h_in = h_in;
+    t.c_out = 3.f * bound * fabsf(rr);  // relative error of the weights
+    t.h_out = fmaxf(fabsf(hi), fabsf(hj));
+    decided = (umin > bound) & (t.c_out <= kCrossingTol);
+    clear = acc.clear(C, t, z_in, z_out, &ch) & decided & (next <= kLinkLast);
+  }
+
+  // the triangle of the exit face
+  __device__ __forceinline__ void advance(Tri32& s) const {
+    const float xi = pick(s.x1, s.x2, s.x0), yi = pick(s.y1, s.y2, s.y0);
+    const float xj = pick(s.x2, s.x0, s.x1), yj = pick(s.y2, s.y0, s.y1);
+    s.e01 = w3;
+    s.e12 = prod32(xj, yj, t.X, t.Y);
+    s.e20 = ai;
+    s.x0 = xi;
+    s.y0 = yi;
+    s.z0 = zi;
+    s.x1 = xj;
+    s.y1 = yj;
+    s.z1 = zj;
+    s.x2 = t.X;
+    s.y2 = t.Y;
+    s.z2 = t.a.z;
+  }
+};
+
+// A walk between fast steps, in memory for the rare steps.
+template <class Acc>
+struct FastWalk {
+  WalkState<Acc> w;
+  Tri32 s;
+  uint32_t L;
+  double z_in;
+  float c_in, h_in;
+  int crossed;
+  bool fast;  // s, L and the entry crossing are set
+};
+
+// General steps until the walk is back on a certain triangle: kWalkOn, or the
+// ray's final status.  The state goes through memory, so that the fast loop's
+// registers are its own.
+template <class Acc>
+__device__ __forceinline__ int general_steps(const TetGeo32* __restrict__ R, const MixConf& C,
+                                             FastWalk<Acc>& f, int* visits, int max_record) {
+  WalkState<Acc>& w = f.w;
+  if (f.fast) {
+    const uint32_t L = f.L;
+    // the general step takes this tet, entered through its record's face
+    w.cur = (int)(L / 12u);
+    w.prev = nb_at(__ldg(&C.rows[2 * (size_t)w.cur + 1]), (int)(L / 3u) & 3);
+    w.z_in = f.z_in;
+    w.e_in = FastTet::err(f.c_in, f.h_in);
+    w.carried = true;
+  }
+  w.crossed = f.crossed;
+  do {
+    if (w.crossed >= C.max_visits) return kRayBudget;
+    // the first tet decides its own entry face (its exact crossing is recomputed)
+    w.carried = w.carried && w.crossed > 0;
+    w.ri = -1;
+    const int status = general_step(R, C, w, visits, max_record);
+    f.crossed = w.crossed;
+    if (status != kWalkOn) return status;
+    f.fast = w.ri >= 0 && entry_triangle(C, w.r, w.ri, &f.s);
+  } while (!f.fast);
+  f.L = 3u * (uint32_t)w.ri;
+  f.z_in = w.z_in;
+  f.c_in = 0.f;
+  f.h_in = w.e_in * (1.f / (8.f * kEps));  // err(c_in, h_in) = w.e_in
   return kWalkOn;
 }
 
 // The mixed walk.  Same control flow as walk64 (src/dtfe.c:247-374); returns
 // the status and the crossing count, and hands each crossed tet's chord to
 // the accumulator.  A tet entered through a known face, with the crossing
-// there in hand, takes the fast step on its record for that entry face; any
-// tet the fast step declines takes the general step.  The first tet is
-// entered through the hull triangle the sample was located in (ft_tri; its
-// face is known from the hull build), at the exact crossing.
+// there in hand, takes the fast step; any tet the fast step declines takes the
+// general step.  The first tet is entered through the hull triangle the sample
+// was located in (ft_tri; its face is known from the hull build), at the exact
+// crossing.
 template <class Acc>
-__device__ __forceinline__ int walk_mixed(const TetRot32* __restrict__ R, const MixConf& C, int ft,
-                                          int ft_tri, double x, double y, uint64_t ray,
-                                          const unsigned char* __restrict__ lut, Acc& acc,
+__device__ __forceinline__ int walk_mixed(const TetGeo32* __restrict__ R, const MixConf& C, int ft,
+                                          int ft_tri, double x, double y, uint64_t ray, Acc& acc,
                                           int* crossed_out, int* fallbacks_out, int* visits,
                                           int max_record) {
   *crossed_out = 0;
   *fallbacks_out = 0;
   if (ft < 0) return kRayMiss;
-  RayState r;
-  r.ox = x;
-  r.oy = y;
-  ray_setup(r, C);
-  uint64_t ctr = 0;
-  double z_in = 0.0;
-  float e_in = 0.f;
-  bool carried = false;
-  int crossed = 0, fallbacks = 0;
-  int cur = ft, prev = -1;
-  int ri = -1;  // cur's record for its entry face (-1: general step)
-  int status = kWalkOn;
-  if (C.rot && ft_tri >= 0) {  // enter through the located hull face, exactly
+  FastWalk<Acc> f;
+  f.w.r.ox = x;
+  f.w.r.oy = y;
+  ray_setup(f.w.r, C);
+  f.w.ray = ray;
+  f.w.ctr = 0;
+  f.w.fallbacks = 0;
+  f.w.cur = ft;
+  f.w.prev = -1;
+  f.w.carried = false;
+  f.w.z_in = 0.0;
+  f.w.e_in = 0.f;
+  f.crossed = 0;
+  f.fast = false;
+  if (C.link && ft_tri >= 0) {  // enter through the located hull face, exactly
     const int F = C.tri_face[ft_tri];
-    z_in = exact_crossing(R, C.rec64, C.exact32, C.lz, ft, F, r.ox, r.oy);
-    acc.enter(z_in);
-    ++fallbacks;
-    carried = true;
-    ri = 4 * ft + F;
+    f.w.z_in = exact_crossing(R, C.rec64, C.exact32, C.lz, ft, F, x, y);
+    acc.enter(f.w.z_in);
+    ++f.w.fallbacks;
+    f.fast = entry_triangle(C, f.w.r, 4 * ft + F, &f.s);
+    f.L = 3u * (4u * (uint32_t)ft + (uint32_t)F);
+    f.z_in = f.w.z_in;
+    f.c_in = f.h_in = 0.f;  // the crossing is exact
   }
+  int status = kWalkOn;
+  if (!f.fast) {
+    f.w.acc = acc;
+    status = general_steps(R, C, f, visits, max_record);
+    acc = f.w.acc;
+  }
+  Origin32 r(f.w.r);
+  Tri32 s = f.s;
+  uint32_t L = f.L;
+  double z_in = f.z_in;
+  float c_in = f.c_in, h_in = f.h_in;
+  int crossed = f.crossed;
+  // general steps, from the fast walk's state and back to it
+  const auto general = [&]() {
+    f.L = L;
+    f.z_in = z_in;
+    f.c_in = c_in;
+    f.h_in = h_in;
+    f.crossed = crossed;
+    f.w.acc = acc;
+    status = general_steps(R, C, f, visits, max_record);
+    acc = f.w.acc;
+    r = Origin32(f.w.r);
+    s = f.s;
+    L = f.L;
+    z_in = f.z_in;
+    c_in = f.c_in;
+    h_in = f.h_in;
+    crossed = f.crossed;
+    x = f.w.r.ox;
+    y = f.w.r.oy;
+  };
   for (;;) {
-    if (crossed >= C.max_visits) {
-      status = kRayBudget;
-      break;
-    }
-    if (ri >= 0) {
-      FastStep o;
-      if (fast_step(C, r, ri, z_in, e_in, acc, &o)) {
-        if (visits != nullptr && crossed < max_record) visits[crossed] = cur;
-        ++crossed;
-        if (o.next < 0) {  // left the mesh
+    while (status == kWalkOn) {
+      const FastStep<Acc> p(C, r, acc, s, L, z_in, c_in, h_in);
+      if (p.clear & (crossed < C.max_visits)) {
+        acc.add(p.t, p.ch, x, y);
+      } else if (p.decided && crossed < C.max_visits && p.next != kLinkGeneral &&
+                 (Acc::kHullLast && p.next == kLinkHull ||
+                  acc.settle(C, p.t, p.next == kLinkHull, z_in, p.z_out, p.ch))) {
+        if (p.next == kLinkHull) {  // leaves the mesh
+          if (Acc::kHullLast) {
+            status = kWalkHull;
+            break;
+          }
+          if (visits != nullptr && crossed < max_record) visits[crossed] = (int)(L / 12u);
+          ++crossed;
           status = kRayOk;
           break;
         }
-        z_in = o.z_out;
-        e_in = o.e_out;
-        prev = cur;
-        ri = o.next;
-        cur = ri >> 2;
+      } else {
+        general();
         continue;
       }
+      if (visits != nullptr && crossed < max_record) visits[crossed] = (int)(L / 12u);
+      ++crossed;
+      p.advance(s);
+      L = p.next;
+      z_in = p.z_out;
+      c_in = p.t.c_out;
+      h_in = p.t.h_out;
     }
-    WalkState<Acc> w;
-    w.r = r;
-    w.acc = acc;
-    w.z_in = z_in;
-    w.e_in = e_in;
-    w.ctr = ctr;
-    w.crossed = crossed;
-    w.fallbacks = fallbacks;
-    w.cur = cur;
-    w.prev = prev;
-    w.ri = -1;
-    // the first tet decides its own entry face (its exact crossing is recomputed)
-    w.carried = carried && crossed > 0;
-    status = general_step(R, C, ray, lut, w, visits, max_record);
-    r = w.r;
-    acc = w.acc;
-    z_in = w.z_in;
-    e_in = w.e_in;
-    ctr = w.ctr;
-    crossed = w.crossed;
-    fallbacks = w.fallbacks;
-    cur = w.cur;
-    prev = w.prev;
-    ri = w.ri;
-    carried = w.carried;
-    if (status != kWalkOn) break;
+    if (!Acc::kHullLast || status != kWalkHull) break;
+    general();
   }
   // as the reference (and walk64): a ray that fails reports no crossings, so
   // that the pixel mean leaves it out
   *crossed_out = status == kRayOk ? crossed : 0;
-  *fallbacks_out = fallbacks;
+  *fallbacks_out = f.w.fallbacks;
   return status;
 }
 
 // The surface-density walk: the ray's integral in *rho_out (0 unless the
 // ray's status is kRayOk).
-__device__ __forceinline__ int walk32(const TetRot32* __restrict__ R, const MixConf& C, int ft,
-                                      int ft_tri, double x, double y, uint64_t ray,
-                                      const unsigned char* __restrict__ lut, double* rho_out,
+__device__ __forceinline__ int walk32(const TetGeo32* __restrict__ R, const MixConf& C, int ft,
+                                      int ft_tri, double x, double y, uint64_t ray, double* rho_out,
                                       int* crossed_out, int* fallbacks_out, int* visits,
                                       int max_record) {
   SurfaceAcc32 acc;
-  const int status = walk_mixed(R, C, ft, ft_tri, x, y, ray, lut, acc, crossed_out, fallbacks_out,
+  const int status = walk_mixed(R, C, ft, ft_tri, x, y, ray, acc, crossed_out, fallbacks_out,
                                 visits, max_record);
   *rho_out = status == kRayOk ? acc.sum : 0.0;
   return status;
 }
 
-// Shared-memory table of the general step: the face rule on 64 sign patterns.
-constexpr int kLutBytes = 64;
-
-__device__ __forceinline__ void fill_lut(unsigned char* lut) {
-  for (int i = threadIdx.x; i < kLutBytes; i += blockDim.x) lut[i] = (unsigned char)face_lut_entry(i);
-}
-
 struct MapArgs32 {
-  const TetRot32* __restrict__ rec;
+  const TetGeo32* __restrict__ rec;
   const TriRec64* __restrict__ tri;
   int n_tri;
   double* __restrict__ map;
@@ -958,8 +1144,7 @@ __device__ __forceinline__ void add_stats32(unsigned long long* stats, bool acti
 // and status of its own walk.
 template <int BLOCK>
 __device__ __forceinline__ void map_tile32(const MapArgs32& a, int tile,
-                                           const int2* __restrict__ loc,
-                                           const unsigned char* __restrict__ lut, double* s_val,
+                                           const int2* __restrict__ loc, double* s_val,
                                            unsigned char* s_ok) {
   const int P = a.TW * a.TH;
   const int tx0 = (tile % a.tiles_x) * a.TW, ty0 = (tile / a.tiles_x) * a.TH;
@@ -979,7 +1164,7 @@ __device__ __forceinline__ void map_tile32(const MapArgs32& a, int tile,
       int ft_tri = -1;
       int ft = locate_from_tile(a.tri, __ldg(loc), xt, yt, a.loc_budget, &status, &ft_tri);
       if (ft >= 0)
-        status = walk32(a.rec, a.C, ft, ft_tri, xt, yt, rid, lut, &v, &crossed, &fb, nullptr, 0);
+        status = walk32(a.rec, a.C, ft, ft_tri, xt, yt, rid, &v, &crossed, &fb, nullptr, 0);
       if (status != kRayOk) v = 0.0;
       if (a.ray_rho) {
         a.ray_rho[rid] = v;
@@ -1012,11 +1197,8 @@ template <int BLOCK, int MINB>
 __global__ void __launch_bounds__(BLOCK, MINB)
     k_map32(const __grid_constant__ MapArgs32 a, const int2* __restrict__ loc) {
   extern __shared__ double s_val32[];  // P*S doubles, then P*S success bytes
-  __shared__ unsigned char s_lut[kLutBytes];
-  fill_lut(s_lut);
-  __syncthreads();
   unsigned char* s_ok = reinterpret_cast<unsigned char*>(s_val32 + a.TW * a.TH * a.S);
-  map_tile32<BLOCK>(a, blockIdx.x, loc + blockIdx.x, s_lut, s_val32, s_ok);
+  map_tile32<BLOCK>(a, blockIdx.x, loc + blockIdx.x, s_val32, s_ok);
 }
 
 // Every tile's shared point location, one thread per tile, before the map
@@ -1077,9 +1259,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
     k_batch32(const __grid_constant__ BatchTable32 P, unsigned long long* __restrict__ queue,
               const int2* __restrict__ loc) {
   extern __shared__ double s_val32[];
-  __shared__ unsigned char s_lut[kLutBytes];
   __shared__ long long s_tile[2];
-  fill_lut(s_lut);
   if (threadIdx.x == 0) s_tile[0] = (long long)atomicAdd(queue, 1ull);
   __syncthreads();
   for (int it = 0;; ++it) {
@@ -1091,13 +1271,13 @@ __global__ void __launch_bounds__(BLOCK, MINB)
     const int j = job_of(P, tile);
     const MapArgs32& a = P.jobs[j].args;
     unsigned char* s_ok = reinterpret_cast<unsigned char*>(s_val32 + a.TW * a.TH * a.S);
-    map_tile32<BLOCK>(a, P.jobs[j].tile0 + (int)(tile - P.jobs[j].first), loc + tile, s_lut,
-                      s_val32, s_ok);
+    map_tile32<BLOCK>(a, P.jobs[j].tile0 + (int)(tile - P.jobs[j].first), loc + tile, s_val32,
+                      s_ok);
     __syncthreads();  // s_val and the claimed slot are reused next
   }
 }
 
-__global__ void __launch_bounds__(128) k_trace32(const TetRot32* __restrict__ rec,
+__global__ void __launch_bounds__(128) k_trace32(const TetGeo32* __restrict__ rec,
                                                  const TriRec64* __restrict__ tri, int n_tri,
                                                  int n_rays, const double* __restrict__ xs,
                                                  const double* __restrict__ ys,
@@ -1106,9 +1286,6 @@ __global__ void __launch_bounds__(128) k_trace32(const TetRot32* __restrict__ re
                                                  int* __restrict__ crossed,
                                                  int* __restrict__ status,
                                                  int* __restrict__ visits, int max_record) {
-  __shared__ unsigned char s_lut[kLutBytes];
-  fill_lut(s_lut);
-  __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_rays) return;
   int st = kRayMiss, c = 0, fb = 0;
@@ -1116,7 +1293,7 @@ __global__ void __launch_bounds__(128) k_trace32(const TetRot32* __restrict__ re
   int ft_tri = -1;
   const int ft = n_tri > 0 ? locate64(tri, 0, xs[i], ys[i], loc_budget, &st, &ft_tri) : -1;
   if (ft >= 0)
-    st = walk32(rec, C, ft, ft_tri, xs[i], ys[i], (uint64_t)i, s_lut, &v, &c, &fb,
+    st = walk32(rec, C, ft, ft_tri, xs[i], ys[i], (uint64_t)i, &v, &c, &fb,
                 visits ? visits + (size_t)i * max_record : nullptr, max_record);
   rho[i] = st == kRayOk ? v : 0.0;
   crossed[i] = c;
@@ -1128,7 +1305,7 @@ __global__ void __launch_bounds__(128) k_trace32(const TetRot32* __restrict__ re
 // reference's positions, each located on the projected hull from triangle 0
 // and walked with ColumnAcc32.  No two threads touch the same column.
 struct GridArgs32 {
-  const TetRot32* __restrict__ rec;
+  const TetGeo32* __restrict__ rec;
   const TriRec64* __restrict__ tri;
   int n_tri, G, ss, loc_budget;
   double dxy, offx, offy;
@@ -1140,9 +1317,6 @@ struct GridArgs32 {
 };
 
 __global__ void __launch_bounds__(128) k_grid32(const __grid_constant__ GridArgs32 a) {
-  __shared__ unsigned char s_lut[kLutBytes];
-  fill_lut(s_lut);
-  __syncthreads();
   int i, j;
   const bool active = grid_column(a.G, &i, &j);
   const long long cidx = (long long)i * a.G + j;
@@ -1168,7 +1342,7 @@ __global__ void __launch_bounds__(128) k_grid32(const __grid_constant__ GridArgs
         const int ft = a.n_tri > 0 ? locate64(a.tri, 0, x, y, a.loc_budget, &st, &ft_tri) : -1;
         if (ft >= 0) {
           const uint64_t rid = ((uint64_t)cidx * a.ss + (uint64_t)is) * a.ss + (uint64_t)js;
-          st = walk_mixed(a.rec, a.C, ft, ft_tri, x, y, rid, s_lut, acc, &c, &fb, nullptr, 0);
+          st = walk_mixed(a.rec, a.C, ft, ft_tri, x, y, rid, acc, &c, &fb, nullptr, 0);
         }
         visits += c;
         fallbacks += fb;
@@ -1194,7 +1368,8 @@ MixConf mix_conf(const Mesh& m, int axis, double z0, double lz, double dist, uin
   C.max_visits = max_visits;
   C.rec64 = m.ax[axis].rec64;
   C.exact32 = m.fp32_exact ? 1 : 0;
-  C.rot = m.ax[axis].rot32;
+  C.geo = m.ax[axis].geo32;
+  C.link = m.ax[axis].link32;
   C.tri_face = m.ax[axis].tri_face;
   C.rows = m.rows;
   C.pos = m.pos;
@@ -1209,6 +1384,11 @@ MixConf mix_conf(const Mesh& m, int axis, double z0, double lz, double dist, uin
   const double G = 64.0 * 5.9604644775390625e-08 * (Z + H) + 2.0 * (double)kCrossingTol * H;
   C.zlo_in = C.z0d + G;
   C.zhi_in = C.z1d - G;
+  // The float test's own error: the midpoint above the apex, the apex from zc
+  // and their sum are each rounded once.
+  C.zc = (float)(C.z0d + 0.5 * lz);
+  const double half = fmin(C.zhi_in - (double)C.zc, (double)C.zc - C.zlo_in);
+  C.zh = (float)((half - 16.0 * 5.9604644775390625e-08 * (Z + H)) * (1.0 - 1e-6));
   return C;
 }
 
@@ -1265,7 +1445,7 @@ static_assert(sizeof(kBatch32) / sizeof(kBatch32[0]) == kNumVariants32, "one bat
 // Checks that an axis has what the mixed walk reads.
 dtfe_status_t check_mixed(const Mesh& m, int axis) {
   const AxisData& A = m.ax[axis];
-  if (!A.rot32 || !A.hull_built) return set_error(DTFE_ERR_INVALID, "mixed walk without FP32 records");
+  if (!A.geo32 || !A.hull_built) return set_error(DTFE_ERR_INVALID, "mixed walk without FP32 records");
   if (!m.fp32_exact && !A.rec64)
     return set_error(DTFE_ERR_INVALID, "coordinates are not floats and no FP64 records are kept");
   return DTFE_OK;
@@ -1281,7 +1461,7 @@ dtfe_status_t map_args32(Mesh& m, const MapGeom& g, int vi, double* d_map,
   const AxisData& A = m.ax[g.axis];
   const Variant32& V = kVariants32[vi];
   MapArgs32& a = *out;
-  a.rec = A.rot32;
+  a.rec = A.geo32;
   a.tri = A.tri;
   a.n_tri = A.n_tri;
   a.map = d_map;
@@ -1347,7 +1527,7 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
   if ((long long)G * ss > (1LL << 30))
     return set_error(DTFE_ERR_UNSUPPORTED, "grid_dim %d x supersampling %u: too many nodes", G, ss);
   GridArgs32 a;
-  a.rec = A.rot32;
+  a.rec = A.geo32;
   a.tri = A.tri;
   a.n_tri = A.n_tri;
   a.G = G;
@@ -1369,7 +1549,7 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
   a.stats = m.stats;
   SDTFE_CUDA(cudaMemsetAsync(m.stats, 0, sizeof(unsigned long long) * kStatCount, s));
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
-  k_grid32<<<grid_blocks(G), 128, 0, s>>>(a);
+  k_grid32<<<grid_warps(G) / 4, 128, 0, s>>>(a);
   count_launch();
   SDTFE_CUDA(cudaGetLastError());
   SDTFE_CUDA(cudaEventRecord(m.ev1, s));
@@ -1385,7 +1565,7 @@ dtfe_status_t launch_trace32(Mesh& m, int axis, int n_rays, const double* d_x, c
   const AxisData& A = m.ax[axis];
   MixConf C = mix_conf(m, axis, z0, lz, (dxy / 2.0) / kPerturbMax, seed, max_visits);
   if (n_rays > 0) {
-    k_trace32<<<(n_rays + 127) / 128, 128, 0, s>>>(A.rot32, A.tri, A.n_tri, n_rays, d_x, d_y, C,
+    k_trace32<<<(n_rays + 127) / 128, 128, 0, s>>>(A.geo32, A.tri, A.n_tri, n_rays, d_x, d_y, C,
                                                    4 * A.n_tri + 64, d_rho, d_crossed, d_status,
                                                    d_visits, max_record);
     count_launch();

@@ -363,18 +363,20 @@ struct SurfaceAcc64 {
 __device__ __forceinline__ void cell_add(double* cell, double v) { atomicAdd(cell, v); }
 
 // This thread's grid column (i: x index, j: y index) in a launch of
-// grid_blocks(G) blocks of 128 threads: a block covers 8 x 16 columns and
-// each of its warps a 4 x 8 patch, so that a warp's columns are neighbours
-// and cross many of the same tets.  False for the columns past the grid.
+// grid_warps(G) warps: each warp covers a 4 x 8 patch and four in a row an
+// 8 x 16 tile, so that a warp's columns are neighbours and cross many of the
+// same tets.  False for the columns past the grid.
 __device__ __forceinline__ bool grid_column(int G, int* i, int* j) {
+  const int warp = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  const int tile = warp >> 2, wq = warp & 3;
   const int tiles_j = (G + 15) >> 4;
-  const int ti = (int)blockIdx.x / tiles_j, tj = (int)blockIdx.x - ti * tiles_j;
-  const int lane = (int)threadIdx.x & 31, wq = (int)threadIdx.x >> 5;
+  const int ti = tile / tiles_j, tj = tile - ti * tiles_j;
+  const int lane = (int)threadIdx.x & 31;
   *i = ti * 8 + (wq >> 1) * 4 + (lane >> 3);
   *j = tj * 16 + (wq & 1) * 8 + (lane & 7);
   return *i < G && *j < G;
 }
-inline unsigned grid_blocks(int G) { return (unsigned)(((G + 7) / 8) * ((G + 15) / 16)); }
+inline unsigned grid_warps(int G) { return 4u * (unsigned)(((G + 7) / 8) * ((G + 15) / 16)); }
 
 // a12: 3-D column, src/dtfe.c:489-513.  The field is sampled at the fine z
 // nodes inside the chord and added, with weight 1/ss^3, to the column cell.
