@@ -1,0 +1,152 @@
+// grid_rays.cuh - 3-D grids with one thread per sub-ray.
+//
+// A cell of a supersampled grid receives the node values of ss^2 sub-rays, and
+// the reference adds them sub-ray by sub-ray, each in walk order
+// (src/dtfe.c:710-729).  One thread per column keeps that order by walking its
+// ss^2 rays one after the other, which leaves most of the GPU idle below a few
+// hundred columns a side: 120^2 columns at ss = 2 are 450 warps, each waiting
+// through four walks.  Here every sub-ray has its thread and writes its node
+// values to a row of its own; a second kernel adds each cell's values in the
+// reference's order, so the cells are the same to the bit.  A node no chord
+// holds is written as -0.0, which changes no sum.  A ray that comes back to a
+// node it has passed (after a turn-around or a perturbation) has no place for
+// the second value: its column is marked and walked by the one-thread kernel.
+#pragma once
+
+#include "mesh.h"
+
+namespace sdtfe {
+namespace {
+
+// where a column's node values go: its cells directly ...
+struct CellSink {
+  double* col;
+  int ss;
+  __device__ __forceinline__ void begin(int) {}
+  __device__ __forceinline__ void put(int is, double v) {
+    cell_add(col + (int)((unsigned)is / (unsigned)ss), v);
+  }
+};
+
+// ... or the ray's row of nodes
+struct NodeSink {
+  double* row;
+  int done;        // nodes written so far
+  bool irregular;  // came back to one of them
+  __device__ __forceinline__ void begin(int is) {
+    if (is < done) irregular = true;
+    for (; done < is; ++done) row[done] = -0.0;
+  }
+  __device__ __forceinline__ void put(int is, double v) {
+    if (is < done) return;
+    row[is] = v;
+    done = is + 1;
+  }
+};
+
+// A grid's sub-rays.
+struct GridRays {
+  int G, ss;
+  double* nodes;  // row (i*G + j)*ss^2 + is*ss + js of G*ss nodes
+  int* col;       // per column: bit k for a ray of status k, and kIrregular
+};
+constexpr int kIrregular = 1 << 8;
+
+__device__ __forceinline__ int worst_status(int marks) {
+  return 31 - __clz((marks & (kIrregular - 1)) | 1);
+}
+
+// This thread's sub-ray, (column i, j; sub-ray is, js), in a launch over
+// ray_warps(): warps cover compact patches of the fine grid.
+__device__ __forceinline__ bool ray_of_grid(const GridRays& a, int* i, int* j, int* is, int* js) {
+  const int nf = a.G * a.ss;  // fine columns a side
+  const int warp = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  const int tiles_j = (nf + 7) >> 3;
+  const int lane = (int)threadIdx.x & 31;
+  const int fi = (warp / tiles_j) * 4 + (lane >> 3), fj = (warp % tiles_j) * 8 + (lane & 7);
+  *i = fi / a.ss;
+  *j = fj / a.ss;
+  *is = fi % a.ss;
+  *js = fj % a.ss;
+  return fi < nf && fj < nf;
+}
+inline long long ray_warps(const GridRays& a) {
+  const long long nf = (long long)a.G * a.ss;
+  return ((nf + 3) / 4) * ((nf + 7) / 8);
+}
+
+__device__ __forceinline__ double* ray_nodes(const GridRays& a, int i, int j, int is, int js) {
+  const size_t ray = (((size_t)i * a.G + j) * a.ss + is) * a.ss + js;
+  return a.nodes + ray * ((size_t)a.G * a.ss);
+}
+
+__device__ __forceinline__ void ray_done(const GridRays& a, int i, int j, NodeSink& out, int status) {
+  for (const int n = a.G * a.ss; out.done < n; ++out.done) out.row[out.done] = -0.0;
+  atomicOr(a.col + (size_t)i * a.G + j, 1 << status | (out.irregular ? kIrregular : 0));
+}
+
+// One thread per cell: its ss^3 node values, sub-ray by sub-ray.
+__global__ void __launch_bounds__(256) k_grid_sum(const GridRays a, double* __restrict__ grid) {
+  const long long cell = blockIdx.x * 256LL + threadIdx.x;
+  if (cell >= (long long)a.G * a.G * a.G) return;
+  const int iz = (int)(cell % a.G);
+  const long long c = cell / a.G;
+  if (a.col[c] & kIrregular) return;
+  const int nzs = a.G * a.ss;
+  const double* v = a.nodes + (size_t)c * a.ss * a.ss * nzs + iz * a.ss;
+  double sum = grid[cell];
+  for (int r = 0; r < a.ss * a.ss; ++r, v += nzs)
+    for (int k = 0; k < a.ss; ++k) sum += v[k];
+  grid[cell] = sum;
+}
+
+// Which grids are walked by sub-rays: all with several a column, as long as the
+// rows of nodes (8 B times the fine grid) stay within 4 GiB - up to 406^3 cells
+// at ss = 2, 268^3 at 3, 203^3 at 4.  One thread a column is slower below and,
+// measured, still at that size (83k-point lattice, mixed / FP64, one thread a
+// column -> sub-rays): 128^3 ss 4 15.1 / 11.3 -> 3.2 / 2.4 ms, 200^3 ss 2 3.8 /
+// 2.8 -> 2.8 / 1.6, 256^3 ss 3 12.8 / 9.6 -> 6.7 / 5.3, 384^3 ss 2 8.8 / 7.0 ->
+// 6.8 / 5.6.  Batches of the rows lose that again to one tail each (384^3 in 1
+// GiB batches: 12.8 / 6.7).
+constexpr size_t kNodeBytes = size_t(4) << 30;
+inline bool grid_takes_rays(int G, unsigned ss) {
+  const double n = (double)G * ss;
+  return ss > 1 && 8.0 * n * n * n <= (double)kNodeBytes;
+}
+
+// The grid by sub-rays: rays(GridRays) launches the walks, serial(GridRays) the
+// one-thread columns, which counts the columns' outcomes and walks those that are
+// marked irregular.  *taken is false when the grid is not for this, or its
+// scratch is not to be had: nothing has been done.
+template <class Rays, class Serial>
+dtfe_status_t grid_by_rays(int G, unsigned ss, double* d_grid, cudaStream_t s, bool* taken,
+                           Rays&& rays, Serial&& serial) {
+  *taken = false;
+  if (!grid_takes_rays(G, ss)) return DTFE_OK;
+  const size_t n = (size_t)G * ss, col_bytes = sizeof(int) * (size_t)G * G;
+  void *nodes = nullptr, *col = nullptr;
+  if (scratch_alloc_async(&nodes, sizeof(double) * n * n * n, s) != DTFE_OK ||
+      scratch_alloc_async(&col, col_bytes, s) != DTFE_OK) {
+    scratch_free_async(nodes, s);
+    cudaGetLastError();
+    dtfe_clear_error();
+    return DTFE_OK;
+  }
+  *taken = true;
+  const GridRays a{G, (int)ss, static_cast<double*>(nodes), static_cast<int*>(col)};
+  cudaError_t e = cudaMemsetAsync(col, 0, col_bytes, s);
+  if (e == cudaSuccess) {
+    rays(a);
+    k_grid_sum<<<(unsigned)(((long long)G * G * G + 255) / 256), 256, 0, s>>>(a, d_grid);
+    serial(a);
+    count_launch(3);
+    e = cudaGetLastError();
+  }
+  scratch_free_async(nodes, s);
+  scratch_free_async(col, s);
+  SDTFE_CUDA(e);
+  return DTFE_OK;
+}
+
+}  // namespace
+}  // namespace sdtfe

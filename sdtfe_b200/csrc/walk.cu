@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 
+#include "grid_rays.cuh"
 #include "mesh.h"
 
 namespace sdtfe {
@@ -197,44 +198,71 @@ __global__ void __launch_bounds__(128) k_trace64(const TetRec64* __restrict__ re
   status[i] = st;
 }
 
+struct GridArgs64 {
+  const TetRec64* __restrict__ rec;
+  const TriRec64* __restrict__ tri;
+  int n_tri, G, ss, loc_budget;
+  double dxy, offx, offy, offz, dzs, w;
+  WalkConf64 walk;
+  double* __restrict__ grid;
+  unsigned long long* __restrict__ stats;
+};
+
+// Sub-ray (is, js) of column (i, j) (src/dtfe.c:710-729): its status and crossings.
+template <class Sink>
+__device__ __forceinline__ int grid_ray64(const GridArgs64& a, int i, int j, int is, int js,
+                                          ColumnAcc64<Sink>& acc, int* crossed) {
+  const double ds = a.dxy / a.ss;
+  const double x = i * a.dxy + a.offx + is * ds + ds / 2.;
+  const double y = j * a.dxy + a.offy + js * ds + ds / 2.;
+  int st = kRayMiss;
+  *crossed = 0;
+  const int ft = a.n_tri > 0 ? locate64(a.tri, 0, x, y, a.loc_budget, &st) : -1;
+  if (ft < 0) return st;
+  const uint64_t rid = (((uint64_t)i * a.G + j) * a.ss + (uint64_t)is) * a.ss + (uint64_t)js;
+  return walk64(a.rec, ft, x, y, a.walk, rid, acc, crossed, nullptr, 0);
+}
+
 // One thread per grid column (i, j); its ss^2 sub-rays run in (is, js) order
 // and add into the column in walk order, as interpolate_to_3d_grid does
-// (src/dtfe.c:710-729).  No two threads touch the same column.
-__global__ void __launch_bounds__(128) k_grid64(const TetRec64* __restrict__ rec,
-                                                const TriRec64* __restrict__ tri, int n_tri, int G,
-                                                double dxy, double offx, double offy, double offz,
-                                                double box_len, int ss, WalkConf64 walk,
-                                                int loc_budget, double* __restrict__ grid,
-                                                unsigned long long* __restrict__ stats) {
+// (src/dtfe.c:710-729).  No two threads touch the same column.  Marked: after the
+// sub-rays of r, to count the columns' outcomes and walk the irregular ones.
+template <bool Marked>
+__global__ void __launch_bounds__(128) k_grid64(const GridArgs64 a, const GridRays r) {
   int i, j;
-  const bool active = grid_column(G, &i, &j);
-  const long long cidx = (long long)i * G + j;
+  bool active = grid_column(a.G, &i, &j);
+  const int marks = Marked && active ? r.col[(size_t)i * a.G + j] : 0;
   int worst = kRayOk, visits = 0;
-  if (active) {
-    const double ds = dxy / ss;
-    ColumnAcc64 acc;
-    acc.col = grid + (size_t)cidx * G;
-    acc.z0 = offz;
-    const double dz = box_len / G;
-    acc.dzs = dz / ss;
-    acc.nzs = G * ss;
-    acc.w = 1. / ((unsigned)ss * (unsigned)ss * (unsigned)ss);
-    acc.ss = ss;
-    for (int is = 0; is < ss; ++is)
-      for (int js = 0; js < ss; ++js) {
-        const double x = i * dxy + offx + is * ds + ds / 2.;
-        const double y = j * dxy + offy + js * ds + ds / 2.;
-        int st = kRayMiss, c = 0;
-        const int ft = n_tri > 0 ? locate64(tri, 0, x, y, loc_budget, &st) : -1;
-        if (ft >= 0) {
-          const uint64_t rid = ((uint64_t)cidx * ss + (uint64_t)is) * ss + (uint64_t)js;
-          st = walk64(rec, ft, x, y, walk, rid, acc, &c, nullptr, 0);
-        }
+  if (Marked ? (marks & kIrregular) != 0 : active) {
+    ColumnAcc64<CellSink> acc{{a.grid + ((size_t)i * a.G + j) * a.G, a.ss}, a.offz, a.dzs, a.w,
+                              a.G * a.ss};
+    for (int is = 0; is < a.ss; ++is)
+      for (int js = 0; js < a.ss; ++js) {
+        int c;
+        const int st = grid_ray64(a, i, j, is, js, acc, &c);
         visits += c;
         if (st > worst) worst = st;
       }
   }
-  add_stats(stats, active, visits, worst, 0);
+  if (Marked) {  // the rays' crossings have been counted
+    active = marks != 0;
+    visits = 0;
+    worst = worst_status(marks);
+  }
+  add_stats(a.stats, active, visits, worst, 0);
+}
+
+// One thread per sub-ray, node values to the ray's row (grid_rays.cuh).
+__global__ void __launch_bounds__(64) k_grid_rays64(const GridArgs64 a, const GridRays r) {
+  int i, j, is, js, c = 0;
+  if (ray_of_grid(r, &i, &j, &is, &js)) {
+    ColumnAcc64<NodeSink> acc{{ray_nodes(r, i, j, is, js), 0, false}, a.offz, a.dzs, a.w,
+                              a.G * a.ss};
+    const int st = grid_ray64(a, i, j, is, js, acc, &c);
+    ray_done(r, i, j, acc.out, st);
+  }
+  const unsigned sum = __reduce_add_sync(0xffffffffu, (unsigned)c);
+  if ((threadIdx.x & 31) == 0 && sum) atomicAdd(a.stats + kStatVisits, (unsigned long long)sum);
 }
 
 }  // namespace
@@ -426,16 +454,36 @@ dtfe_status_t launch_grid64(Mesh& m, int G, double box_len, const double center[
                             uint64_t seed, int max_visits, double* d_grid, cudaStream_t s) {
   const AxisData& A = m.ax[DTFE_AXIS_Z];
   if (!A.rec64 || !A.hull_built) return set_error(DTFE_ERR_INVALID, "grid before its records");
-  const double dxy = box_len / G;
-  const double offx = -(box_len / 2.0) + center[0];
-  const double offy = -(box_len / 2.0) + center[1];
-  const double offz = -(box_len / 2.0) + center[2];
-  WalkConf64 w{box_len, (dxy / 2.0) / kPerturbMax, seed, max_visits};
+  GridArgs64 a;
+  a.rec = A.rec64;
+  a.tri = A.tri;
+  a.n_tri = A.n_tri;
+  a.G = G;
+  a.ss = (int)ss;
+  a.loc_budget = 4 * A.n_tri + 64;
+  // src/dtfe.c:668-735 and :398-404: cell and node spacing, weight 1/ss^3
+  a.dxy = box_len / G;
+  a.offx = -(box_len / 2.0) + center[0];
+  a.offy = -(box_len / 2.0) + center[1];
+  a.offz = -(box_len / 2.0) + center[2];
+  a.dzs = box_len / G / a.ss;
+  a.w = 1. / (ss * ss * ss);
+  a.walk = WalkConf64{box_len, (a.dxy / 2.0) / kPerturbMax, seed, max_visits};
+  a.grid = d_grid;
+  a.stats = m.stats;
   SDTFE_CUDA(cudaMemsetAsync(m.stats, 0, sizeof(unsigned long long) * kStatCount, s));
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
-  k_grid64<<<grid_warps(G) / 4, 128, 0, s>>>(A.rec64, A.tri, A.n_tri, G, dxy, offx, offy, offz,
-                                          box_len, (int)ss, w, 4 * A.n_tri + 64, d_grid, m.stats);
-  count_launch();
+  bool taken = false;
+  SDTFE_TRY(grid_by_rays(
+      G, ss, d_grid, s, &taken,
+      [&](const GridRays& r) {
+        k_grid_rays64<<<(unsigned)((ray_warps(r) + 1) / 2), 64, 0, s>>>(a, r);
+      },
+      [&](const GridRays& r) { k_grid64<true><<<grid_warps(G) / 4, 128, 0, s>>>(a, r); }));
+  if (!taken) {
+    k_grid64<false><<<grid_warps(G) / 4, 128, 0, s>>>(a, GridRays{});
+    count_launch();
+  }
   SDTFE_CUDA(cudaGetLastError());
   SDTFE_CUDA(cudaEventRecord(m.ev1, s));
   m.timed = true;

@@ -49,6 +49,7 @@
 #include <cfloat>
 #include <cstring>
 
+#include "grid_rays.cuh"
 #include "mesh.h"
 
 namespace sdtfe {
@@ -566,12 +567,13 @@ __device__ __forceinline__ int rec_next(const MixConf& C, int t, int m) {
 // precision, so the fast step evaluates the per-tet FP64 field k_field64
 // built (k + gx x + gy y + gz z) and the general step the reference's own
 // expression from vertex A.
+template <class Sink>  // grid_rays.cuh
 struct ColumnAcc32 {
   static constexpr bool kHullLast = true;
-  double* col;          // the column's cells (z fastest)
+  Sink out;             // where the node values go
   const double4* __restrict__ fld;  // per-tet FP64 field (mesh_field64)
   double z0, dzs, inv_dzs, w;
-  int nzs, ss;
+  int nzs;
   int i_in;             // index of the first node of the next chord (clamped to [-1, nzs + 1])
   int i_out;            // the general step's exit index
 
@@ -606,10 +608,10 @@ struct ColumnAcc32 {
       const double2* f = reinterpret_cast<const double2*>(fld + t.L / 12u);
       const double2 kx = __ldg(f), yz = __ldg(f + 1);
       const double base = kx.x + kx.y * ox + yz.x * oy;
+      out.begin(i0);
       for (int is = i0; is < i1; ++is) {
-        const int iz = (int)((unsigned)is / (unsigned)ss);
         const double zi = z0 + dzs * is + dzs / 2.;
-        cell_add(col + iz, (base + yz.y * zi) * w);
+        out.put(is, (base + yz.y * zi) * w);
       }
     }
     i_in = ch.i1;
@@ -639,10 +641,10 @@ struct ColumnAcc32 {
     const double gx = C.grad[3 * (size_t)t], gy = C.grad[3 * (size_t)t + 1],
                  gz = C.grad[3 * (size_t)t + 2];
     const double fixed = A.w + gx * (r.ox - A.x) + gy * (r.oy - A.y) - gz * A.z;
+    out.begin(i0);
     for (int is = i0; is < i1; ++is) {
-      const int iz = (int)((unsigned)is / (unsigned)ss);
       const double zi = z0 + dzs * is + dzs / 2.;
-      cell_add(col + iz, (fixed + gz * zi) * w);
+      out.put(is, (fixed + gz * zi) * w);
     }
     ++*fallbacks;
   }
@@ -1316,40 +1318,73 @@ struct GridArgs32 {
   unsigned long long* __restrict__ stats;
 };
 
-__global__ void __launch_bounds__(128) k_grid32(const __grid_constant__ GridArgs32 a) {
+template <class Sink>
+__device__ __forceinline__ ColumnAcc32<Sink> column_acc32(const GridArgs32& a, const Sink& out) {
+  return ColumnAcc32<Sink>{out, a.fld, a.z0, a.dzs, a.inv_dzs, a.w, a.G * a.ss, 0, 0};
+}
+
+// Sub-ray (is, js) of column (i, j): its status, crossings and FP64 fallbacks.
+template <class Sink>
+__device__ __forceinline__ int grid_ray32(const GridArgs32& a, int i, int j, int is, int js,
+                                          ColumnAcc32<Sink>& acc, int* crossed, int* fallbacks) {
+  const double ds = a.dxy / a.ss;
+  const double x = i * a.dxy + a.offx + is * ds + ds / 2.;
+  const double y = j * a.dxy + a.offy + js * ds + ds / 2.;
+  int st = kRayMiss, ft_tri = -1;
+  *crossed = 0;
+  *fallbacks = 0;
+  const int ft = a.n_tri > 0 ? locate64(a.tri, 0, x, y, a.loc_budget, &st, &ft_tri) : -1;
+  if (ft < 0) return st;
+  const uint64_t rid = (((uint64_t)i * a.G + j) * a.ss + (uint64_t)is) * a.ss + (uint64_t)js;
+  return walk_mixed(a.rec, a.C, ft, ft_tri, x, y, rid, acc, crossed, fallbacks, nullptr, 0);
+}
+
+// One thread per column.  Marked: after the sub-rays of r, to count the columns'
+// outcomes and walk the irregular ones.  MinBlocks: what the registers are
+// limited for; a small grid leaves the SMs few columns, and takes its walks
+// without spills (launch_grid32).
+template <bool Marked, int MinBlocks>
+__global__ void __launch_bounds__(128, MinBlocks)
+    k_grid32(const __grid_constant__ GridArgs32 a, const GridRays r) {
   int i, j;
-  const bool active = grid_column(a.G, &i, &j);
-  const long long cidx = (long long)i * a.G + j;
+  bool active = grid_column(a.G, &i, &j);
+  const int marks = Marked && active ? r.col[(size_t)i * a.G + j] : 0;
   int worst = kRayOk, visits = 0, fallbacks = 0;
-  if (active) {
-    const double ds = a.dxy / a.ss;
-    ColumnAcc32 acc;
-    acc.col = a.grid + (size_t)cidx * a.G;
-    acc.fld = a.fld;
-    acc.z0 = a.z0;
-    acc.dzs = a.dzs;
-    acc.inv_dzs = a.inv_dzs;
-    acc.w = a.w;
-    acc.nzs = a.G * a.ss;
-    acc.ss = a.ss;
-    acc.i_in = 0;
-    acc.i_out = 0;
+  if (Marked ? (marks & kIrregular) != 0 : active) {
+    auto acc = column_acc32(a, CellSink{a.grid + ((size_t)i * a.G + j) * a.G, a.ss});
     for (int is = 0; is < a.ss; ++is)
       for (int js = 0; js < a.ss; ++js) {
-        const double x = i * a.dxy + a.offx + is * ds + ds / 2.;
-        const double y = j * a.dxy + a.offy + js * ds + ds / 2.;
-        int st = kRayMiss, c = 0, fb = 0, ft_tri = -1;
-        const int ft = a.n_tri > 0 ? locate64(a.tri, 0, x, y, a.loc_budget, &st, &ft_tri) : -1;
-        if (ft >= 0) {
-          const uint64_t rid = ((uint64_t)cidx * a.ss + (uint64_t)is) * a.ss + (uint64_t)js;
-          st = walk_mixed(a.rec, a.C, ft, ft_tri, x, y, rid, acc, &c, &fb, nullptr, 0);
-        }
+        int c, fb;
+        const int st = grid_ray32(a, i, j, is, js, acc, &c, &fb);
         visits += c;
         fallbacks += fb;
         if (st > worst) worst = st;
       }
   }
+  if (Marked) {  // the rays' crossings have been counted
+    active = marks != 0;
+    visits = 0;
+    worst = worst_status(marks);
+    fallbacks = 0;
+  }
   add_stats32(a.stats, active, visits, worst, fallbacks);
+}
+
+// One thread per sub-ray, node values to the ray's row (grid_rays.cuh).
+__global__ void __launch_bounds__(64)
+    k_grid_rays32(const __grid_constant__ GridArgs32 a, const GridRays r) {
+  int i, j, is, js, c = 0, fb = 0;
+  if (ray_of_grid(r, &i, &j, &is, &js)) {
+    auto acc = column_acc32(a, NodeSink{ray_nodes(r, i, j, is, js), 0, false});
+    const int st = grid_ray32(a, i, j, is, js, acc, &c, &fb);
+    ray_done(r, i, j, acc.out, st);
+  }
+  const unsigned v = __reduce_add_sync(0xffffffffu, (unsigned)c);
+  const unsigned f = __reduce_add_sync(0xffffffffu, (unsigned)fb);
+  if ((threadIdx.x & 31) == 0) {
+    if (v) atomicAdd(a.stats + kStatVisits, (unsigned long long)v);
+    if (f) atomicAdd(a.stats + kStatFallback, (unsigned long long)f);
+  }
 }
 
 MixConf mix_conf(const Mesh& m, int axis, double z0, double lz, double dist, uint64_t seed,
@@ -1549,8 +1584,21 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
   a.stats = m.stats;
   SDTFE_CUDA(cudaMemsetAsync(m.stats, 0, sizeof(unsigned long long) * kStatCount, s));
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
-  k_grid32<<<grid_warps(G) / 4, 128, 0, s>>>(a);
-  count_launch();
+  bool taken = false;
+  SDTFE_TRY(grid_by_rays(
+      G, ss, d_grid, s, &taken,
+      [&](const GridRays& r) {
+        k_grid_rays32<<<(unsigned)((ray_warps(r) + 1) / 2), 64, 0, s>>>(a, r);
+      },
+      [&](const GridRays& r) { k_grid32<true, 4><<<grid_warps(G) / 4, 128, 0, s>>>(a, r); }));
+  if (!taken) {
+    // four blocks of 128 columns per SM are all of a grid of up to 148 x 512
+    // columns; a larger one gains more from six blocks per SM than it loses to
+    // spills (83k-point lattice: 256^3 0.736 against 0.771 ms, 512^3 2.47 against 2.42)
+    const bool small = (long long)G * G <= 148 * 512;
+    (small ? k_grid32<false, 4> : k_grid32<false, 6>)<<<grid_warps(G) / 4, 128, 0, s>>>(a, GridRays{});
+    count_launch();
+  }
   SDTFE_CUDA(cudaGetLastError());
   SDTFE_CUDA(cudaEventRecord(m.ev1, s));
   m.timed = true;

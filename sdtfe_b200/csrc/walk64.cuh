@@ -380,10 +380,11 @@ inline unsigned grid_warps(int G) { return 4u * (unsigned)(((G + 7) / 8) * ((G +
 
 // a12: 3-D column, src/dtfe.c:489-513.  The field is sampled at the fine z
 // nodes inside the chord and added, with weight 1/ss^3, to the column cell.
+template <class Sink>  // grid_rays.cuh
 struct ColumnAcc64 {
-  double* col;
+  Sink out;
   double z0, dzs, w;
-  int nzs, ss;
+  int nzs;
   __device__ __forceinline__ void visit(double ox, double oy, const double2& xyA, double zA,
                                         double rhoA, double gx, double gy, double gz, double z_in,
                                         double z_out) {
@@ -393,10 +394,10 @@ struct ColumnAcc64 {
     i1 = i1 > nzs ? nzs : i1;
     if (i1 > i0) {
       const double fixed = rhoA + gx * (ox - xyA.x) + gy * (oy - xyA.y) - gz * zA;
+      out.begin(i0);
       for (int is = i0; is < i1; ++is) {
-        const int iz = (int)((unsigned)is / (unsigned)ss);
         const double zi = z0 + dzs * is + dzs / 2.;
-        cell_add(col + iz, (fixed + gz * zi) * w);
+        out.put(is, (fixed + gz * zi) * w);
       }
     }
   }
