@@ -171,18 +171,57 @@ __global__ void k_field64(const double4* __restrict__ pos, const int4* __restric
   out[t] = make_double4(a.w - gx * a.x - gy * a.y - gz * a.z, gx, gy, gz);
 }
 
+// The links of every (tet, entry face), in their three rotations
+// (tet_links.cuh): a thread per record, 48 contiguous bytes each.  A face
+// across which the two tets list other vertices or another orientation, or
+// whose neighbour is also the one behind the entry face (the walk would turn
+// around there), is left to the general step.
+__global__ void k_links(const int4* __restrict__ rows, int nt, uint4* __restrict__ link) {
+  const long long rec = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (rec >= 4LL * nt) return;
+  const int t = (int)(rec >> 2), F = (int)(rec & 3);
+  const int4 v = rows[2 * (size_t)t], nb = rows[2 * (size_t)t + 1];
+  const auto at = [](const int4& a, int k) { return k == 0 ? a.x : (k == 1 ? a.y : (k == 2 ? a.z : a.w)); };
+  const int from = at(nb, F);
+  uint32_t lk[3];
+  unsigned roles[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {  // leaving behind record slot k, through face m
+    const int m = rot_slot(F, k), n = at(nb, m);
+    lk[k] = kLinkGeneral;
+    roles[k] = exit_roles(F, k);
+    if (n < 0) {
+      lk[k] = kLinkHull;
+    } else if (n != from) {
+      const int4 w = rows[2 * (size_t)n], b = rows[2 * (size_t)n + 1];
+      const int f = b.x == t ? 0 : (b.y == t ? 1 : (b.z == t ? 2 : (b.w == t ? 3 : -1)));
+      if (f >= 0) {
+        const int u[3] = {at(v, rot_slot(F, (k + 1) % 3)), at(v, rot_slot(F, (k + 2) % 3)), at(v, F)};
+        const int ws[3] = {at(w, rot_slot(f, 0)), at(w, rot_slot(f, 1)), at(w, rot_slot(f, 2))};
+        const int r = link_rotation(u, ws);
+        if (r >= 0) {
+          lk[k] = 3u * (4u * (uint32_t)n + (uint32_t)f) + (uint32_t)r;
+          roles[k] |= entry_roles(f, r) << 4;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+    link[3 * (size_t)rec + r] =
+        make_uint4(lk[r], lk[(r + 1) % 3], lk[(r + 2) % 3],
+                   roles[r] | roles[(r + 1) % 3] << 8 | roles[(r + 2) % 3] << 16);
+}
+
 // Walk records for projection axis `axis`: positions and gradient permuted
-// cyclically.  The FP64 record carries rho_A, the gradient and the neighbour
-// links; the mixed walk's are one TetGeo32 per (tet, entry face) and, in
-// `link`, the three rotations of its links (walk32.cuh).
+// cyclically; the FP64 walk's TetRec64 per tet, the mixed walk's TetGeo32 per
+// (tet, entry face).
 __global__ void k_records(const double4* __restrict__ pos, const int4* __restrict__ rows,
                           const double* __restrict__ grad, int nt, int axis,
-                          TetRec64* __restrict__ r64, TetGeo32* __restrict__ geo,
-                          uint4* __restrict__ link) {
+                          TetRec64* __restrict__ r64, TetGeo32* __restrict__ geo) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   const int4 v = rows[2 * (size_t)t];
-  const int4 nb = rows[2 * (size_t)t + 1];
   double4 p[4] = {pos[v.x], pos[v.y], pos[v.z], pos[v.w]};
   double q[4][3];
 #pragma unroll
@@ -193,13 +232,8 @@ __global__ void k_records(const double4* __restrict__ pos, const int4* __restric
   if (r64) {
     TetRec64 r;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) r.xy[k] = make_double2(q[k][0], q[k][1]);
-    r.zab = make_double2(q[0][2], q[1][2]);
-    r.zcd = make_double2(q[2][2], q[3][2]);
-    r.rg0 = make_double2(p[0].w, g[0]);
-    r.rg1 = make_double2(g[1], g[2]);
-    r.nb = nb;
-    r.vid = v;
+    for (int k = 0; k < 4; ++k) r.v[k] = make_double4(q[k][0], q[k][1], q[k][2], 0.0);
+    r.f = make_double4(p[0].w, g[0], g[1], g[2]);
     r64[t] = r;
   }
   if (geo) {
@@ -238,46 +272,6 @@ __global__ void k_records(const double4* __restrict__ pos, const int4* __restric
       o[0] = make_float4((float)q[F][0], (float)q[F][1], (float)q[F][2], (float)p[F].w);
       o[1] = make_float4((float)g[0], (float)g[1], (float)g[2], trusted ? ext : INFINITY);
     }
-  }
-  if (link) {
-    const int vid[4] = {v.x, v.y, v.z, v.w}, nbo[4] = {nb.x, nb.y, nb.z, nb.w};
-    uint4* o = link + 12 * (size_t)t;
-    uint32_t lk[4][3];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {  // exit through face m, into neighbour n
-      const int n = nbo[m];
-      int4 w = make_int4(-1, -1, -1, -1);
-      int f = -1;
-      if (n >= 0) {
-        w = rows[2 * (size_t)n];
-        const int4 b = rows[2 * (size_t)n + 1];
-        f = b.x == t ? 0 : (b.y == t ? 1 : (b.z == t ? 2 : (b.w == t ? 3 : -1)));
-      }
-      const int wid[4] = {w.x, w.y, w.z, w.w};
-      int ws[3];  // the neighbour's entry face in its listed order
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const int sl = f >= 0 ? rot_slot(f, k) : 0;
-        ws[k] = sl == 0 ? wid[0] : (sl == 1 ? wid[1] : (sl == 2 ? wid[2] : wid[3]));
-      }
-#pragma unroll
-      for (int F = 0; F < 4; ++F) {  // entered through face F
-        if (F == m) continue;
-        const int k = rot_inv(F, m);  // record slot of the vertex left behind
-        const int u[3] = {vid[rot_slot(F, (k + 1) % 3)], vid[rot_slot(F, (k + 2) % 3)], vid[F]};
-        uint32_t L = n < 0 ? kLinkHull : kLinkGeneral;
-        if (f >= 0) {
-          const int r = link_rotation(u, ws);
-          if (r >= 0) L = 3u * (4u * (uint32_t)n + (uint32_t)f) + (uint32_t)r;
-        }
-        lk[F][k] = L;
-      }
-    }
-#pragma unroll
-    for (int F = 0; F < 4; ++F)
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-        o[3 * F + r] = make_uint4(lk[F][r], lk[F][(r + 1) % 3], lk[F][(r + 2) % 3], 0u);
   }
 }
 
@@ -604,9 +598,9 @@ dtfe_status_t mesh_field64(Mesh* m) {
   return DTFE_OK;
 }
 
-static void drop_mixed_records(AxisData& A, Mesh* m) {
-  dfree_async(A.geo32, 4 * (size_t)m->nt, m);
-  dfree_async(A.link32, 12 * (size_t)m->nt, m);
+static bool has_links(const Mesh& m) { return m.nt <= kMaxLinkedTets; }
+static size_t link_bytes(const Mesh& m) {
+  return has_links(m) ? kLinkRowsPerTet * sizeof(uint4) * (size_t)m.nt : 0;
 }
 
 dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32) {
@@ -616,29 +610,33 @@ dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32) {
   const bool need64 = want64 && !A.rec64, need32 = want32 && !A.geo32;
   if (!need64 && !need32) return DTFE_OK;
   // the mixed walk's records address 4*t + F in an int: up to 2^29 - 1 tets
-  const bool links = need32 && m->nt <= kMaxLinkedTets;
   if (need32 && m->nt >= (1 << 29))
     return set_error(DTFE_ERR_UNSUPPORTED, "mixed maps of %d tets (at most 2^29 - 1)", m->nt);
+  const bool links = !A.link && has_links(*m);
   // all or nothing: a record array that exists has been built; stream-ordered
   // allocations, so that building records for one mesh does not stall the
   // device (the serving loop builds and drops them while maps run)
   dtfe_status_t st = DTFE_OK;
   if (need64) st = dmalloc_async(&A.rec64, m->nt, m);
   if (st == DTFE_OK && need32) st = dmalloc_async(&A.geo32, 4 * (size_t)m->nt, m);
-  if (st == DTFE_OK && links) st = dmalloc_async(&A.link32, 12 * (size_t)m->nt, m);
+  if (st == DTFE_OK && links) st = dmalloc_async(&A.link, kLinkRowsPerTet * (size_t)m->nt, m);
   if (st == DTFE_OK && m->nt) {
     k_records<<<grid_for(m->nt), kBlock, 0, m->stream>>>(m->pos, m->rows, m->grad, m->nt, axis,
                                                          need64 ? A.rec64 : nullptr,
-                                                         need32 ? A.geo32 : nullptr,
-                                                         links ? A.link32 : nullptr);
+                                                         need32 ? A.geo32 : nullptr);
     count_launch();
+    if (links) {
+      k_links<<<grid_for(4LL * m->nt), kBlock, 0, m->stream>>>(m->rows, m->nt, A.link);
+      count_launch();
+    }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
       st = set_error(DTFE_ERR_CUDA, "walk records: %s", cudaGetErrorString(e));
   }
   if (st != DTFE_OK) {
     if (need64) dfree_async(A.rec64, m->nt, m);
-    if (need32) drop_mixed_records(A, m);
+    if (need32) dfree_async(A.geo32, 4 * (size_t)m->nt, m);
+    if (links) dfree_async(A.link, kLinkRowsPerTet * (size_t)m->nt, m);
     return st;
   }
   return DTFE_OK;
@@ -647,14 +645,16 @@ dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32) {
 size_t mesh_record_bytes(const Mesh& m, int axis) {
   const AxisData& A = m.ax[axis];
   const size_t nt = (size_t)m.nt;
-  return (A.geo32 ? mixed_record_bytes(m.nt) : 0) + (A.rec64 ? sizeof(TetRec64) * nt : 0);
+  return (A.geo32 ? 4 * sizeof(TetGeo32) * nt : 0) + (A.rec64 ? sizeof(TetRec64) * nt : 0) +
+         (A.link ? link_bytes(m) : 0);
 }
 
 size_t mesh_missing_record_bytes(const Mesh& m, int axis, int precision) {
   const AxisData& A = m.ax[axis];
   const size_t nt = (size_t)m.nt;
   size_t b = 0;
-  if (precision == DTFE_MIXED && !A.geo32) b += mixed_record_bytes(m.nt);
+  if (precision == DTFE_MIXED && !A.geo32) b += 4 * sizeof(TetGeo32) * nt;
+  if (!A.link) b += link_bytes(m);
   // the mixed walk reads FP64 records only when the coordinates are not floats
   const bool want64 = precision == DTFE_FP64 ||
                       (!m.fp32_exact && !(m.flags & DTFE_MESH_NO_FP64_REC));
@@ -666,8 +666,10 @@ size_t mesh_missing_record_bytes(const Mesh& m, int axis, int precision) {
 // ordered on the mesh stream.
 void mesh_drop_records(Mesh* m, int axis) {
   if (axis < 0 || axis > 2) return;
-  dfree_async(m->ax[axis].rec64, m->nt, m);
-  drop_mixed_records(m->ax[axis], m);
+  AxisData& A = m->ax[axis];
+  dfree_async(A.rec64, m->nt, m);
+  dfree_async(A.geo32, 4 * (size_t)m->nt, m);
+  dfree_async(A.link, kLinkRowsPerTet * (size_t)m->nt, m);
 }
 
 dtfe_status_t mesh_hull_mask(Mesh* m, int axis, uint32_t* host_mask_out, int* count_out) {
@@ -771,7 +773,8 @@ void mesh_free(Mesh* m) {
   // is then synchronised (the caller's own streams are done with the mesh)
   for (auto& A : m->ax) {
     dfree_async(A.rec64, m->nt, m);
-    drop_mixed_records(A, m);
+    dfree_async(A.geo32, 4 * (size_t)m->nt, m);
+    dfree_async(A.link, kLinkRowsPerTet * (size_t)m->nt, m);
   }
   dfree_async(m->fld64, m->nt, m);
   dfree_async(m->pos, m->n, m);

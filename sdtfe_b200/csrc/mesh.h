@@ -55,7 +55,7 @@ struct AxisData {
   // walk records in this axis' projected frame (built on demand, per precision)
   TetRec64* rec64 = nullptr;
   TetGeo32* geo32 = nullptr;  // 4 per tet (one per entry face): the mixed walk's records
-  uint4* link32 = nullptr;    // 12 per tet: their links (none beyond kMaxLinkedTets)
+  uint4* link = nullptr;      // 12 per tet: their links (none beyond kMaxLinkedTets)
 };
 
 struct Mesh {

@@ -19,8 +19,16 @@ namespace sdtfe {
 
 namespace {
 
+// Threads per block of the FP64 maps and the blocks per SM their registers
+// allow (96 a thread).  The walk waits on FP64 latencies, so warps count more
+// than the few spills around its out-of-line step: 131k clustered points, 512^2
+// x 16, while the walk still picked each crossing's operands: 2 x 256 threads of
+// 128 registers 10.03 ms, 4 x 128 9.77, 10 x 64 of 96 9.39, 12 x 64 of 80 10.7
+// (spills in the loop).  Blocks of two warps also lose less at the end-of-tile
+// barrier than blocks of eight.
+constexpr int kBlock64 = 64, kBlocks64 = 10;
+
 struct MapArgs64 {
-  const TetRec64* __restrict__ rec;
   const TriRec64* __restrict__ tri;
   int n_tri;
   double* __restrict__ map;
@@ -82,12 +90,12 @@ __device__ __forceinline__ void map_tile64(const MapArgs64& a, int tile, double*
       const double xt = x + sdtfe_sample_u01(a.walk.seed, (uint64_t)p, (uint32_t)s, 0) * a.scale;
       const double yt = y + sdtfe_sample_u01(a.walk.seed, (uint64_t)p, (uint32_t)s, 1) * a.scale;
       const uint64_t rid = (uint64_t)p * (uint64_t)a.S + (uint64_t)s;
-      int ft = -1;
-      if (a.loc) ft = locate_from_tile(a.tri, __ldg(a.loc + tile), xt, yt, a.loc_budget, &status);
-      else if (a.n_tri > 0) ft = locate64(a.tri, 0, xt, yt, a.loc_budget, &status);
+      int ft = -1, tri = -1;
+      if (a.loc) ft = locate_from_tile(a.tri, __ldg(a.loc + tile), xt, yt, a.loc_budget, &status, &tri);
+      else if (a.n_tri > 0) ft = locate64(a.tri, 0, xt, yt, a.loc_budget, &status, &tri);
       if (ft >= 0) {
         SurfaceAcc64 acc{a.offz, a.offz + a.lz, 0.0};
-        status = walk64(a.rec, ft, xt, yt, a.walk, rid, acc, &crossed, nullptr, 0);
+        status = walk64(a.walk, ft, tri, xt, yt, rid, acc, &crossed, nullptr, 0);
         if (status == kRayOk) v = acc.rho;
       }
       if (a.ray_rho) {
@@ -114,7 +122,7 @@ __device__ __forceinline__ void map_tile64(const MapArgs64& a, int tile, double*
   }
 }
 
-__global__ void __launch_bounds__(256) k_map64(const MapArgs64 a) {
+__global__ void __launch_bounds__(kBlock64, kBlocks64) k_map64(const MapArgs64 a) {
   extern __shared__ double s_val[];  // P*S doubles, then P*S bytes of success flags
   unsigned char* s_ok = reinterpret_cast<unsigned char*>(s_val + a.TW * a.TH * a.S);
   map_tile64(a, blockIdx.x, s_val, s_ok);
@@ -144,7 +152,7 @@ __device__ __forceinline__ void claim_tile64(const BatchJob64* __restrict__ jobs
   *job = lo;
 }
 
-__global__ void __launch_bounds__(256) k_batch64(const BatchJob64* __restrict__ jobs, int n_jobs,
+__global__ void __launch_bounds__(kBlock64, kBlocks64) k_batch64(const BatchJob64* __restrict__ jobs, int n_jobs,
                                                  long long total_tiles,
                                                  unsigned long long* __restrict__ queue) {
   extern __shared__ double s_val[];
@@ -174,8 +182,7 @@ __global__ void __launch_bounds__(256) k_batch64(const BatchJob64* __restrict__ 
   }
 }
 
-__global__ void __launch_bounds__(128) k_trace64(const TetRec64* __restrict__ rec,
-                                                 const TriRec64* __restrict__ tri, int n_tri,
+__global__ void __launch_bounds__(128) k_trace64(const TriRec64* __restrict__ tri, int n_tri,
                                                  int n_rays, const double* __restrict__ xs,
                                                  const double* __restrict__ ys, double z0,
                                                  WalkConf64 walk, int loc_budget,
@@ -186,10 +193,11 @@ __global__ void __launch_bounds__(128) k_trace64(const TetRec64* __restrict__ re
   if (i >= n_rays) return;
   int st = kRayMiss, c = 0;
   double v = 0.0;
-  const int ft = n_tri > 0 ? locate64(tri, 0, xs[i], ys[i], loc_budget, &st) : -1;
+  int ft_tri = -1;
+  const int ft = n_tri > 0 ? locate64(tri, 0, xs[i], ys[i], loc_budget, &st, &ft_tri) : -1;
   if (ft >= 0) {
     SurfaceAcc64 acc{z0, z0 + walk.lz, 0.0};
-    st = walk64(rec, ft, xs[i], ys[i], walk, (uint64_t)i, acc, &c,
+    st = walk64(walk, ft, ft_tri, xs[i], ys[i], (uint64_t)i, acc, &c,
                 visits ? visits + (size_t)i * max_record : nullptr, max_record);
     if (st == kRayOk) v = acc.rho;
   }
@@ -199,7 +207,6 @@ __global__ void __launch_bounds__(128) k_trace64(const TetRec64* __restrict__ re
 }
 
 struct GridArgs64 {
-  const TetRec64* __restrict__ rec;
   const TriRec64* __restrict__ tri;
   int n_tri, G, ss, loc_budget;
   double dxy, offx, offy, offz, dzs, w;
@@ -215,12 +222,12 @@ __device__ __forceinline__ int grid_ray64(const GridArgs64& a, int i, int j, int
   const double ds = a.dxy / a.ss;
   const double x = i * a.dxy + a.offx + is * ds + ds / 2.;
   const double y = j * a.dxy + a.offy + js * ds + ds / 2.;
-  int st = kRayMiss;
+  int st = kRayMiss, ft_tri = -1;
   *crossed = 0;
-  const int ft = a.n_tri > 0 ? locate64(a.tri, 0, x, y, a.loc_budget, &st) : -1;
+  const int ft = a.n_tri > 0 ? locate64(a.tri, 0, x, y, a.loc_budget, &st, &ft_tri) : -1;
   if (ft < 0) return st;
   const uint64_t rid = (((uint64_t)i * a.G + j) * a.ss + (uint64_t)is) * a.ss + (uint64_t)js;
-  return walk64(a.rec, ft, x, y, a.walk, rid, acc, crossed, nullptr, 0);
+  return walk64(a.walk, ft, ft_tri, x, y, rid, acc, crossed, nullptr, 0);
 }
 
 // One thread per grid column (i, j); its ss^2 sub-rays run in (is, js) order
@@ -290,9 +297,9 @@ MapGeom map_geometry(const Mesh& m, const dtfe_map_params_t& p) {
   return g;
 }
 
-// tile of pixels per block: TW x TH pixels x S samples <= 256 threads
+// tile of pixels per block: TW x TH pixels x S samples <= kBlock64 threads
 static void tile_shape(int S, int* TW, int* TH) {
-  int P = 256 / S;
+  int P = kBlock64 / S;
   if (P < 1) P = 1;
   int lg = 31 - __builtin_clz((unsigned)P);
   int tw = 1 << ((lg + 1) / 2);
@@ -302,6 +309,12 @@ static void tile_shape(int S, int* TW, int* TH) {
   *TH = th;
 }
 
+static WalkConf64 walk_conf64(const Mesh& m, int axis, double lz, double dist, uint64_t seed,
+                              int max_visits) {
+  const AxisData& A = m.ax[axis];
+  return WalkConf64{lz, dist, seed, max_visits, A.rec64, m.rows, A.link, A.tri_face};
+}
+
 // The kernel arguments of one FP64 map; *tiles_y receives its rows of tiles.
 static dtfe_status_t map_args64(Mesh& m, const MapGeom& g, double* d_map,
                                 unsigned long long* stats, double* ray_rho, int* ray_crossed,
@@ -309,7 +322,6 @@ static dtfe_status_t map_args64(Mesh& m, const MapGeom& g, double* d_map,
   const AxisData& A = m.ax[g.axis];
   if (!A.rec64 || !A.hull_built) return set_error(DTFE_ERR_INVALID, "FP64 map before its records");
   MapArgs64& a = *out;
-  a.rec = A.rec64;
   a.tri = A.tri;
   a.n_tri = A.n_tri;
   a.map = d_map;
@@ -325,7 +337,7 @@ static dtfe_status_t map_args64(Mesh& m, const MapGeom& g, double* d_map,
   a.lz = g.lz;
   a.scale = g.scale;
   a.soff = g.soff;
-  a.walk = WalkConf64{g.lz, g.dist, g.seed, g.max_visits};
+  a.walk = walk_conf64(m, g.axis, g.lz, g.dist, g.seed, g.max_visits);
   a.loc_budget = 4 * A.n_tri + 64;
   a.loc = nullptr;
   a.stats = stats;
@@ -342,7 +354,7 @@ dtfe_status_t launch_map64(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
   SDTFE_TRY(map_args64(m, g, d_map, m.stats, ray_rho, ray_crossed, ray_status, &a, &tiles_y));
   const int P = a.TW * a.TH;
   int threads = P * g.S;
-  threads = threads > 256 ? 256 : ((threads + 31) / 32) * 32;
+  threads = threads > kBlock64 ? kBlock64 : ((threads + 31) / 32) * 32;
   const size_t smem = (size_t)P * g.S * (sizeof(double) + 1);
   if (smem > 48 * 1024)
     SDTFE_CUDA(cudaFuncSetAttribute(k_map64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -414,10 +426,10 @@ dtfe_status_t batch_grid64(size_t smem, int* grid, int* block) {
   SDTFE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (smem > 48 * 1024)
     SDTFE_CUDA(cudaFuncSetAttribute(k_batch64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  SDTFE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch64, 256, smem));
+  SDTFE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch64, kBlock64, smem));
   if (per_sm < 1) return set_error(DTFE_ERR_UNSUPPORTED, "FP64 batch: %zu B of shared memory per block", smem);
   *grid = per_sm * sms;
-  *block = 256;
+  *block = kBlock64;
   return DTFE_OK;
 }
 
@@ -426,7 +438,7 @@ dtfe_status_t launch_batch64(const BatchPlan& plan, const void* d_jobs, unsigned
   if (plan.n_jobs == 0) return DTFE_OK;
   if (plan.smem > 48 * 1024)
     SDTFE_CUDA(cudaFuncSetAttribute(k_batch64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
-  k_batch64<<<grid, 256, plan.smem, s>>>(static_cast<const BatchJob64*>(d_jobs), plan.n_jobs,
+  k_batch64<<<grid, kBlock64, plan.smem, s>>>(static_cast<const BatchJob64*>(d_jobs), plan.n_jobs,
                                          plan.total_tiles, d_queue);
   count_launch();
   SDTFE_CUDA(cudaGetLastError());
@@ -439,9 +451,9 @@ dtfe_status_t launch_trace64(Mesh& m, int axis, int n_rays, const double* d_x, c
                              int max_record, cudaStream_t s) {
   const AxisData& A = m.ax[axis];
   if (!A.rec64 || !A.hull_built) return set_error(DTFE_ERR_INVALID, "FP64 trace before its records");
-  WalkConf64 w{lz, (dxy / 2.0) / kPerturbMax, seed, max_visits};
+  const WalkConf64 w = walk_conf64(m, axis, lz, (dxy / 2.0) / kPerturbMax, seed, max_visits);
   if (n_rays > 0) {
-    k_trace64<<<(n_rays + 127) / 128, 128, 0, s>>>(A.rec64, A.tri, A.n_tri, n_rays, d_x, d_y, z0, w,
+    k_trace64<<<(n_rays + 127) / 128, 128, 0, s>>>(A.tri, A.n_tri, n_rays, d_x, d_y, z0, w,
                                                    4 * A.n_tri + 64, d_rho, d_crossed, d_status,
                                                    d_visits, max_record);
     count_launch();
@@ -455,7 +467,6 @@ dtfe_status_t launch_grid64(Mesh& m, int G, double box_len, const double center[
   const AxisData& A = m.ax[DTFE_AXIS_Z];
   if (!A.rec64 || !A.hull_built) return set_error(DTFE_ERR_INVALID, "grid before its records");
   GridArgs64 a;
-  a.rec = A.rec64;
   a.tri = A.tri;
   a.n_tri = A.n_tri;
   a.G = G;
@@ -468,7 +479,7 @@ dtfe_status_t launch_grid64(Mesh& m, int G, double box_len, const double center[
   a.offz = -(box_len / 2.0) + center[2];
   a.dzs = box_len / G / a.ss;
   a.w = 1. / (ss * ss * ss);
-  a.walk = WalkConf64{box_len, (a.dxy / 2.0) / kPerturbMax, seed, max_visits};
+  a.walk = walk_conf64(m, DTFE_AXIS_Z, box_len, (a.dxy / 2.0) / kPerturbMax, seed, max_visits);
   a.grid = d_grid;
   a.stats = m.stats;
   SDTFE_CUDA(cudaMemsetAsync(m.stats, 0, sizeof(unsigned long long) * kStatCount, s));

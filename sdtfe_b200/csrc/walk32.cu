@@ -153,15 +153,15 @@ __device__ __forceinline__ double2 xy64_at(const TetGeo32* __restrict__ R32,
     const float4 a = vertex32(R32, t, k);
     return make_double2(a.x, a.y);
   }
-  return __ldg(&R64[t].xy[k]);
+  const double4 v = load256(&R64[t].v[k]);
+  return make_double2(v.x, v.y);
 }
 
 __device__ __forceinline__ double z64_at(const TetGeo32* __restrict__ R32,
                                          const TetRec64* __restrict__ R64, int exact32, int t,
                                          int k) {
   if (exact32) return (double)vertex32(R32, t, k).z;
-  const double2 zz = __ldg(k < 2 ? &R64[t].zab : &R64[t].zcd);
-  return (k & 1) ? zz.y : zz.x;
+  return load256(&R64[t].v[k]).z;
 }
 
 // The reference's FP64 product for edge P->Q, operands and order as in
@@ -1404,7 +1404,7 @@ MixConf mix_conf(const Mesh& m, int axis, double z0, double lz, double dist, uin
   C.rec64 = m.ax[axis].rec64;
   C.exact32 = m.fp32_exact ? 1 : 0;
   C.geo = m.ax[axis].geo32;
-  C.link = m.ax[axis].link32;
+  C.link = m.ax[axis].link;
   C.tri_face = m.ax[axis].tri_face;
   C.rows = m.rows;
   C.pos = m.pos;

@@ -8,10 +8,10 @@
 // the walk therefore visits the same tets and returns the same doubles.
 //
 // Data layout (built by mesh.cu):
-//   TetRec64  160 B per tet: the (x, y) and z of its four vertices in the
-//             projected frame, rho_A, the gradient and the neighbour links.
-//             One walk step reads one record: the next tet id and everything
-//             the Plücker test and the integral need arrive together.
+//   TetRec64  160 B per tet: its four vertices in the projected frame, rho_A
+//             and the gradient; three 256-bit loads a step (the vertex not yet
+//             seen, vertex A and the field).
+//   links     16 B per (tet, entry face, rotation): tet_links.cuh.
 //   TriRec64   64 B per projected hull triangle: (x, y) of its corners, the
 //             three edge neighbours and the tet under it.
 #pragma once
@@ -19,6 +19,7 @@
 #include <cstdint>
 
 #include "sdtfe_rng.h"
+#include "tet_links.cuh"
 
 namespace sdtfe {
 
@@ -36,13 +37,8 @@ enum RayStatus : int {
 };
 
 struct __align__(32) TetRec64 {
-  double2 xy[4];  // vertices A..D in the projected frame
-  double2 zab;    // (z_A, z_B)
-  double2 zcd;    // (z_C, z_D)
-  double2 rg0;    // (rho_A, grad_x)
-  double2 rg1;    // (grad_y, grad_z)
-  int4 nb;        // neighbours across faces BDC, ACD, ADB, ABC (-1: hull)
-  int4 vid;       // vertex ids A..D
+  double4 v[4];  // vertices A..D in the projected frame (w unused)
+  double4 f;     // rho_A, grad_x, grad_y, grad_z
 };
 static_assert(sizeof(TetRec64) == 160, "TetRec64 layout");
 
@@ -52,8 +48,17 @@ struct __align__(16) TriRec64 {
 };
 static_assert(sizeof(TriRec64) == 64, "TriRec64 layout");
 
+// 32 B in one load
+__device__ __forceinline__ double4 load256(const double4* p) {
+  double4 v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+      : "l"(p));
+  return v;
+}
+
 template <class T>
-__device__ __forceinline__ T sel4(int k, T a, T b, T c, T d) {
+__host__ __device__ __forceinline__ T sel4(int k, T a, T b, T c, T d) {
   return k == 0 ? a : (k == 1 ? b : (k == 2 ? c : d));
 }
 
@@ -116,7 +121,7 @@ __device__ __forceinline__ Hit64 plucker_faces(const int s[6]) {
 
 // z of the point where the ray crosses face f: the face normaliser is summed
 // in the reference's order, then ((1 - w1) - w2)*z0 + w1*z1 + w2*z2.
-__device__ __forceinline__ double face_z64(int f, const double u[6], const double z[4]) {
+__host__ __device__ __forceinline__ double face_z64(int f, const double u[6], const double z[4]) {
   const double a0 = sel4(f, -u[0], u[1], u[5], u[2]);
   const double a1 = sel4(f, u[3], -u[3], u[4], u[0]);
   const double a2 = sel4(f, -u[4], -u[5], -u[2], -u[1]);
@@ -342,14 +347,19 @@ __device__ __forceinline__ int locate_from_tile(const TriRec64* __restrict__ tri
 struct SurfaceAcc64 {
   double z0, z1;
   double rho;
-  __device__ __forceinline__ void visit(double ox, double oy, const double2& xyA, double zA,
-                                        double rhoA, double gx, double gy, double gz, double z_in,
+  // what visit() reads of a tet's record, loaded ahead of it
+  struct Field {
+    double4 A, f;
+    __device__ __forceinline__ explicit Field(const TetRec64* __restrict__ t)
+        : A(load256(&t->v[0])), f(load256(&t->f)) {}
+  };
+  __device__ __forceinline__ void visit(double ox, double oy, const Field& t, double z_in,
                                         double z_out) {
     const double d = z_out - z_in;
     const double zm = d / 2 + z_in;
     if (zm > z0 && zm < z1) {
-      const double fixed = rhoA + (gx * (ox - xyA.x)) + (gy * (oy - xyA.y)) - (gz * zA);
-      rho += (fixed + gz * zm) * d;
+      const double fixed = t.f.x + (t.f.y * (ox - t.A.x)) + (t.f.z * (oy - t.A.y)) - (t.f.w * t.A.z);
+      rho += (fixed + t.f.w * zm) * d;
     }
   }
 };
@@ -385,19 +395,24 @@ struct ColumnAcc64 {
   Sink out;
   double z0, dzs, w;
   int nzs;
-  __device__ __forceinline__ void visit(double ox, double oy, const double2& xyA, double zA,
-                                        double rhoA, double gx, double gy, double gz, double z_in,
+  // most chords of a fine mesh hold no node: the record is read when one does
+  struct Field {
+    const TetRec64* __restrict__ t;
+    __device__ __forceinline__ explicit Field(const TetRec64* __restrict__ p) : t(p) {}
+  };
+  __device__ __forceinline__ void visit(double ox, double oy, const Field& r, double z_in,
                                         double z_out) {
     int i0 = (int)ceil((z_in - z0 - dzs / 2.) / dzs);
     i0 = i0 < 0 ? 0 : i0;
     int i1 = (int)ceil((z_out - z0 - dzs / 2.) / dzs);
     i1 = i1 > nzs ? nzs : i1;
     if (i1 > i0) {
-      const double fixed = rhoA + gx * (ox - xyA.x) + gy * (oy - xyA.y) - gz * zA;
+      const double4 A = load256(&r.t->v[0]), f = load256(&r.t->f);
+      const double fixed = f.x + f.y * (ox - A.x) + f.z * (oy - A.y) - f.w * A.z;
       out.begin(i0);
       for (int is = i0; is < i1; ++is) {
         const double zi = z0 + dzs * is + dzs / 2.;
-        out.put(is, (fixed + gz * zi) * w);
+        out.put(is, (fixed + f.w * zi) * w);
       }
     }
   }
@@ -408,85 +423,274 @@ struct WalkConf64 {
   double dist;      // perturbation step (delta_xy/2)/PERTURB_MAX
   uint64_t seed;    // perturbation stream key
   int max_visits;   // visit budget
+  const TetRec64* __restrict__ rec;
+  const int4* __restrict__ rows;             // tetra_data rows (vertex ids, neighbours)
+  const uint4* __restrict__ link;            // links (NULL: general steps only)
+  const signed char* __restrict__ tri_face;  // the tet face under each hull triangle
 };
 
 // ---------------------------------------------------------------------------
-// a9 + a10: the tet walk (src/dtfe.c:247-374).  On failure *crossed_out stays 0
-// and the status says why; column accumulators keep what they already added,
-// as evaluate_3d_ray_on_grid does.  Starts as if it had just left
-// a virtual tet through face 0 into `ft`; follows the neighbour across the
-// leave face; turns around (swaps enter and leave) when that neighbour is the
-// tet it came from; perturbs the ray towards a generator-chosen corner while
-// a chosen face has a zero edge sign.
+// a9 + a10: the tet walk (src/dtfe.c:247-374).  On failure the crossing count
+// stays 0 and the status says why; column accumulators keep what they already
+// added, as evaluate_3d_ray_on_grid does.  The walk follows the neighbour
+// across the leave face, turns around (swaps enter and leave) when that
+// neighbour is the tet it came from, and perturbs the ray towards a
+// generator-chosen corner while a chosen face has a zero edge sign.
+//
+// Two kinds of step, as in the mixed walk (walk32.cu).  The fast step knows the
+// face the ray came in through and carries its triangle; the general step
+// takes a tet in the mesh's vertex order and decides everything from its six
+// products.
+
+constexpr int kWalk64On = -1;  // the walk continues
+
+// A walk between steps, for the general step.
 template <class Acc>
-__device__ __forceinline__ int walk64(const TetRec64* __restrict__ R, int ft, double ox, double oy,
-                                      const WalkConf64& W, uint64_t ray, Acc& acc, int* crossed_out,
-                                      int* visits, int max_record) {
+struct Walk64 {
+  double ox, oy;
+  uint64_t ray, ctr;  // perturbation stream and draws so far
+  Acc acc;
+  int crossed, cur, prev;
+  int rec;            // cur's record for its entry face (-1: not known)
+};
+
+template <class Acc>
+__device__ __noinline__ int general_step64(const WalkConf64& W, Walk64<Acc>& w, int* visits,
+                                           int max_record) {
+  if (w.crossed >= W.max_visits) return kRayBudget;
+  const TetRec64* rec = W.rec + w.cur;
+  double2 xy[4];
+  double z[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double4 v = load256(&rec->v[k]);
+    xy[k] = make_double2(v.x, v.y);
+    z[k] = v.z;
+  }
+  const int4 nb = __ldg(&W.rows[2 * (size_t)w.cur + 1]);
+  Ray64 ry{W.lz, -W.lz * w.oy, W.lz * w.ox};
+  double u[6];
+  Hit64 h = ray_tet64(ry, xy, u);
+  if (!h.ok) return kRayNoExit;
+  int np = 0;
+  while (h.special) {  // src/dtfe.c:329-349, perturb_ray at :219-245
+    const int r = sdtfe_rand31(W.seed, w.ray, w.ctr++) % 4;
+    const double2 vr = sel4(r, xy[0], xy[1], xy[2], xy[3]);
+    double dx = vr.x - w.ox;
+    double dy = vr.y - w.oy;
+    const double mag = sqrt(dx * dx + dy * dy);
+    if (mag > W.dist) {
+      dx = dx / mag;
+      dy = dy / mag;
+      dx = dx * W.dist;
+      dy = dy * W.dist;
+    }
+    w.ox = w.ox + dx;
+    w.oy = w.oy + dy;
+    ry.m_oy = -W.lz * w.oy;
+    ry.ox_l = W.lz * w.ox;
+    if (++np > kPerturbMax) return kRayPerturbMax;
+    h = ray_tet64(ry, xy, u);
+    if (!h.ok) return kRayNoExit;
+  }
+  const double z_in = face_z64(h.enter, u, z);
+  const double z_out = face_z64(h.leave, u, z);
+  if (visits != nullptr && w.crossed < max_record) visits[w.crossed] = w.cur;
+  ++w.crossed;
+  w.acc.visit(w.ox, w.oy, typename Acc::Field(rec), z_in, z_out);
+  int m = h.leave;
+  int nx = nb_at(nb, m);
+  if (nx == -1) return kRayOk;
+  if (nx == w.prev) {  // turn around
+    m = h.enter;
+    nx = nb_at(nb, m);
+    if (nx == -1) return kRayOk;
+  }
+  w.rec = -1;
+  if (W.link) {
+    const int G = m == 0 ? 1 : 0;  // a record of cur whose entry face is not m
+    const uint4 lk = __ldg(W.link + 3 * (4 * (size_t)w.cur + G));
+    const int k = rot_inv(G, m);
+    const uint32_t L = k == 0 ? lk.x : (k == 1 ? lk.y : lk.z);
+    if (L <= kLinkLast) w.rec = (int)(L / 3u);
+  }
+  w.prev = w.cur;
+  w.cur = nx;
+  return kWalk64On;
+}
+
+// The triangle a fast walk carries: the face the ray last crossed and its
+// cyclic products U(0,1), U(1,2), U(2,0) (edge_u64), all below -kZero.
+struct Tri64 {
+  double x0, y0, z0, x1, y1, z1, x2, y2, z2;
+  double e01, e12, e20;
+};
+
+// z where the ray crosses a carried triangle, as the face_z64 of the face in
+// the given roles (tet_links.cuh): n0..n2 are the products opposite slots
+// 0..2, sum their sum with the right one added last (product_sums), and the
+// corners follow in state order (an entry) or against it (an exit).  The sign
+// of all three products cancels.  The point is formed for each slot as corner 0
+// and then picked: 12 FP64 operations more than picking the five operands, but
+// 16 selects and a dozen registers less.
+struct ProductSums {
+  double last0, last1, last2;  // by the slot whose product is added last
+};
+__host__ __device__ __forceinline__ ProductSums product_sums(double n0, double n1, double n2) {
+  return {n1 + n2 + n0, n0 + n2 + n1, n0 + n1 + n2};
+}
+
+template <bool Exit>
+__host__ __device__ __forceinline__ double crossing64(double n0, double n1, double n2, double z0,
+                                                      double z1, double z2, const ProductSums& s,
+                                                      unsigned roles) {
+  const bool f0 = (roles & 3u) == 0u, f1 = (roles & 3u) == 1u;   // corner 0's slot (else 2)
+  const bool l0 = (roles & 12u) == 0u, l2 = (roles & 12u) == 8u;  // the last added (else 1)
+  const double sum = l0 ? s.last0 : (l2 ? s.last2 : s.last1);
+  const double inv = 1.0 / sum;
+  const double w0 = n0 * inv, w1 = n1 * inv, w2 = n2 * inv;
+  const double m0 = w0 * z0, m1 = w1 * z1, m2 = w2 * z2;
+  const double c0 = Exit ? (1 - w2 - w1) * z0 + m2 + m1 : (1 - w1 - w2) * z0 + m1 + m2;
+  const double c1 = Exit ? (1 - w0 - w2) * z1 + m0 + m2 : (1 - w2 - w0) * z1 + m2 + m0;
+  const double c2 = Exit ? (1 - w1 - w0) * z2 + m1 + m0 : (1 - w0 - w1) * z2 + m0 + m1;
+  return f0 ? c0 : (f1 ? c1 : c2);
+}
+
+// The triangle of record rec's entry face, in the record's order, and the
+// ray's crossing of it.  False when its products are not all below -kZero:
+// the general step takes the tet.
+__device__ __forceinline__ bool entry_triangle64(const WalkConf64& W, const Ray64& r, int rec,
+                                                 Tri64* s, double* z_in) {
+  const int F = rec & 3;
+  const TetRec64* t = W.rec + (rec >> 2);
+  const double4 a = load256(&t->v[rot_slot(F, 0)]), b = load256(&t->v[rot_slot(F, 1)]),
+                c = load256(&t->v[rot_slot(F, 2)]);
+  s->x0 = a.x;
+  s->y0 = a.y;
+  s->z0 = a.z;
+  s->x1 = b.x;
+  s->y1 = b.y;
+  s->z1 = b.z;
+  s->x2 = c.x;
+  s->y2 = c.y;
+  s->z2 = c.z;
+  s->e01 = edge_u64(r, make_double2(a.x, a.y), make_double2(b.x, b.y));
+  s->e12 = edge_u64(r, make_double2(b.x, b.y), make_double2(c.x, c.y));
+  s->e20 = edge_u64(r, make_double2(c.x, c.y), make_double2(a.x, a.y));
+  *z_in = crossing64<false>(s->e12, s->e20, s->e01, a.z, b.z, c.z,
+                             product_sums(s->e12, s->e20, s->e01), entry_roles(F, 0));
+  return s->e01 < -kZero && s->e12 < -kZero && s->e20 < -kZero;
+}
+
+// The walk of one ray from the tet ft, located under hull triangle ft_tri (-1:
+// not known), whose face the ray comes in through.
+//
+// The fast step.  Of the tet's six products (src/dtfe.c:44-64) the entry
+// face's three are the previous step's, up to the exact sign that the
+// reference's formula gives a reversed edge; the apex V adds a_k = U(V, P_k).
+// When all three are clear of kZero the reference enters through the known
+// face and leaves through the one without P_k, a_{k+1} < 0 < a_{k+2} (walk32.cu
+// proves the rule).  The exit crossing and the next tet's entry crossing are
+// the same point of the same triangle, each computed in the order the
+// reference computes it for that face of that tet (crossing64).
+//
+// What bounds it: latency, with the FP64 and the ALU pipe each near half of
+// their rate (56 % issue at 16 to 20 warps per SM; about 270 warp instructions
+// a visit, a third of them FP64).  All six products in the mesh's order, the
+// face rule on their signs and each face's operands picked by its index took
+// 456, at 24 of 32 lanes.  131k clustered points, 512^2 x 16: 15.7 -> 8.8 ms;
+// 32k uniform points, 256^2 x 4: 0.864 -> 0.549 ms.  Measured and not kept: the
+// field's record read only when the midpoint is known (2 to 8 % slower), its
+// constant part formed before the crossing (5 % slower), the next vertex and
+// links fetched a step ahead in grids (1 to 6 % slower).
+template <class Acc>
+__device__ __forceinline__ int walk64(const WalkConf64& W, int ft, int ft_tri, double ox, double oy,
+                                      uint64_t ray, Acc& acc, int* crossed_out, int* visits,
+                                      int max_record) {
   *crossed_out = 0;
   if (ft < 0) return kRayMiss;
-  Ray64 ry{W.lz, -W.lz * oy, W.lz * ox};
-  uint64_t ctr = 0;
-  int crossed = 0;
-  int4 nb = make_int4(ft, -1, -1, -1);
-  int leave = 0, enter = -1;
-  int cur = ft, prev = -1;
-  for (;;) {
-    int nx = nb_at(nb, leave);
-    if (nx == -1) break;
-    if (nx == prev) {  // turn around
-      const int t = enter;
-      enter = leave;
-      leave = t;
-      nx = nb_at(nb, leave);
-      if (nx == -1) break;
-    }
-    prev = cur;
-    cur = nx;
-    if (crossed >= W.max_visits) return kRayBudget;
-
-    const TetRec64* rec = R + cur;
-    double2 xy[4];
-    xy[0] = __ldg(&rec->xy[0]);
-    xy[1] = __ldg(&rec->xy[1]);
-    xy[2] = __ldg(&rec->xy[2]);
-    xy[3] = __ldg(&rec->xy[3]);
-    const double2 zab = __ldg(&rec->zab), zcd = __ldg(&rec->zcd);
-    const double2 rg0 = __ldg(&rec->rg0), rg1 = __ldg(&rec->rg1);
-    nb = __ldg(&rec->nb);
-    const double z[4] = {zab.x, zab.y, zcd.x, zcd.y};
-
-    double u[6];
-    Hit64 h = ray_tet64(ry, xy, u);
-    if (!h.ok) return kRayNoExit;
-    int np = 0;
-    while (h.special) {  // src/dtfe.c:329-349, perturb_ray at :219-245
-      const int r = sdtfe_rand31(W.seed, ray, ctr++) % 4;
-      const double2 vr = sel4(r, xy[0], xy[1], xy[2], xy[3]);
-      double dx = vr.x - ox;
-      double dy = vr.y - oy;
-      const double mag = sqrt(dx * dx + dy * dy);
-      if (mag > W.dist) {
-        dx = dx / mag;
-        dy = dy / mag;
-        dx = dx * W.dist;
-        dy = dy * W.dist;
+  Walk64<Acc> w;
+  w.ox = ox;
+  w.oy = oy;
+  w.ray = ray;
+  w.ctr = 0;
+  w.crossed = 0;
+  w.cur = ft;
+  w.prev = ft;  // (the reference's walk starts as if it had come from ft itself)
+  w.rec = W.link && ft_tri >= 0 ? 4 * ft + W.tri_face[ft_tri] : -1;
+  Ray64 r{W.lz, -W.lz * oy, W.lz * ox};
+  Tri64 s;
+  double z_in = 0.0;
+  uint32_t L = 3u * (uint32_t)w.rec;
+  int crossed = 0, status = kWalk64On;
+  bool fast = w.rec >= 0 && entry_triangle64(W, r, w.rec, &s, &z_in);
+  while (status == kWalk64On) {
+    if (fast) {
+      const uint32_t rec = L / 3u;
+      const TetRec64* t = W.rec + (rec >> 2);
+      const double4 V = load256(&t->v[rec & 3u]);
+      const uint4 lk = __ldg(W.link + L);
+      const typename Acc::Field field(t);
+      const double2 v = make_double2(V.x, V.y);
+      const double a0 = edge_u64(r, v, make_double2(s.x0, s.y0));
+      const double a1 = edge_u64(r, v, make_double2(s.x1, s.y1));
+      const double a2 = edge_u64(r, v, make_double2(s.x2, s.y2));
+      const bool sure = (fabs(a0) > kZero) & (fabs(a1) > kZero) & (fabs(a2) > kZero);
+      // (a_0, a_1, a_2 are not all of one sign)
+      const bool p2 = a2 > 0.0;
+      const bool k0 = p2 & (a1 < 0.0), k1 = !p2 & (a0 > 0.0);  // else k = 2
+      const auto pick = [k0, k1](auto a, auto b, auto c) { return k0 ? a : (k1 ? b : c); };
+      const uint32_t next = pick(lk.x, lk.y, lk.z);
+      if (sure & (next != kLinkGeneral) & (crossed < W.max_visits)) {
+        const unsigned roles = lk.w >> pick(0u, 8u, 16u);
+        // the exit face: slots i = k+1, j = k+2 (mod 3) and the apex
+        const double xi = pick(s.x1, s.x2, s.x0), yi = pick(s.y1, s.y2, s.y0);
+        const double xj = pick(s.x2, s.x0, s.x1), yj = pick(s.y2, s.y0, s.y1);
+        const double zi = pick(s.z1, s.z2, s.z0), zj = pick(s.z2, s.z0, s.z1);
+        const double ei = pick(a1, a2, a0), ej = -pick(a2, a0, a1);
+        s.e01 = pick(s.e12, s.e20, s.e01);
+        s.e12 = ej;
+        s.e20 = ei;
+        s.x0 = xi;
+        s.y0 = yi;
+        s.z0 = zi;
+        s.x1 = xj;
+        s.y1 = yj;
+        s.z1 = zj;
+        s.x2 = V.x;
+        s.y2 = V.y;
+        s.z2 = V.z;
+        const ProductSums sums = product_sums(s.e12, s.e20, s.e01);
+        const double z_out =
+            crossing64<true>(s.e12, s.e20, s.e01, s.z0, s.z1, s.z2, sums, roles);
+        if (visits != nullptr && crossed < max_record) visits[crossed] = (int)(rec >> 2);
+        ++crossed;
+        acc.visit(ox, oy, field, z_in, z_out);
+        if (next == kLinkHull) {
+          status = kRayOk;
+          break;
+        }
+        z_in = crossing64<false>(s.e12, s.e20, s.e01, s.z0, s.z1, s.z2, sums, roles >> 4);
+        L = next;
+        continue;
       }
-      ox = ox + dx;
-      oy = oy + dy;
-      ry.m_oy = -W.lz * oy;
-      ry.ox_l = W.lz * ox;
-      if (++np > kPerturbMax) return kRayPerturbMax;
-      h = ray_tet64(ry, xy, u);
-      if (!h.ok) return kRayNoExit;
+      w.cur = (int)(rec >> 2);
+      w.prev = crossed > 0 ? nb_at(__ldg(&W.rows[2 * (size_t)w.cur + 1]), (int)(rec & 3u)) : w.cur;
     }
-    enter = h.enter;
-    leave = h.leave;
-    const double z_in = face_z64(enter, u, z);
-    const double z_out = face_z64(leave, u, z);
-    if (visits != nullptr && crossed < max_record) visits[crossed] = cur;
-    ++crossed;
-    acc.visit(ox, oy, xy[0], z[0], rg0.x, rg0.y, rg1.x, rg1.y, z_in, z_out);
+    w.acc = acc;
+    w.crossed = crossed;
+    status = general_step64(W, w, visits, max_record);
+    acc = w.acc;
+    crossed = w.crossed;
+    if (status != kWalk64On) break;
+    ox = w.ox;
+    oy = w.oy;
+    r.m_oy = -W.lz * oy;
+    r.ox_l = W.lz * ox;
+    fast = w.rec >= 0 && entry_triangle64(W, r, w.rec, &s, &z_in);
+    L = 3u * (uint32_t)w.rec;
   }
+  if (status != kRayOk) return status;
   *crossed_out = crossed;
   return kRayOk;
 }
