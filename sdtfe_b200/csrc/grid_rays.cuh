@@ -46,7 +46,7 @@ struct NodeSink {
 
 // A grid's sub-rays.
 struct GridRays {
-  int G, ss;
+  int G, ss, lanes;  // lanes: rays a warp walks
   double* nodes;  // row (i*G + j)*ss^2 + is*ss + js of G*ss nodes
   int* col;       // per column: bit k for a ray of status k, and kIrregular
 };
@@ -61,18 +61,20 @@ __device__ __forceinline__ int worst_status(int marks) {
 __device__ __forceinline__ bool ray_of_grid(const GridRays& a, int* i, int* j, int* is, int* js) {
   const int nf = a.G * a.ss;  // fine columns a side
   const int warp = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
-  const int tiles_j = (nf + 7) >> 3;
+  const int pi = patch_rows(a.lanes), pj = patch_cols(a.lanes);
+  const int tiles_j = (nf + pj - 1) / pj;
   const int lane = (int)threadIdx.x & 31;
-  const int fi = (warp / tiles_j) * 4 + (lane >> 3), fj = (warp % tiles_j) * 8 + (lane & 7);
+  const int fi = (warp / tiles_j) * pi + lane / pj, fj = (warp % tiles_j) * pj + lane % pj;
   *i = fi / a.ss;
   *j = fj / a.ss;
   *is = fi % a.ss;
   *js = fj % a.ss;
-  return fi < nf && fj < nf;
+  return lane < a.lanes && fi < nf && fj < nf;
 }
 inline long long ray_warps(const GridRays& a) {
   const long long nf = (long long)a.G * a.ss;
-  return ((nf + 3) / 4) * ((nf + 7) / 8);
+  const int pi = patch_rows(a.lanes), pj = patch_cols(a.lanes);
+  return ((nf + pi - 1) / pi) * ((nf + pj - 1) / pj);
 }
 
 __device__ __forceinline__ double* ray_nodes(const GridRays& a, int i, int j, int is, int js) {
@@ -119,8 +121,8 @@ inline bool grid_takes_rays(int G, unsigned ss) {
 // marked irregular.  *taken is false when the grid is not for this, or its
 // scratch is not to be had: nothing has been done.
 template <class Rays, class Serial>
-dtfe_status_t grid_by_rays(int G, unsigned ss, double* d_grid, cudaStream_t s, bool* taken,
-                           Rays&& rays, Serial&& serial) {
+dtfe_status_t grid_by_rays(int G, unsigned ss, int lanes, double* d_grid, cudaStream_t s,
+                           bool* taken, Rays&& rays, Serial&& serial) {
   *taken = false;
   if (!grid_takes_rays(G, ss)) return DTFE_OK;
   const size_t n = (size_t)G * ss, col_bytes = sizeof(int) * (size_t)G * G;
@@ -133,7 +135,7 @@ dtfe_status_t grid_by_rays(int G, unsigned ss, double* d_grid, cudaStream_t s, b
     return DTFE_OK;
   }
   *taken = true;
-  const GridRays a{G, (int)ss, static_cast<double*>(nodes), static_cast<int*>(col)};
+  const GridRays a{G, (int)ss, lanes, static_cast<double*>(nodes), static_cast<int*>(col)};
   cudaError_t e = cudaMemsetAsync(col, 0, col_bytes, s);
   if (e == cudaSuccess) {
     rays(a);

@@ -1100,6 +1100,7 @@ struct MapArgs32 {
   int n_tri;
   double* __restrict__ map;
   int G, S, TW, TH, tiles_x;
+  int lanes;  // rays a warp walks at a time (map_lanes32)
   double dxy, offx, offy, scale, soff;
   MixConf C;
   int loc_budget;
@@ -1144,13 +1145,19 @@ __device__ __forceinline__ void add_stats32(unsigned long long* stats, bool acti
 // (*loc, from tile_location): a ray resumes the walk from triangle 0 where
 // the tile's rectangle straddled a test, so it reaches exactly the triangle
 // and status of its own walk.
-template <int BLOCK>
+template <int BLOCK, bool Sparse = false>
 __device__ __forceinline__ void map_tile32(const MapArgs32& a, int tile,
                                            const int2* __restrict__ loc, double* s_val,
                                            unsigned char* s_ok) {
   const int P = a.TW * a.TH;
   const int tx0 = (tile % a.tiles_x) * a.TW, ty0 = (tile / a.tiles_x) * a.TH;
-  for (int t = threadIdx.x; t < P * a.S; t += BLOCK) {
+  const int lane = (int)(threadIdx.x & 31u), n_rays = P * a.S;
+  int t0 = threadIdx.x, step = BLOCK;
+  if (Sparse) {
+    t0 = lane < a.lanes ? (int)(threadIdx.x >> 5) * a.lanes + lane : n_rays;
+    step = (BLOCK / 32) * a.lanes;
+  }
+  for (int t = t0; t < n_rays; t += step) {
     const int lp = t / a.S, s = t % a.S;
     const int col = tx0 + lp % a.TW, row = ty0 + lp / a.TW;
     const bool active = col < a.G && row < a.G;
@@ -1195,12 +1202,12 @@ __device__ __forceinline__ void map_tile32(const MapArgs32& a, int tile,
 // One block per tile.  BLOCK threads per block and MINB blocks per SM (the
 // register budget) are compile-time; the autotuner picks among the
 // instantiations.
-template <int BLOCK, int MINB>
+template <int BLOCK, int MINB, bool Sparse = false>
 __global__ void __launch_bounds__(BLOCK, MINB)
     k_map32(const __grid_constant__ MapArgs32 a, const int2* __restrict__ loc) {
   extern __shared__ double s_val32[];  // P*S doubles, then P*S success bytes
   unsigned char* s_ok = reinterpret_cast<unsigned char*>(s_val32 + a.TW * a.TH * a.S);
-  map_tile32<BLOCK>(a, blockIdx.x, loc + blockIdx.x, s_val32, s_ok);
+  map_tile32<BLOCK, Sparse>(a, blockIdx.x, loc + blockIdx.x, s_val32, s_ok);
 }
 
 // Every tile's shared point location, one thread per tile, before the map
@@ -1309,7 +1316,7 @@ __global__ void __launch_bounds__(128) k_trace32(const TetGeo32* __restrict__ re
 struct GridArgs32 {
   const TetGeo32* __restrict__ rec;
   const TriRec64* __restrict__ tri;
-  int n_tri, G, ss, loc_budget;
+  int n_tri, G, ss, loc_budget, lanes;
   double dxy, offx, offy;
   double z0, dzs, inv_dzs, w;
   MixConf C;
@@ -1347,7 +1354,7 @@ template <bool Marked, int MinBlocks>
 __global__ void __launch_bounds__(128, MinBlocks)
     k_grid32(const __grid_constant__ GridArgs32 a, const GridRays r) {
   int i, j;
-  bool active = grid_column(a.G, &i, &j);
+  bool active = grid_column(a.G, a.lanes, &i, &j);
   const int marks = Marked && active ? r.col[(size_t)i * a.G + j] : 0;
   int worst = kRayOk, visits = 0, fallbacks = 0;
   if (Marked ? (marks & kIrregular) != 0 : active) {
@@ -1468,6 +1475,10 @@ const Variant32 kVariants32[] = {
 };
 constexpr int kNumVariants32 = sizeof(kVariants32) / sizeof(kVariants32[0]);
 constexpr int kDefaultVariant32 = 7;  // (128, 8): the usual winner on B200
+// The default variant's small maps (map_lanes32): 80 registers, as few warps are
+// left to hide spills (65,536 rays 354 us, with 64 registers 377; 128 registers
+// are no faster).
+const MapKernel32 kSparseMap32 = k_map32<128, 6, true>;
 
 typedef void (*BatchKernel32)(const BatchTable32, unsigned long long*, const int2*);
 const BatchKernel32 kBatch32[] = {k_batch32<256, 2>, k_batch32<256, 3>, k_batch32<256, 4>,
@@ -1488,8 +1499,22 @@ dtfe_status_t check_mixed(const Mesh& m, int axis) {
 
 int pick_variant32(int v) { return (v >= 0 && v < kNumVariants32) ? v : kDefaultVariant32; }
 
+// Rays a warp of a single mixed map walks.  A small map is over when its slowest
+// warp is, and a warp's lanes wait for its longest ray and, one at a time, for
+// each other's general steps: 16,384 rays are 512 full warps, fewer than the
+// GPU's 592 schedulers.  Full -> 16 -> 8 -> 4 lanes, us: 8,192 rays 191, 154, 129,
+// 110; 16,384 169, 147, 128, 116; 32,768 135, 134, 138, 160; 65,536 423, 377, 346,
+// 475; 131,044 425, 435, 553.  At 16 lanes 64,800 rays gain too (211 -> 190).  A block keeps room for one pixel's samples, which
+// otherwise would take turns.
+int map_lanes32(const MapGeom& g, int block) {
+  const long long rays = (long long)g.G * g.G * g.S;
+  int lanes = rays <= 16384 ? 4 : (rays <= 65536 ? 16 : 32);
+  while (lanes < 32 && block / 32 * lanes < g.S) lanes *= 2;
+  return lanes;
+}
+
 // The kernel arguments of one mixed map; *tiles_y receives its rows of tiles.
-dtfe_status_t map_args32(Mesh& m, const MapGeom& g, int vi, double* d_map,
+dtfe_status_t map_args32(Mesh& m, const MapGeom& g, int vi, int lanes, double* d_map,
                          unsigned long long* stats, double* ray_rho, int* ray_crossed,
                          int* ray_status, MapArgs32* out, int* tiles_y) {
   SDTFE_TRY(check_mixed(m, g.axis));
@@ -1502,7 +1527,8 @@ dtfe_status_t map_args32(Mesh& m, const MapGeom& g, int vi, double* d_map,
   a.map = d_map;
   a.G = g.G;
   a.S = g.S;
-  tile_shape32(V.block * V.rpt, g.S, V.wide, &a.TW, &a.TH);
+  a.lanes = lanes;
+  tile_shape32(V.block * V.rpt * lanes / 32, g.S, V.wide, &a.TW, &a.TH);
   a.tiles_x = (g.G + a.TW - 1) / a.TW;
   *tiles_y = (g.G + a.TH - 1) / a.TH;
   a.dxy = g.dxy;
@@ -1529,12 +1555,14 @@ dtfe_status_t launch_map32(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
                            double* ray_rho, int* ray_crossed, int* ray_status) {
   const int vi = pick_variant32(m.tune32);
   const Variant32& V = kVariants32[vi];
+  const int lanes = vi == kDefaultVariant32 ? map_lanes32(g, V.block) : 32;
+  const MapKernel32 kernel = lanes < 32 ? kSparseMap32 : V.kernel;
   MapArgs32 a;
   int tiles_y = 0;
-  SDTFE_TRY(map_args32(m, g, vi, d_map, m.stats, ray_rho, ray_crossed, ray_status, &a, &tiles_y));
+  SDTFE_TRY(map_args32(m, g, vi, lanes, d_map, m.stats, ray_rho, ray_crossed, ray_status, &a, &tiles_y));
   const size_t smem = (size_t)a.TW * a.TH * g.S * (sizeof(double) + 1);
   if (smem > 40 * 1024)
-    SDTFE_CUDA(cudaFuncSetAttribute(V.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SDTFE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long long blocks = (long long)a.tiles_x * tiles_y;
   SDTFE_CUDA(cudaMemsetAsync(m.stats, 0, sizeof(unsigned long long) * kStatCount, s));
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
@@ -1543,7 +1571,7 @@ dtfe_status_t launch_map32(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
   k_locate_map32<<<(unsigned)((blocks + 127) / 128), 128, 0, s>>>(a, (int)blocks,
                                                                   static_cast<int2*>(loc));
   count_launch();
-  V.kernel<<<(unsigned)blocks, V.block, smem, s>>>(a, static_cast<const int2*>(loc));
+  kernel<<<(unsigned)blocks, V.block, smem, s>>>(a, static_cast<const int2*>(loc));
   count_launch();
   const cudaError_t e = cudaGetLastError();
   scratch_free_async(loc, s);
@@ -1551,6 +1579,17 @@ dtfe_status_t launch_map32(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
   SDTFE_CUDA(cudaEventRecord(m.ev1, s));
   m.timed = true;
   return DTFE_OK;
+}
+
+// Columns or sub-rays a warp of the mixed grid walks.  A launch that leaves the
+// SMs few warps waits for each warp's longest walk, its most nodes and its
+// general steps, one lane at a time; fewer lanes a warp shorten all three while
+// all warps are still resident (16 a SM).  Full -> 16 -> 8 lanes, ms: 64^3
+// 0.222, 0.170, 0.146; 128^3 0.337, 0.277, 0.253; 160^3 0.326, 0.281, 0.377; 180^3
+// 0.547, 0.437, 0.603; 256^3 0.703, 0.813; sub-rays at ss 2 or 3: 30^3 0.323, 0.276,
+// 0.233; 48^3 0.541, 0.459, 0.450; 100^3 1.10, 0.82, 0.91.
+static int grid_lanes32(long long n) {
+  return n <= 148 * 16 * 8 ? 8 : (n <= 148 * 18 * 16 ? 16 : 32);
 }
 
 dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[3], unsigned ss,
@@ -1567,6 +1606,7 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
   a.n_tri = A.n_tri;
   a.G = G;
   a.ss = (int)ss;
+  a.lanes = grid_lanes32((long long)G * G);
   a.loc_budget = 4 * A.n_tri + 64;
   // src/dtfe.c:668-735 and :398-404: cell and node spacing, weight 1/ss^3
   a.dxy = box_len / G;
@@ -1586,17 +1626,17 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
   bool taken = false;
   SDTFE_TRY(grid_by_rays(
-      G, ss, d_grid, s, &taken,
+      G, ss, grid_lanes32((long long)G * ss * G * ss), d_grid, s, &taken,
       [&](const GridRays& r) {
         k_grid_rays32<<<(unsigned)((ray_warps(r) + 1) / 2), 64, 0, s>>>(a, r);
       },
-      [&](const GridRays& r) { k_grid32<true, 4><<<grid_warps(G) / 4, 128, 0, s>>>(a, r); }));
+      [&](const GridRays& r) { k_grid32<true, 4><<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, r); }));
   if (!taken) {
     // four blocks of 128 columns per SM are all of a grid of up to 148 x 512
     // columns; a larger one gains more from six blocks per SM than it loses to
     // spills (83k-point lattice: 256^3 0.736 against 0.771 ms, 512^3 2.47 against 2.42)
     const bool small = (long long)G * G <= 148 * 512;
-    (small ? k_grid32<false, 4> : k_grid32<false, 6>)<<<grid_warps(G) / 4, 128, 0, s>>>(a, GridRays{});
+    (small ? k_grid32<false, 4> : k_grid32<false, 6>)<<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, GridRays{});
     count_launch();
   }
   SDTFE_CUDA(cudaGetLastError());
@@ -1646,7 +1686,7 @@ dtfe_status_t plan_batch32(const BatchMap* maps, int n, int variant, BatchPlan* 
     const BatchMap& b = maps[i];
     BatchJob32 j;
     int tiles_y = 0;
-    SDTFE_TRY(map_args32(*b.mesh, b.g, vi, b.d_map, b.stats, nullptr, nullptr, nullptr, &j.args,
+    SDTFE_TRY(map_args32(*b.mesh, b.g, vi, 32, b.d_map, b.stats, nullptr, nullptr, nullptr, &j.args,
                          &tiles_y));
     const long long tiles = (long long)j.args.tiles_x * tiles_y;
     const long long cnt = b.count < 0 ? tiles - b.tile0 : b.count;

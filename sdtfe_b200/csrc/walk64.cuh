@@ -372,21 +372,31 @@ struct SurfaceAcc64 {
 // loop (src/dtfe.c:505-511).
 __device__ __forceinline__ void cell_add(double* cell, double v) { atomicAdd(cell, v); }
 
+// The patch of neighbouring columns or rays that a warp walks on its first
+// `lanes` lanes: 4 x 8, 4 x 4 or 2 x 4.  (A launch too small for the GPU takes
+// fewer of them a warp: grid_lanes32 in walk32.cu, grid_lanes64 in walk.cu.)
+__host__ __device__ constexpr int patch_rows(int lanes) { return lanes <= 8 ? 2 : 4; }
+__host__ __device__ constexpr int patch_cols(int lanes) { return lanes <= 16 ? 4 : 8; }
+
 // This thread's grid column (i: x index, j: y index) in a launch of
-// grid_warps(G) warps: each warp covers a 4 x 8 patch and four in a row an
-// 8 x 16 tile, so that a warp's columns are neighbours and cross many of the
-// same tets.  False for the columns past the grid.
-__device__ __forceinline__ bool grid_column(int G, int* i, int* j) {
+// grid_warps(G, lanes) warps: each warp covers a patch and four in a row two by
+// two of them, so that a warp's columns are neighbours and cross many of the
+// same tets.  False for the columns past the grid and the lanes past the patch.
+__device__ __forceinline__ bool grid_column(int G, int lanes, int* i, int* j) {
   const int warp = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
   const int tile = warp >> 2, wq = warp & 3;
-  const int tiles_j = (G + 15) >> 4;
+  const int pi = patch_rows(lanes), pj = patch_cols(lanes);
+  const int tiles_j = (G + 2 * pj - 1) / (2 * pj);
   const int ti = tile / tiles_j, tj = tile - ti * tiles_j;
   const int lane = (int)threadIdx.x & 31;
-  *i = ti * 8 + (wq >> 1) * 4 + (lane >> 3);
-  *j = tj * 16 + (wq & 1) * 8 + (lane & 7);
-  return *i < G && *j < G;
+  *i = (2 * ti + (wq >> 1)) * pi + lane / pj;
+  *j = (2 * tj + (wq & 1)) * pj + lane % pj;
+  return lane < lanes && *i < G && *j < G;
 }
-inline unsigned grid_warps(int G) { return 4u * (unsigned)(((G + 7) / 8) * ((G + 15) / 16)); }
+inline unsigned grid_warps(int G, int lanes) {
+  const int pi = 2 * patch_rows(lanes), pj = 2 * patch_cols(lanes);
+  return 4u * (unsigned)(((G + pi - 1) / pi) * ((G + pj - 1) / pj));
+}
 
 // a12: 3-D column, src/dtfe.c:489-513.  The field is sampled at the fine z
 // nodes inside the chord and added, with weight 1/ss^3, to the column cell.
