@@ -13,6 +13,7 @@
 #include <cstring>
 #include <vector>
 
+#include "density.cuh"
 #include "mesh.h"
 
 namespace sdtfe {
@@ -52,87 +53,22 @@ __global__ void k_fp32_exact(const double4* __restrict__ pos, int n, int* __rest
   atomicMax(max_bits, __float_as_int(mx));
 }
 
-// a3 part 1: |det(A-D, B-D, C-D)|/6, the reference's expansion order
-// (src/triangulate.c:191-215).
-__global__ void k_volume(const double4* __restrict__ pos, const int4* __restrict__ rows, int nt,
-                         double* __restrict__ vol) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  const int4 v = rows[2 * (size_t)t];
-  const double4 a = pos[v.x], b = pos[v.y], c = pos[v.z], d = pos[v.w];
-  const double r0 = (a.x - d.x) * ((b.y - d.y) * (c.z - d.z) - (b.z - d.z) * (c.y - d.y));
-  const double r1 = (a.y - d.y) * ((b.z - d.z) * (c.x - d.x) - (b.x - d.x) * (c.z - d.z));
-  const double r2 = (a.z - d.z) * ((b.x - d.x) * (c.y - d.y) - (b.y - d.y) * (c.x - d.x));
-  vol[t] = fabs((r0 + r1 + r2) / 6);
-}
-
-// CSR of (key -> value) pairs, built in three deterministic steps: integer
-// counts, exclusive scan, fill.  The fill order inside a segment depends on
-// atomic scheduling; segments that need an order are sorted afterwards.
-__global__ void k_count_tet_vertices(const int4* __restrict__ rows, int nt, int* __restrict__ cnt) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  const int4 v = rows[2 * (size_t)t];
-  atomicAdd(cnt + v.x, 1);
-  atomicAdd(cnt + v.y, 1);
-  atomicAdd(cnt + v.z, 1);
-  atomicAdd(cnt + v.w, 1);
-}
-
-__global__ void k_fill_tet_vertices(const int4* __restrict__ rows, int nt,
-                                    const int* __restrict__ off, int* __restrict__ cursor,
-                                    int* __restrict__ idx) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  const int4 v = rows[2 * (size_t)t];
-  idx[off[v.x] + atomicAdd(cursor + v.x, 1)] = t;
-  idx[off[v.y] + atomicAdd(cursor + v.y, 1)] = t;
-  idx[off[v.z] + atomicAdd(cursor + v.z, 1)] = t;
-  idx[off[v.w] + atomicAdd(cursor + v.w, 1)] = t;
-}
-
-// Sort each vertex's tets by index, so that the density sum below adds the
-// volumes in increasing tet order, the order of the reference's scatter loop
-// (src/triangulate.c:190-221).  Shell sort over a diminishing gap sequence
-// (Ciura's gaps, then x2.25): plain insertion sort for the usual ~27 tets of
-// a vertex, and O(d^1.3) rather than O(d^2) for the rare hub vertex with
-// hundreds or thousands of tets.  The tet ids of a segment are distinct, so
-// the sorted order is unique.
-__global__ void k_sort_segments(const int* __restrict__ off, int n, int* __restrict__ idx) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  const int b = off[v], d = off[v + 1] - b;
-  int* a = idx + b;
-  constexpr int kGaps[] = {1, 4, 10, 23, 57, 132, 301, 701, 1577, 3548, 7983, 17961, 40412};
-  int g = 0;
-  while (g + 1 < (int)(sizeof(kGaps) / sizeof(kGaps[0])) && kGaps[g + 1] < d) ++g;
-  for (; g >= 0; --g) {
-    const int gap = kGaps[g];
-    for (int i = gap; i < d; ++i) {
-      const int key = a[i];
-      int j = i;
-      while (j >= gap && a[j - gap] > key) {
-        a[j] = a[j - gap];
-        j -= gap;
-      }
-      a[j] = key;
-    }
-  }
-}
-
 // a3 part 2: rho_v = m*(1+3) / sum of adjacent volumes, the sum taken
 // sequentially from 0 in increasing tet order (bit-identical to the
-// reference's in-place scatter-add).  No float atomics.
-__global__ void k_density(const int* __restrict__ off, const int* __restrict__ idx,
-                          const double* __restrict__ vol, int n, double m4,
-                          double4* __restrict__ pos, int* __restrict__ adj) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+// reference's in-place scatter-add).  No float atomics.  A warp per vertex
+// (density.cuh).
+__global__ void __launch_bounds__(32 * kDensityWarps)
+    k_density(const int* __restrict__ off, int* __restrict__ idx, const double* __restrict__ vol,
+              int n, double m4, double4* __restrict__ pos, int* __restrict__ adj) {
+  __shared__ double row[kDensityWarps][kRankedTets];
+  const int w = (int)(threadIdx.x >> 5), v = blockIdx.x * kDensityWarps + w;
   if (v >= n) return;
-  const int b = off[v], e = off[v + 1];
-  double s = 0;
-  for (int i = b; i < e; ++i) s += vol[idx[i]];
-  pos[v].w = m4 / s;
-  adj[v] = e - b;
+  const int b = off[v], d = off[v + 1] - b;
+  const double s = volume_sum(idx + b, d, vol, row[w]);
+  if ((threadIdx.x & 31) == 0) {
+    pos[v].w = m4 / s;
+    adj[v] = d;
+  }
 }
 
 __device__ __forceinline__ double det3(double a, double b, double c, double d, double e, double f,
@@ -544,23 +480,18 @@ dtfe_status_t mesh_density(Mesh* m) {
   SDTFE_CUDA(cudaMallocAsync(&idx, sizeof(int) * (4 * (size_t)nt + 1), s));
   SDTFE_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (n + 1), s));
   if (nt) {
-    k_volume<<<grid_for(nt), kBlock, 0, s>>>(m->pos, m->rows, nt, vol);
-    count_launch();
-    k_count_tet_vertices<<<grid_for(nt), kBlock, 0, s>>>(m->rows, nt, cnt);
+    k_volume_count<false><<<grid_for(nt), kBlock, 0, s>>>(m->pos, m->rows, nt, n, vol, cnt, nullptr);
     count_launch();
   }
   SDTFE_TRY(exclusive_scan(cnt, off, n, s));
-  SDTFE_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (n + 1), s));
   if (nt) {
-    k_fill_tet_vertices<<<grid_for(nt), kBlock, 0, s>>>(m->rows, nt, off, cnt, idx);
+    k_tet_fill<false><<<grid_for(nt), kBlock, 0, s>>>(m->rows, nt, n, off, cnt, idx);
     count_launch();
   }
   if (n) {
-    k_sort_segments<<<grid_for(n), kBlock, 0, s>>>(off, n, idx);
-    count_launch();
     // p_mass*(1+DIM) is a float product in the reference (float * int)
     const double m4 = (double)(m->p_mass * 4);
-    k_density<<<grid_for(n), kBlock, 0, s>>>(off, idx, vol, n, m4, m->pos, m->adj);
+    k_density<<<grid_for(n, kDensityWarps), 32 * kDensityWarps, 0, s>>>(off, idx, vol, n, m4, m->pos, m->adj);
     count_launch();
   }
   cudaFreeAsync(vol, s);

@@ -26,13 +26,14 @@
 // that first call is also when the 48 MiB are reserved on the device, so a
 // caller makes one call per device at start-up (n_particles == 0 does only the
 // set-up), before its memory pool takes the device's memory and before any
-// stream capture.  Each call waits on its stream twice (for the validation
-// flag, and for its own work before it returns): it blocks the calling thread.
+// stream capture.  Each call waits for its own work (and the validation flag
+// that comes back behind it) before it returns: it blocks the calling thread.
 #include <cub/device/device_scan.cuh>
 
 #include <cstring>
 #include <mutex>
 
+#include "density.cuh"
 #include "mesh.h"
 
 namespace sdtfe {
@@ -51,61 +52,17 @@ inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 inline unsigned blocks_for(long long n) { return (unsigned)((n + kBlk - 1) / kBlk > 0 ? (n + kBlk - 1) / kBlk : 1); }
 
-__global__ void k_na_validate(const int4* __restrict__ rows, int nt, int n, int* __restrict__ err) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  const int4 v = rows[2 * (size_t)t];
-  if ((unsigned)v.x >= (unsigned)n || (unsigned)v.y >= (unsigned)n || (unsigned)v.z >= (unsigned)n ||
-      (unsigned)v.w >= (unsigned)n)
-    atomicOr(err, 1);
-}
-
-__global__ void k_na_volume_count(const double4* __restrict__ pos, const int4* __restrict__ rows,
-                                  int nt, double* __restrict__ vol, int* __restrict__ cnt) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  const int4 v = rows[2 * (size_t)t];
-  const double4 a = pos[v.x], b = pos[v.y], c = pos[v.z], d = pos[v.w];
-  const double r0 = (a.x - d.x) * ((b.y - d.y) * (c.z - d.z) - (b.z - d.z) * (c.y - d.y));
-  const double r1 = (a.y - d.y) * ((b.z - d.z) * (c.x - d.x) - (b.x - d.x) * (c.z - d.z));
-  const double r2 = (a.z - d.z) * ((b.x - d.x) * (c.y - d.y) - (b.y - d.y) * (c.x - d.x));
-  vol[t] = fabs((r0 + r1 + r2) / 6);
-  atomicAdd(cnt + v.x, 1);
-  atomicAdd(cnt + v.y, 1);
-  atomicAdd(cnt + v.z, 1);
-  atomicAdd(cnt + v.w, 1);
-}
-
-__global__ void k_na_fill(const int4* __restrict__ rows, int nt, const int* __restrict__ off,
-                          int* __restrict__ cursor, int* __restrict__ idx) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nt) return;
-  const int4 v = rows[2 * (size_t)t];
-  idx[off[v.x] + atomicAdd(cursor + v.x, 1)] = t;
-  idx[off[v.y] + atomicAdd(cursor + v.y, 1)] = t;
-  idx[off[v.z] + atomicAdd(cursor + v.z, 1)] = t;
-  idx[off[v.w] + atomicAdd(cursor + v.w, 1)] = t;
-}
-
-// sort each vertex's tets by index, then sum their volumes in that order
-__global__ void k_na_density(const int* __restrict__ off, int* __restrict__ idx,
-                             const double* __restrict__ vol, int n, double m4,
-                             double* __restrict__ rho) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  const int b = off[v], e = off[v + 1];
-  for (int i = b + 1; i < e; ++i) {
-    const int key = idx[i];
-    int j = i - 1;
-    while (j >= b && idx[j] > key) {
-      idx[j + 1] = idx[j];
-      --j;
-    }
-    idx[j + 1] = key;
-  }
-  double s = 0;
-  for (int i = b; i < e; ++i) s += vol[idx[i]];
-  rho[v] = m4 / s;
+// A vertex's volumes summed in tet order, a warp per vertex (density.cuh).
+// Nothing is written when a tet was out of range.
+__global__ void __launch_bounds__(32 * kDensityWarps)
+    k_na_density(const int* __restrict__ off, int* __restrict__ idx, const double* __restrict__ vol,
+                 int n, double m4, const int* __restrict__ err, double* __restrict__ rho) {
+  __shared__ double row[kDensityWarps][kRankedTets];
+  const int w = (int)(threadIdx.x >> 5), v = blockIdx.x * kDensityWarps + w;
+  if (v >= n || *err) return;
+  const int b = off[v];
+  const double s = volume_sum(idx + b, off[v + 1] - b, vol, row[w]);
+  if ((threadIdx.x & 31) == 0) rho[v] = m4 / s;
 }
 
 // the scratch array's device address on the current device (looked up once)
@@ -138,12 +95,12 @@ extern "C" dtfe_status_t dtfe_density_noalloc(const double* d_particle_data, int
     return set_error(DTFE_ERR_INVALID, "NULL device pointer");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int n = n_particles, nt = n_tetra;
-  // carve the scratch: error flag | vol | cnt (n+1) | off (n+1) | idx (4 nt) | scan temp;
+  // carve the scratch: error flag | cnt (n+1) | off (n+1) | vol | idx (4 nt) | scan temp;
   // the fixed part is checked first, in size_t, so that n + 1 below is an int
-  const size_t o_vol = 256;
-  const size_t o_cnt = align256(o_vol + sizeof(double) * (size_t)nt);
+  const size_t o_cnt = 256;
   const size_t o_off = align256(o_cnt + sizeof(int) * ((size_t)n + 1));
-  const size_t o_idx = align256(o_off + sizeof(int) * ((size_t)n + 1));
+  const size_t o_vol = align256(o_off + sizeof(int) * ((size_t)n + 1));
+  const size_t o_idx = align256(o_vol + sizeof(double) * (size_t)nt);
   const size_t o_tmp = align256(o_idx + sizeof(int) * 4 * (size_t)nt);
   if (o_tmp > kNoAllocScratchBytes)
     return set_error(DTFE_ERR_UNSUPPORTED,
@@ -170,31 +127,25 @@ extern "C" dtfe_status_t dtfe_density_noalloc(const double* d_particle_data, int
   const int4* rows = reinterpret_cast<const int4*>(d_tetra_data);
 
   // the array keeps the previous call's contents: clear what starts at zero
-  SDTFE_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
-  SDTFE_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)n + 1), s));
+  SDTFE_CUDA(cudaMemsetAsync(err, 0, o_cnt + sizeof(int) * ((size_t)n + 1), s));
   if (nt) {
-    k_na_validate<<<blocks_for(nt), kBlk, 0, s>>>(rows, nt, n, err);
+    k_volume_count<true><<<blocks_for(nt), kBlk, 0, s>>>(pos, rows, nt, n, vol, cnt, err);
     count_launch();
   }
+  SDTFE_CUDA(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, cnt, off, n + 1, s));
+  if (nt) {
+    k_tet_fill<true><<<blocks_for(nt), kBlk, 0, s>>>(rows, nt, n, off, cnt, idx);
+    count_launch();
+  }
+  const double m4 = (double)(p_mass * 4);  // float product, as in the reference
+  k_na_density<<<(unsigned)(((long long)n + kDensityWarps - 1) / kDensityWarps), 32 * kDensityWarps, 0, s>>>(
+      off, idx, vol, n, m4, err, d_rho);
+  count_launch();
+  SDTFE_CUDA(cudaGetLastError());
   int h_err = 0;
   SDTFE_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
   SDTFE_CUDA(cudaStreamSynchronize(s));
   if (h_err)
     return set_error(DTFE_ERR_MESH, "tetra_data holds a vertex id outside [0, %d)", n);
-  if (nt) {
-    k_na_volume_count<<<blocks_for(nt), kBlk, 0, s>>>(pos, rows, nt, vol, cnt);
-    count_launch();
-  }
-  SDTFE_CUDA(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, cnt, off, n + 1, s));
-  SDTFE_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)n + 1), s));
-  if (nt) {
-    k_na_fill<<<blocks_for(nt), kBlk, 0, s>>>(rows, nt, off, cnt, idx);
-    count_launch();
-  }
-  const double m4 = (double)(p_mass * 4);  // float product, as in the reference
-  k_na_density<<<blocks_for(n), kBlk, 0, s>>>(off, idx, vol, n, m4, d_rho);
-  count_launch();
-  SDTFE_CUDA(cudaGetLastError());
-  SDTFE_CUDA(cudaStreamSynchronize(s));
   return DTFE_OK;
 }
