@@ -299,7 +299,7 @@ dtfe_status_t dtfe_autotune(dtfe_mesh_t h, const dtfe_map_params_t* p, int* best
   cudaStream_t s = m.stream;
   double* d_map = nullptr;
   const size_t bytes = sizeof(double) * (size_t)q.grid_dim * q.grid_dim;
-  SDTFE_CUDA(cudaMallocAsync(&d_map, bytes, s));
+  SDTFE_TRY(scratch_alloc_async(&d_map, bytes, s));
   const int nv = num_map32_variants();
   int best_v = -1;
   float best_ms = 0.f;
@@ -352,7 +352,7 @@ dtfe_status_t map_to_host(Mesh& m, const dtfe_map_params_t* p, double* map, F&& 
   cudaStream_t s = m.stream;
   const size_t bytes = sizeof(double) * (size_t)p->grid_dim * p->grid_dim;
   double* d_map = nullptr;
-  SDTFE_CUDA(cudaMallocAsync(&d_map, bytes, s));
+  SDTFE_TRY(scratch_alloc_async(&d_map, bytes, s));
   cudaError_t e = cudaMemcpyAsync(d_map, map, bytes, cudaMemcpyHostToDevice, s);
   dtfe_status_t st = e == cudaSuccess ? launch_map(m, p, d_map, s)
                                       : set_error(DTFE_ERR_CUDA, "map: %s", cudaGetErrorString(e));
@@ -417,10 +417,7 @@ dtfe_status_t dtfe_map_rays(dtfe_mesh_t h, const dtfe_map_params_t* p, double* m
   void* host[4] = {map, ray_rho, ray_crossed, ray_status};
   dtfe_status_t st = DTFE_OK;
   for (int k = 0; k < 4 && st == DTFE_OK; ++k) {
-    const cudaError_t e = cudaMallocAsync(&d[k], sz[k], s);
-    if (e != cudaSuccess)
-      st = set_error(e == cudaErrorMemoryAllocation ? DTFE_ERR_NOMEM : DTFE_ERR_CUDA,
-                     "map_rays: %s", cudaGetErrorString(e));
+    st = scratch_alloc_async(&d[k], sz[k], s);
   }
   if (st == DTFE_OK) {
     const cudaError_t e = cudaMemcpyAsync(d[0], map, bytes, cudaMemcpyHostToDevice, s);
@@ -459,14 +456,14 @@ dtfe_status_t dtfe_trace(dtfe_mesh_t h, const dtfe_map_params_t* p, int n_rays, 
   const int max_visits = (int)(mv > 0x7fffffff ? 0x7fffffff : mv);
   double *dx, *dy, *dr;
   int *dc, *ds, *dv = nullptr;
-  SDTFE_CUDA(cudaMallocAsync(&dx, sizeof(double) * n_rays, s));
-  SDTFE_CUDA(cudaMallocAsync(&dy, sizeof(double) * n_rays, s));
-  SDTFE_CUDA(cudaMallocAsync(&dr, sizeof(double) * n_rays, s));
-  SDTFE_CUDA(cudaMallocAsync(&dc, sizeof(int) * n_rays, s));
-  SDTFE_CUDA(cudaMallocAsync(&ds, sizeof(int) * n_rays, s));
+  SDTFE_TRY(scratch_alloc_async(&dx, sizeof(double) * n_rays, s));
+  SDTFE_TRY(scratch_alloc_async(&dy, sizeof(double) * n_rays, s));
+  SDTFE_TRY(scratch_alloc_async(&dr, sizeof(double) * n_rays, s));
+  SDTFE_TRY(scratch_alloc_async(&dc, sizeof(int) * n_rays, s));
+  SDTFE_TRY(scratch_alloc_async(&ds, sizeof(int) * n_rays, s));
   const size_t vbytes = visits ? sizeof(int) * (size_t)n_rays * max_record : 0;
   if (visits) {
-    SDTFE_CUDA(cudaMallocAsync(&dv, vbytes, s));
+    SDTFE_TRY(scratch_alloc_async(&dv, vbytes, s));
     SDTFE_CUDA(cudaMemsetAsync(dv, 0xff, vbytes, s));
   }
   SDTFE_CUDA(cudaMemcpyAsync(dx, x, sizeof(double) * n_rays, cudaMemcpyHostToDevice, s));
@@ -533,7 +530,7 @@ dtfe_status_t grid_to_host(Mesh& m, int G, double box_len, const double center[3
   cudaStream_t s = m.stream;
   const size_t bytes = sizeof(double) * (size_t)G * G * G;
   double* d = nullptr;
-  SDTFE_CUDA(cudaMallocAsync(&d, bytes, s));
+  SDTFE_TRY(scratch_alloc_async(&d, bytes, s));
   cudaError_t e = cudaMemcpyAsync(d, grid, bytes, cudaMemcpyHostToDevice, s);
   dtfe_status_t st = e == cudaSuccess ? launch_grid(m, G, box_len, center, ss, seed, precision, d, s)
                                       : set_error(DTFE_ERR_CUDA, "grid: %s", cudaGetErrorString(e));

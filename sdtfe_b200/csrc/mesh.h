@@ -102,6 +102,10 @@ size_t mesh_record_bytes(const Mesh& m, int axis);
 void mesh_trim_record_pool();
 // per-call device scratch, stream-ordered on s from the walk-record pool
 dtfe_status_t scratch_alloc_async(void** p, size_t bytes, cudaStream_t s);
+template <class T>
+dtfe_status_t scratch_alloc_async(T** p, size_t bytes, cudaStream_t s) {
+  return scratch_alloc_async(reinterpret_cast<void**>(p), bytes, s);
+}
 void scratch_free_async(void* p, cudaStream_t s);
 size_t mesh_missing_record_bytes(const Mesh& m, int axis, int precision);
 // host_mask (optional) replaces the forward-face test with a caller's bitmap
