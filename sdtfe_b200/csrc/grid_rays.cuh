@@ -20,6 +20,7 @@ namespace {
 
 // where a column's node values go: its cells directly ...
 struct CellSink {
+  static constexpr bool kShortChain = false;  // reciprocal_near, walk64.cuh
   double* col;
   int ss;
   __device__ __forceinline__ void begin(int) {}
@@ -30,6 +31,7 @@ struct CellSink {
 
 // ... or the ray's row of nodes
 struct NodeSink {
+  static constexpr bool kShortChain = true;
   double* row;
   int done;        // nodes written so far
   bool irregular;  // came back to one of them

@@ -345,6 +345,7 @@ __device__ __forceinline__ int locate_from_tile(const TriRec64* __restrict__ tri
 // strictly inside (z0, z1); the linear field there times the chord length is
 // added.
 struct SurfaceAcc64 {
+  static constexpr bool kShortChain = false;
   double z0, z1;
   double rho;
   // what visit() reads of a tet's record, loaded ahead of it
@@ -402,6 +403,7 @@ inline unsigned grid_warps(int G, int lanes) {
 // nodes inside the chord and added, with weight 1/ss^3, to the column cell.
 template <class Sink>  // grid_rays.cuh
 struct ColumnAcc64 {
+  static constexpr bool kShortChain = Sink::kShortChain;
   Sink out;
   double z0, dzs, w;
   int nzs;
@@ -551,13 +553,9 @@ __host__ __device__ __forceinline__ ProductSums product_sums(double n0, double n
 }
 
 template <bool Exit>
-__host__ __device__ __forceinline__ double crossing64(double n0, double n1, double n2, double z0,
-                                                      double z1, double z2, const ProductSums& s,
-                                                      unsigned roles) {
-  const bool f0 = (roles & 3u) == 0u, f1 = (roles & 3u) == 1u;   // corner 0's slot (else 2)
-  const bool l0 = (roles & 12u) == 0u, l2 = (roles & 12u) == 8u;  // the last added (else 1)
-  const double sum = l0 ? s.last0 : (l2 ? s.last2 : s.last1);
-  const double inv = 1.0 / sum;
+__host__ __device__ __forceinline__ double crossing_by(double n0, double n1, double n2, double z0,
+                                                       double z1, double z2, double inv, bool f0,
+                                                       bool f1) {
   const double w0 = n0 * inv, w1 = n1 * inv, w2 = n2 * inv;
   const double m0 = w0 * z0, m1 = w1 * z1, m2 = w2 * z2;
   const double c0 = Exit ? (1 - w2 - w1) * z0 + m2 + m1 : (1 - w1 - w2) * z0 + m1 + m2;
@@ -566,9 +564,61 @@ __host__ __device__ __forceinline__ double crossing64(double n0, double n1, doub
   return f0 ? c0 : (f1 ? c1 : c2);
 }
 
+template <bool Exit>
+__host__ __device__ __forceinline__ double crossing64(double n0, double n1, double n2, double z0,
+                                                      double z1, double z2, const ProductSums& s,
+                                                      unsigned roles) {
+  const bool f0 = (roles & 3u) == 0u, f1 = (roles & 3u) == 1u;   // corner 0's slot (else 2)
+  const bool l0 = (roles & 12u) == 0u, l2 = (roles & 12u) == 8u;  // the last added (else 1)
+  const double sum = l0 ? s.last0 : (l2 ? s.last2 : s.last1);
+  const double inv = 1.0 / sum;
+  return crossing_by<Exit>(n0, n1, n2, z0, z1, z2, inv, f0, f1);
+}
+
+// the same with the reciprocal of role_sum in hand
+__device__ __forceinline__ double role_sum(const ProductSums& s, unsigned roles) {
+  const bool l0 = (roles & 12u) == 0u, l2 = (roles & 12u) == 8u;
+  return l0 ? s.last0 : (l2 ? s.last2 : s.last1);
+}
+template <bool Exit>
+__device__ __forceinline__ double crossing64(double n0, double n1, double n2, double z0, double z1,
+                                             double z2, double inv, unsigned roles) {
+  return crossing_by<Exit>(n0, n1, n2, z0, z1, z2, inv, (roles & 3u) == 0u, (roles & 3u) == 1u);
+}
+
+// 1/s, correctly rounded, from y = 1/s' of an s' within a few ulps of s.  A
+// Newton step with exact remainders takes y, itself a few ulps off, to within
+// one ulp of 1/s, and a second one rounds it correctly unless s has a mantissa
+// of all ones (P. Markstein, IBM J. Res. Dev. 34, 1990, theorem 7); s and 1/s
+// far from over- and underflow.  Four operations for a division's dozen: the
+// sub-rays of grids, which wait for their own chain of operations, gain (32k
+// clustered points, 120^3 at ss 2: 0.579 -> 0.528 ms; 48^3 at ss 3 0.380 ->
+// 0.360); maps (-0.4 to +2.3 %) and one-thread columns (0 to +1 %) do not, so
+// only accumulators with kShortChain use it.
+__host__ __device__ __forceinline__ double reciprocal_near(double s, double y) {
+  y = fma(fma(-s, y, 1.0), y, y);
+  return fma(fma(-s, y, 1.0), y, y);
+}
+__device__ __forceinline__ bool mantissa_all_ones(double s) {
+  return ((uint32_t)__double2loint(s) & ((uint32_t)__double2hiint(s) | 0xFFF00000u)) == 0xFFFFFFFFu;
+}
+
+// Whether three products are all above kZero in magnitude, and below 2^512 (no
+// sum of them, or its reciprocal, is then near over- or underflow).  From the
+// high words alone: what lies within 2^-20 of kZero is left to the general step.
+constexpr uint32_t kZeroHigh = 0x3D838800u;
+static_assert(kZero == 0x1.388p-39, "kZeroHigh is kZero's high word, its low word is 0");
+__device__ __forceinline__ bool all_clear(double a, double b, double c) {
+  constexpr uint32_t lo = 2u * (kZeroHigh + 1u), span = 2u * 0x5FF00000u - lo;
+  const uint32_t u = 2u * (uint32_t)__double2hiint(a) - lo, v = 2u * (uint32_t)__double2hiint(b) - lo,
+                 w = 2u * (uint32_t)__double2hiint(c) - lo;
+  return max(max(u, v), w) < span;
+}
+
 // The triangle of record rec's entry face, in the record's order, and the
 // ray's crossing of it.  False when its products are not all below -kZero:
 // the general step takes the tet.
+template <bool ShortChain>
 __device__ __forceinline__ bool entry_triangle64(const WalkConf64& W, const Ray64& r, int rec,
                                                  Tri64* s, double* z_in) {
   const int F = rec & 3;
@@ -589,7 +639,8 @@ __device__ __forceinline__ bool entry_triangle64(const WalkConf64& W, const Ray6
   s->e20 = edge_u64(r, make_double2(c.x, c.y), make_double2(a.x, a.y));
   *z_in = crossing64<false>(s->e12, s->e20, s->e01, a.z, b.z, c.z,
                              product_sums(s->e12, s->e20, s->e01), entry_roles(F, 0));
-  return s->e01 < -kZero && s->e12 < -kZero && s->e20 < -kZero;
+  return s->e01 < -kZero && s->e12 < -kZero && s->e20 < -kZero &&
+         (!ShortChain || all_clear(s->e01, s->e12, s->e20));
 }
 
 // The walk of one ray from the tet ft, located under hull triangle ft_tri (-1:
@@ -633,7 +684,7 @@ __device__ __forceinline__ int walk64(const WalkConf64& W, int ft, int ft_tri, d
   double z_in = 0.0;
   uint32_t L = 3u * (uint32_t)w.rec;
   int crossed = 0, status = kWalk64On;
-  bool fast = w.rec >= 0 && entry_triangle64(W, r, w.rec, &s, &z_in);
+  bool fast = w.rec >= 0 && entry_triangle64<Acc::kShortChain>(W, r, w.rec, &s, &z_in);
   while (status == kWalk64On) {
     if (fast) {
       const uint32_t rec = L / 3u;
@@ -645,7 +696,8 @@ __device__ __forceinline__ int walk64(const WalkConf64& W, int ft, int ft_tri, d
       const double a0 = edge_u64(r, v, make_double2(s.x0, s.y0));
       const double a1 = edge_u64(r, v, make_double2(s.x1, s.y1));
       const double a2 = edge_u64(r, v, make_double2(s.x2, s.y2));
-      const bool sure = (fabs(a0) > kZero) & (fabs(a1) > kZero) & (fabs(a2) > kZero);
+      const bool sure = Acc::kShortChain ? all_clear(a0, a1, a2)
+                                         : (fabs(a0) > kZero) & (fabs(a1) > kZero) & (fabs(a2) > kZero);
       // (a_0, a_1, a_2 are not all of one sign)
       const bool p2 = a2 > 0.0;
       const bool k0 = p2 & (a1 < 0.0), k1 = !p2 & (a0 > 0.0);  // else k = 2
@@ -671,8 +723,13 @@ __device__ __forceinline__ int walk64(const WalkConf64& W, int ft, int ft_tri, d
         s.y2 = V.y;
         s.z2 = V.z;
         const ProductSums sums = product_sums(s.e12, s.e20, s.e01);
-        const double z_out =
-            crossing64<true>(s.e12, s.e20, s.e01, s.z0, s.z1, s.z2, sums, roles);
+        double inv = 0.0, z_out;
+        if constexpr (Acc::kShortChain) {
+          inv = 1.0 / role_sum(sums, roles);
+          z_out = crossing64<true>(s.e12, s.e20, s.e01, s.z0, s.z1, s.z2, inv, roles);
+        } else {
+          z_out = crossing64<true>(s.e12, s.e20, s.e01, s.z0, s.z1, s.z2, sums, roles);
+        }
         if (visits != nullptr && crossed < max_record) visits[crossed] = (int)(rec >> 2);
         ++crossed;
         acc.visit(ox, oy, field, z_in, z_out);
@@ -680,7 +737,13 @@ __device__ __forceinline__ int walk64(const WalkConf64& W, int ft, int ft_tri, d
           status = kRayOk;
           break;
         }
-        z_in = crossing64<false>(s.e12, s.e20, s.e01, s.z0, s.z1, s.z2, sums, roles >> 4);
+        if constexpr (Acc::kShortChain) {
+          const double sum = role_sum(sums, roles >> 4);
+          const double y = mantissa_all_ones(sum) ? 1.0 / sum : reciprocal_near(sum, inv);
+          z_in = crossing64<false>(s.e12, s.e20, s.e01, s.z0, s.z1, s.z2, y, roles >> 4);
+        } else {
+          z_in = crossing64<false>(s.e12, s.e20, s.e01, s.z0, s.z1, s.z2, sums, roles >> 4);
+        }
         L = next;
         continue;
       }
@@ -697,7 +760,7 @@ __device__ __forceinline__ int walk64(const WalkConf64& W, int ft, int ft_tri, d
     oy = w.oy;
     r.m_oy = -W.lz * oy;
     r.ox_l = W.lz * ox;
-    fast = w.rec >= 0 && entry_triangle64(W, r, w.rec, &s, &z_in);
+    fast = w.rec >= 0 && entry_triangle64<Acc::kShortChain>(W, r, w.rec, &s, &z_in);
     L = 3u * (uint32_t)w.rec;
   }
   if (status != kRayOk) return status;
