@@ -60,7 +60,7 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-BYTES_PER_VISIT = {"mixed": 96, "fp64": 160}  # tet record bytes read per walk step
+BYTES_PER_VISIT = {"mixed": 48, "fp64": 112}  # bytes a walk step reads: one vertex, its links and the tet's field
 
 
 def parse():
@@ -385,7 +385,7 @@ def roofline(kernel, visits, n_tets, bytes_per_visit, kern_ms, sm_mhz, n_sm, hbm
     launch's tet visits x the warp instructions per visit that ncu counted on
     the profiled workload, over the event-timed duration.  DRAM traffic is the
     profile's bytes per tet (each tet's records are read from DRAM about once
-    per map), scaled to this mesh; the algorithmic bytes (96 B per mixed
+    per map), scaled to this mesh; the algorithmic bytes (48 B per mixed
     visit) are mostly served from L1/L2, and are reported beside it."""
     t = kern_ms / 1e3
     alg_gbs = visits * bytes_per_visit / t / 1e9
@@ -1000,8 +1000,10 @@ def run_ours(args, pre=None):
     hbm_note = "measured" if hbm else "fallback"
     hbm = hbm or 6650.0
     kname = "k_map32" if args.precision == "mixed" else "k_map64"
-    roof = roofline(kname, visits, len(tetra), bpv, kern_ms, clk.get("sm_mhz") or 1965.0,
+    # (the profile's key "k_map32" is the walk that read all four vertices of a tet)
+    roof = roofline({"k_map32": "k_map32_apex"}.get(kname, kname), visits, len(tetra), bpv, kern_ms, clk.get("sm_mhz") or 1965.0,
                     torch.cuda.get_device_properties(dev).multi_processor_count, hbm, hbm_note)
+    roof["kernel"] = kname
 
     cpu = None
     if rank == 0 and not args.no_cpu_baseline:

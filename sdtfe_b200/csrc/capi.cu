@@ -304,6 +304,7 @@ dtfe_status_t dtfe_autotune(dtfe_mesh_t h, const dtfe_map_params_t* p, int* best
   int best_v = -1;
   float best_ms = 0.f;
   dtfe_status_t st = DTFE_OK;
+  m.full_warps = q.grid_dim < p->grid_dim;  // the window stands for a larger map
   for (int v = 0; v < nv && st == DTFE_OK; ++v) {
     m.tune32 = v;
     float ms_v = 0.f;
@@ -327,6 +328,7 @@ dtfe_status_t dtfe_autotune(dtfe_mesh_t h, const dtfe_map_params_t* p, int* best
     }
   }
   cudaFreeAsync(d_map, s);
+  m.full_warps = false;
   m.tune32 = best_v;
   if (best) *best = best_v;
   return st;

@@ -76,6 +76,7 @@ struct Mesh {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool timed = false;       // ev0/ev1 bracket the last walk launch
   int tune32 = -1;          // mixed-map kernel variant chosen by the autotuner (-1: default)
+  bool full_warps = false;  // (autotuner) small mixed maps fill their warps too
   int fp64_location = DTFE_LOCATE_PER_RAY;  // FP64 maps' point location (dtfe_locate_t)
   size_t bytes = 0;
 };

@@ -1476,7 +1476,7 @@ const Variant32 kVariants32[] = {
 constexpr int kNumVariants32 = sizeof(kVariants32) / sizeof(kVariants32[0]);
 constexpr int kDefaultVariant32 = 7;  // (128, 8): the usual winner on B200
 // The default variant's small maps (map_lanes32): 80 registers, as few warps are
-// left to hide spills (65,536 rays 354 us, with 64 registers 377; 128 registers
+// left to hide spills (32,768 rays 130 us, with 64 registers 134; 128 registers
 // are no faster).
 const MapKernel32 kSparseMap32 = k_map32<128, 6, true>;
 
@@ -1502,13 +1502,16 @@ int pick_variant32(int v) { return (v >= 0 && v < kNumVariants32) ? v : kDefault
 // Rays a warp of a single mixed map walks.  A small map is over when its slowest
 // warp is, and a warp's lanes wait for its longest ray and, one at a time, for
 // each other's general steps: 16,384 rays are 512 full warps, fewer than the
-// GPU's 592 schedulers.  Full -> 16 -> 8 -> 4 lanes, us: 8,192 rays 191, 154, 129,
-// 110; 16,384 169, 147, 128, 116; 32,768 135, 134, 138, 160; 65,536 423, 377, 346,
-// 475; 131,044 425, 435, 553.  At 16 lanes 64,800 rays gain too (211 -> 190).  A block keeps room for one pixel's samples, which
-// otherwise would take turns.
+// GPU's 592 schedulers.  Full -> 16 -> 8 -> 4 lanes, us a pass: 2,166 rays 130, 117,
+// 106, 96; 7,220 169, 138, 139, 128; 13,225 180, 147, 132, 118; 17,500 281, 207, 176,
+// 178; 20,184 180, 154, 138, 176; 24,576 242, 207, 169, 184; 25,600 165, 159, 165,
+// 192; 31,104 172, 166, 187, 251; 32,400 90, 91, 122.  Above, maps of whole meshes
+// still gain from 16 (53,868 rays 317 -> 301), windows of short rays lose (61,206
+// 118 -> 149).  A block keeps room for one pixel's samples, which otherwise would
+// take turns.
 int map_lanes32(const MapGeom& g, int block) {
   const long long rays = (long long)g.G * g.G * g.S;
-  int lanes = rays <= 16384 ? 4 : (rays <= 65536 ? 16 : 32);
+  int lanes = rays <= 16384 ? 4 : (rays <= 24576 ? 8 : (rays <= 32768 ? 16 : 32));
   while (lanes < 32 && block / 32 * lanes < g.S) lanes *= 2;
   return lanes;
 }
@@ -1555,7 +1558,7 @@ dtfe_status_t launch_map32(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
                            double* ray_rho, int* ray_crossed, int* ray_status) {
   const int vi = pick_variant32(m.tune32);
   const Variant32& V = kVariants32[vi];
-  const int lanes = vi == kDefaultVariant32 ? map_lanes32(g, V.block) : 32;
+  const int lanes = vi == kDefaultVariant32 && !m.full_warps ? map_lanes32(g, V.block) : 32;
   const MapKernel32 kernel = lanes < 32 ? kSparseMap32 : V.kernel;
   MapArgs32 a;
   int tiles_y = 0;
