@@ -1587,12 +1587,13 @@ dtfe_status_t launch_map32(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
 // Columns or sub-rays a warp of the mixed grid walks.  A launch that leaves the
 // SMs few warps waits for each warp's longest walk, its most nodes and its
 // general steps, one lane at a time; fewer lanes a warp shorten all three while
-// all warps are still resident (16 a SM).  Full -> 16 -> 8 lanes, ms: 64^3
-// 0.222, 0.170, 0.146; 128^3 0.337, 0.277, 0.253; 160^3 0.326, 0.281, 0.377; 180^3
-// 0.547, 0.437, 0.603; 256^3 0.703, 0.813; sub-rays at ss 2 or 3: 30^3 0.323, 0.276,
-// 0.233; 48^3 0.541, 0.459, 0.450; 100^3 1.10, 0.82, 0.91.
-static int grid_lanes32(long long n) {
-  return n <= 148 * 16 * 8 ? 8 : (n <= 148 * 18 * 16 ? 16 : 32);
+// all warps are still resident (16 a SM; the sub-ray kernel holds more).  Full ->
+// 16 -> 8 lanes, ms: 64^3 0.222, 0.170, 0.146; 128^3 0.337, 0.277, 0.253; 160^3
+// 0.326, 0.281, 0.377; 180^3 0.547, 0.437, 0.603; 256^3 0.703, 0.813; sub-rays at ss
+// 2 or 3: 30^3 0.323, 0.276, 0.233; 49^3 0.475, 0.398, 0.327; 82^3 0.731, 0.637,
+// 0.574; 85^3 0.426, 0.412, 0.434; 100^3 1.10, 0.82, 0.91.
+static int grid_lanes32(long long n, bool sub_rays) {
+  return n <= 148 * (sub_rays ? 182 : 128) ? 8 : (n <= 148 * 288 ? 16 : 32);
 }
 
 dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[3], unsigned ss,
@@ -1609,7 +1610,7 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
   a.n_tri = A.n_tri;
   a.G = G;
   a.ss = (int)ss;
-  a.lanes = grid_lanes32((long long)G * G);
+  a.lanes = grid_lanes32((long long)G * G, false);
   a.loc_budget = 4 * A.n_tri + 64;
   // src/dtfe.c:668-735 and :398-404: cell and node spacing, weight 1/ss^3
   a.dxy = box_len / G;
@@ -1629,7 +1630,7 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
   bool taken = false;
   SDTFE_TRY(grid_by_rays(
-      G, ss, grid_lanes32((long long)G * ss * G * ss), d_grid, s, &taken,
+      G, ss, grid_lanes32((long long)G * ss * G * ss, true), d_grid, s, &taken,
       [&](const GridRays& r) {
         k_grid_rays32<<<(unsigned)((ray_warps(r) + 1) / 2), 64, 0, s>>>(a, r);
       },

@@ -26,10 +26,10 @@ def mesh(golden, sd):
         yield m
 
 
-# around 16,384 and 65,536 rays, a pixel's samples around a block's room at 4 and
+# around 16,384, 24,576 and 32,768 rays, a pixel's samples around a block's room at 4 and
 # 16 rays a warp, and sides that fill no tile
 @pytest.mark.parametrize("side,samples", [(1, 1), (1, 300), (3, 16), (3, 17), (5, 64), (5, 65), (17, 33), (64, 4),
-                                          (128, 1), (129, 1), (61, 5), (128, 4), (257, 1), (96, 7), (97, 7)])
+                                          (128, 1), (129, 1), (61, 5), (128, 4), (64, 6), (157, 1), (181, 1), (182, 1)])
 def test_maps_equal_full_warps(sd, mesh, side, samples):
     p = sd.map_params(side, 1.0, 1.0, (0.5, 0.5, 0.5), samples, 0.0, 3, precision=sd.DTFE_MIXED)
     out = []
@@ -42,9 +42,11 @@ def test_maps_equal_full_warps(sd, mesh, side, samples):
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
 
 
-# around 8,192 columns or sub-rays (FP64) and 18,944 and 42,624 (mixed)
+# around 8,192 columns or sub-rays (FP64), 18,944 columns, 26,936 sub-rays and
+# 42,624 of either (mixed)
 @pytest.mark.parametrize("G,ss", [(1, 1), (5, 1), (13, 3), (45, 2), (46, 2), (68, 2), (69, 2), (90, 1), (91, 1),
-                                  (103, 2), (104, 2)])
+                                  (82, 2), (83, 2), (103, 2), (104, 2),
+                                  (137, 1), (138, 1)])
 def test_grids(golden, sd, oracle, mesh, G, ss):
     s = golden_set(golden, "clustered")
     got = mesh.grid(G, 1.0, (0.5, 0.5, 0.5), ss, 3)
