@@ -615,6 +615,20 @@ __device__ __forceinline__ bool all_clear(double a, double b, double c) {
   return max(max(u, v), w) < span;
 }
 
+// The face left through, from the apex' products with the vertices of a triangle
+// of three negative products: the one without vertex k, where a_{k+1} < 0 <
+// a_{k+2} (k = 0 if k0, 1 if k1, else 2).  False when the three, none of them
+// zero, have one sign: the reference finds no such face.  Exact products never
+// do, but the reference's are rounded by about lz*x*y*2^-53, which passes kZero in
+// boxes of side 100 and more: the signs at an apex on the ray are then noise.
+__host__ __device__ __forceinline__ bool exit_slot(double a0, double a1, double a2, bool* k0,
+                                                   bool* k1) {
+  const bool p0 = a0 > 0.0, n1 = a1 < 0.0, p2 = a2 > 0.0;
+  *k0 = p2 & n1;
+  *k1 = !p2 & p0;
+  return *k0 | *k1 | !(p0 | n1);
+}
+
 // The triangle of record rec's entry face, in the record's order, and the
 // ray's crossing of it.  False when its products are not all below -kZero:
 // the general step takes the tet.
@@ -649,9 +663,10 @@ __device__ __forceinline__ bool entry_triangle64(const WalkConf64& W, const Ray6
 // The fast step.  Of the tet's six products (src/dtfe.c:44-64) the entry
 // face's three are the previous step's, up to the exact sign that the
 // reference's formula gives a reversed edge; the apex V adds a_k = U(V, P_k).
-// When all three are clear of kZero the reference enters through the known
-// face and leaves through the one without P_k, a_{k+1} < 0 < a_{k+2} (walk32.cu
-// proves the rule).  The exit crossing and the next tet's entry crossing are
+// When all three are clear of kZero and not of one sign the reference enters
+// through the known face and leaves through the one without P_k, a_{k+1} < 0 <
+// a_{k+2} (walk32.cu proves the rule for all 64 combinations of signs, rounded
+// ones too).  Else the general step decides, on all six products.  The exit crossing and the next tet's entry crossing are
 // the same point of the same triangle, each computed in the order the
 // reference computes it for that face of that tet (crossing64).
 //
@@ -696,11 +711,11 @@ __device__ __forceinline__ int walk64(const WalkConf64& W, int ft, int ft_tri, d
       const double a0 = edge_u64(r, v, make_double2(s.x0, s.y0));
       const double a1 = edge_u64(r, v, make_double2(s.x1, s.y1));
       const double a2 = edge_u64(r, v, make_double2(s.x2, s.y2));
-      const bool sure = Acc::kShortChain ? all_clear(a0, a1, a2)
-                                         : (fabs(a0) > kZero) & (fabs(a1) > kZero) & (fabs(a2) > kZero);
-      // (a_0, a_1, a_2 are not all of one sign)
-      const bool p2 = a2 > 0.0;
-      const bool k0 = p2 & (a1 < 0.0), k1 = !p2 & (a0 > 0.0);  // else k = 2
+      bool k0, k1;
+      const bool found = exit_slot(a0, a1, a2, &k0, &k1);
+      const bool sure = found & (Acc::kShortChain ? all_clear(a0, a1, a2)
+                                                  : (fabs(a0) > kZero) & (fabs(a1) > kZero) &
+                                                        (fabs(a2) > kZero));
       const auto pick = [k0, k1](auto a, auto b, auto c) { return k0 ? a : (k1 ? b : c); };
       const uint32_t next = pick(lk.x, lk.y, lk.z);
       if (sure & (next != kLinkGeneral) & (crossed < W.max_visits)) {

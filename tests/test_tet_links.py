@@ -27,6 +27,7 @@ def tl(tmp_path_factory):
     L = ctypes.CDLL(out)
     L.tl_crossings.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_double] + [ctypes.c_void_p] * 3
     L.tl_rotation.argtypes = [ctypes.c_void_p] * 2
+    L.tl_exit_slot.argtypes = [ctypes.c_void_p]
     return L
 
 
@@ -53,3 +54,11 @@ def test_link_rotation(tl):
         assert r == (want[0] if want else -1)
     other = np.array([7, 3, 8], np.int32)
     assert tl.tl_rotation(other.ctypes.data, w.ctypes.data) == -1
+
+
+def test_exit_slot_for_every_combination_of_signs(tl):
+    """The slot k with a_{k+1} < 0 < a_{k+2}; none when the three products, rounded, have one sign."""
+    for signs in itertools.product((-1.0, 1.0), repeat=3):
+        a = np.array(signs) * [1e-11, 3.0, 1e5]
+        want = [k for k in range(3) if a[(k + 1) % 3] < 0 < a[(k + 2) % 3]]
+        assert tl.tl_exit_slot(a.ctypes.data) == (want[0] if want else -1)

@@ -40,3 +40,10 @@ extern "C" void tl_crossings(const double* v, const double* o, double lz, double
 
 extern "C" int tl_exit_face(int F, int k) { return rot_slot(F, k); }
 extern "C" int tl_rotation(const int* u, const int* w) { return link_rotation(u, w); }
+
+// The slot left behind for apex products a[0..2], or -1.
+extern "C" int tl_exit_slot(const double* a) {
+  bool k0, k1;
+  if (!exit_slot(a[0], a[1], a[2], &k0, &k1)) return -1;
+  return k0 ? 0 : (k1 ? 1 : 2);
+}
