@@ -70,8 +70,9 @@ constexpr int kRankedTets = 128;
 constexpr int kDensityWarps = 8;  // warps a block
 
 // Shell sort over a diminishing gap sequence (Ciura's gaps, then x2.25):
-// O(d^1.3) for the rare hub vertex with hundreds or thousands of tets.  The ids
-// of a list are distinct, so the sorted order is unique.
+// O(d^1.3) for the rare hub vertex with hundreds or thousands of tets.  (A tet
+// that lists a vertex twice is in its list twice; the sorted order is the same
+// whichever comes first.)
 __device__ inline void shell_sort(int* a, int d) {
   constexpr int kGaps[] = {1, 4, 10, 23, 57, 132, 301, 701, 1577, 3548, 7983, 17961, 40412};
   int g = 0;
@@ -90,17 +91,20 @@ __device__ inline void shell_sort(int* a, int d) {
   }
 }
 
-// The places of K tets a lane, at list positions lane, lane + 32, ...
+// The places of K tets a lane, at list positions lane, lane + 32, ...  A tet that
+// lists the vertex several times is in the list as often: equal ids take their
+// places in list order, so that every place is taken.
 template <int K>
 __device__ __forceinline__ void rank_volumes(const int* __restrict__ list, int d,
                                              const double* __restrict__ vol, int lane,
                                              double* row) {
-  int id[K], rank[K];
+  unsigned id[K];
+  int rank[K];
   double v[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const int i = 32 * k + lane;
-    id[k] = i < d ? list[i] : 0x7fffffff;  // (no tet has that id)
+    id[k] = i < d ? (unsigned)list[i] : 0u;  // (no place is taken from d on)
     v[k] = i < d ? vol[id[k]] : 0.0;
     rank[k] = 0;
   }
@@ -108,9 +112,12 @@ __device__ __forceinline__ void rank_volumes(const int* __restrict__ list, int d
   for (int c = 0; c < K; ++c) {
     const int m = min(32, d - 32 * c);
     for (int j = 0; j < m; ++j) {
-      const int other = __shfl_sync(0xffffffffu, id[c], j);
+      const unsigned other = __shfl_sync(0xffffffffu, id[c], j);
 #pragma unroll
-      for (int k = 0; k < K; ++k) rank[k] += other < id[k];
+      for (int k = 0; k < K; ++k) {
+        const bool earlier = c < k || (c == k && j < lane);  // in the list
+        rank[k] += other < id[k] + (unsigned)earlier;
+      }
     }
   }
 #pragma unroll

@@ -74,3 +74,45 @@ def test_a_tet_out_of_range_writes_nothing(bad):
     assert status == 4 and np.all(got == -7.0)  # DTFE_ERR_MESH
     tetra[len(tetra) // 2, 2] = 0
     assert noalloc(pos4, tetra, 1.0)[0] == 0
+
+
+def repeated():
+    """hubs() with tets that list their hub twice, three and four times, some twice in a row of one
+    list, in lists on both sides of 32, 64 and 128, and zero-filled padding rows (vertex 0 four times)."""
+    pos4, tetra = hubs()
+    rng = np.random.default_rng(6)
+    for h, d in enumerate(LENGTHS):
+        mine = np.flatnonzero((tetra[:, :4] == h).any(1))
+        for t in rng.choice(mine, min(d, 5), replace=False):
+            tetra[t, rng.choice(4, rng.integers(1, 5), replace=False)] = h
+    pad = np.zeros((7, 8), np.int32)
+    pad[:, 4:] = -1
+    return pos4, np.concatenate([tetra[:50], pad, tetra[50:]])
+
+
+@pytest.mark.parametrize("tets", [2, 7, 16, 19, 20, 37, 38, 39, 75, 77, 78, 300])
+def test_one_list_of_repeated_tets(tets):
+    """A hub that two of three of its tets list twice: lists on both sides of each length class."""
+    rng = np.random.default_rng(tets)
+    pos4 = np.zeros((60, 4))
+    pos4[:, :3] = rng.random((60, 3))
+    tetra = np.full((tets, 8), -1, np.int32)
+    for row in tetra:
+        row[:4] = rng.permutation([0, 0, *(1 + rng.choice(59, 2, replace=False))])
+    # (tets with the hub twice have next to no volume: every third gets one)
+    tetra[::3, 0] = np.where(tetra[::3, 0] == 0, 1 + rng.integers(59, size=len(tetra[::3])), tetra[::3, 0])
+    status, got = noalloc(pos4, tetra, 1.0)
+    assert status == 0 and np.array_equal(got, expected(pos4, tetra, 1.0))
+
+
+def test_tets_that_list_a_vertex_several_times():
+    import sdtfe_b200 as sd
+
+    pos4, tetra = repeated()
+    want = expected(pos4, tetra, 1.0)
+    for _ in range(3):
+        status, got = noalloc(pos4, tetra, 1.0)
+        assert status == 0 and np.array_equal(got, want)
+    with sd.Mesh(pos4, tetra, 1.0, flags=sd.MESH_LAZY) as m:
+        assert np.array_equal(m.density(), want)
+        assert np.array_equal(m.adjacency(), np.bincount(tetra[:, :4].ravel(), minlength=len(pos4)))
