@@ -234,15 +234,15 @@ __device__ __forceinline__ int grid_ray64(const GridArgs64& a, int i, int j, int
 // and add into the column in walk order, as interpolate_to_3d_grid does
 // (src/dtfe.c:710-729).  No two threads touch the same column.  Marked: after the
 // sub-rays of r, to count the columns' outcomes and walk the irregular ones.
-template <bool Marked>
+template <bool Marked, bool Several>
 __global__ void __launch_bounds__(128) k_grid64(const GridArgs64 a, const GridRays r) {
   int i, j;
   bool active = grid_column(a.G, a.lanes, &i, &j);
   const int marks = Marked && active ? r.col[(size_t)i * a.G + j] : 0;
   int worst = kRayOk, visits = 0;
   if (Marked ? (marks & kIrregular) != 0 : active) {
-    ColumnAcc64<CellSink> acc{{a.grid + ((size_t)i * a.G + j) * a.G, a.ss}, a.offz, a.dzs, a.w,
-                              a.G * a.ss};
+    ColumnAcc64<CellSink<Several>> acc{{a.grid + ((size_t)i * a.G + j) * a.G, a.ss}, a.offz, a.dzs,
+                                       a.w, a.G * a.ss};
     for (int is = 0; is < a.ss; ++is)
       for (int js = 0; js < a.ss; ++js) {
         int c;
@@ -499,9 +499,9 @@ dtfe_status_t launch_grid64(Mesh& m, int G, double box_len, const double center[
       [&](const GridRays& r) {
         k_grid_rays64<<<(unsigned)((ray_warps(r) + 1) / 2), 64, 0, s>>>(a, r);
       },
-      [&](const GridRays& r) { k_grid64<true><<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, r); }));
+      [&](const GridRays& r) { k_grid64<true, true><<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, r); }));
   if (!taken) {
-    k_grid64<false><<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, GridRays{});
+    (ss > 1 ? k_grid64<false, true> : k_grid64<false, false>)<<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, GridRays{});
     count_launch();
   }
   SDTFE_CUDA(cudaGetLastError());

@@ -1347,18 +1347,19 @@ __device__ __forceinline__ int grid_ray32(const GridArgs32& a, int i, int j, int
 }
 
 // One thread per column.  Marked: after the sub-rays of r, to count the columns'
-// outcomes and walk the irregular ones.  MinBlocks: what the registers are
-// limited for; a small grid leaves the SMs few columns, and takes its walks
-// without spills (launch_grid32).
-template <bool Marked, int MinBlocks>
-__global__ void __launch_bounds__(128, MinBlocks)
+// outcomes and walk the irregular ones.  Four blocks per SM leave the walk its
+// registers: on a mesh far larger than L2 (61.8M tets, 512^3) 9.7 ms, five
+// blocks 10.2, six 10.9, seven 12.4; on one within it (83k points) 1.85, 1.86, 1.87
+// and 2.01, and 256^3 0.567, 0.556, 0.557, 0.559.
+template <bool Marked>
+__global__ void __launch_bounds__(128, 4)
     k_grid32(const __grid_constant__ GridArgs32 a, const GridRays r) {
   int i, j;
   bool active = grid_column(a.G, a.lanes, &i, &j);
   const int marks = Marked && active ? r.col[(size_t)i * a.G + j] : 0;
   int worst = kRayOk, visits = 0, fallbacks = 0;
   if (Marked ? (marks & kIrregular) != 0 : active) {
-    auto acc = column_acc32(a, CellSink{a.grid + ((size_t)i * a.G + j) * a.G, a.ss});
+    auto acc = column_acc32(a, CellSink<false>{a.grid + ((size_t)i * a.G + j) * a.G, a.ss});
     for (int is = 0; is < a.ss; ++is)
       for (int js = 0; js < a.ss; ++js) {
         int c, fb;
@@ -1634,13 +1635,9 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
       [&](const GridRays& r) {
         k_grid_rays32<<<(unsigned)((ray_warps(r) + 1) / 2), 64, 0, s>>>(a, r);
       },
-      [&](const GridRays& r) { k_grid32<true, 4><<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, r); }));
+      [&](const GridRays& r) { k_grid32<true><<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, r); }));
   if (!taken) {
-    // four blocks of 128 columns per SM are all of a grid of up to 148 x 512
-    // columns; a larger one gains more from six blocks per SM than it loses to
-    // spills (83k-point lattice: 256^3 0.736 against 0.771 ms, 512^3 2.47 against 2.42)
-    const bool small = (long long)G * G <= 148 * 512;
-    (small ? k_grid32<false, 4> : k_grid32<false, 6>)<<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, GridRays{});
+    k_grid32<false><<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, GridRays{});
     count_launch();
   }
   SDTFE_CUDA(cudaGetLastError());

@@ -370,8 +370,13 @@ struct SurfaceAcc64 {
 // grid column belongs to one thread, and one thread's reductions to one
 // address are performed in its program order, so every cell receives exactly
 // the additions, in the order and with the roundings, of the reference's
-// loop (src/dtfe.c:505-511).
-__device__ __forceinline__ void cell_add(double* cell, double v) { atomicAdd(cell, v); }
+// loop (src/dtfe.c:505-511).  The address space is named: the pointer travels
+// through memory with the accumulator (general_step64), where the compiler loses
+// it and turns an atomicAdd into a generic atomic that returns the old value.
+__device__ __forceinline__ void cell_add(double* cell, double v) {
+  __builtin_assume(__isGlobal(cell));
+  atomicAdd(cell, v);
+}
 
 // The patch of neighbouring columns or rays that a warp walks on its first
 // `lanes` lanes: 4 x 8, 4 x 4 or 2 x 4.  (A launch too small for the GPU takes
