@@ -7,10 +7,11 @@
 // hundred columns a side: 120^2 columns at ss = 2 are 450 warps, each waiting
 // through four walks.  Here every sub-ray has its thread and writes its node
 // values to a row of its own; a second kernel adds each cell's values in the
-// reference's order, so the cells are the same to the bit.  A node no chord
-// holds is written as -0.0, which changes no sum.  A ray that comes back to a
-// node it has passed (after a turn-around or a perturbation) has no place for
-// the second value: its column is marked and walked by the one-thread kernel.
+// reference's order, so the cells are the same to the bit.  A ray says from
+// where to where its row is written; a node in between that no chord holds is
+// written as -0.0, which changes no sum.  A ray that comes back to a node it
+// has passed (after a turn-around or a perturbation) has no place for the
+// second value: its column is marked and walked by the one-thread kernel.
 #pragma once
 
 #include "mesh.h"
@@ -27,7 +28,7 @@ struct CellSink {
   static constexpr bool kShortChain = false;  // reciprocal_near, walk64.cuh
   double* col;
   int ss;
-  __device__ __forceinline__ void begin(int) {}
+  __device__ __forceinline__ void begin(int, int) {}
   __device__ __forceinline__ void put(int is, double v) {
     double* const cell = col + (int)((unsigned)is / (unsigned)ss);
     if constexpr (Several)
@@ -41,16 +42,18 @@ struct CellSink {
 struct NodeSink {
   static constexpr bool kShortChain = true;
   double* row;
-  int done;        // nodes written so far
-  bool irregular;  // came back to one of them
-  __device__ __forceinline__ void begin(int is) {
-    if (is < done) irregular = true;
-    for (; done < is; ++done) row[done] = -0.0;
+  int first;       // the row is written from here (-1: nothing yet)
+  int done;        // to here
+  bool irregular;  // came back to a node it had passed
+  // (a value put on a node passed before is lost, with its column's rows)
+  __device__ __forceinline__ void begin(int i0, int i1) {
+    if (first < 0) first = done = i0;
+    if (i0 < done) irregular = true;
+    for (; done < i0; ++done) put(done, -0.0);
+    done = max(done, i1);
   }
-  __device__ __forceinline__ void put(int is, double v) {
-    if (is < done) return;
-    row[is] = v;
-    done = is + 1;
+  __device__ __forceinline__ void put(int is, double v) const {
+    asm volatile("st.global.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(row + is)), "d"(v));
   }
 };
 
@@ -58,9 +61,10 @@ struct NodeSink {
 struct GridRays {
   int G, ss, lanes;  // lanes: rays a warp walks
   double* nodes;  // row (i*G + j)*ss^2 + is*ss + js of G*ss nodes
-  int* col;       // per column: bit k for a ray of status k, and kIrregular
+  int2* range;    // per ray: the nodes its row holds, [x, y)
+  int* col;       // per column: bit k for a ray of status k, and the two marks
 };
-constexpr int kIrregular = 1 << 8;
+constexpr int kIrregular = 1 << 8, kHasNodes = 1 << 9;
 
 __device__ __forceinline__ int worst_status(int marks) {
   return 31 - __clz((marks & (kIrregular - 1)) | 1);
@@ -87,28 +91,59 @@ inline long long ray_warps(const GridRays& a) {
   return ((nf + pi - 1) / pi) * ((nf + pj - 1) / pj);
 }
 
-__device__ __forceinline__ double* ray_nodes(const GridRays& a, int i, int j, int is, int js) {
-  const size_t ray = (((size_t)i * a.G + j) * a.ss + is) * a.ss + js;
-  return a.nodes + ray * ((size_t)a.G * a.ss);
+__device__ __forceinline__ size_t ray_index(const GridRays& a, int i, int j, int is, int js) {
+  return (((size_t)i * a.G + j) * a.ss + is) * a.ss + js;
+}
+__device__ __forceinline__ NodeSink ray_nodes(const GridRays& a, int i, int j, int is, int js) {
+  return {a.nodes + ray_index(a, i, j, is, js) * ((size_t)a.G * a.ss), -1, 0, false};
 }
 
-__device__ __forceinline__ void ray_done(const GridRays& a, int i, int j, NodeSink& out, int status) {
-  for (const int n = a.G * a.ss; out.done < n; ++out.done) out.row[out.done] = -0.0;
-  atomicOr(a.col + (size_t)i * a.G + j, 1 << status | (out.irregular ? kIrregular : 0));
+__device__ __forceinline__ void ray_done(const GridRays& a, int i, int j, int is, int js,
+                                         const NodeSink& out, int status) {
+  const bool any = out.first >= 0;
+  a.range[ray_index(a, i, j, is, js)] = make_int2(any ? out.first : 0, any ? out.done : 0);
+  atomicOr(a.col + (size_t)i * a.G + j,
+           1 << status | (any ? kHasNodes : 0) | (out.irregular ? kIrregular : 0));
 }
 
-// One thread per cell: its ss^3 node values, sub-ray by sub-ray.
+// One thread per cell: its ss^3 node values, sub-ray by sub-ray.  SS: the usual
+// supersamplings, whose loads are all in flight together (0: any).
+template <int SS>
 __global__ void __launch_bounds__(256) k_grid_sum(const GridRays a, double* __restrict__ grid) {
   const long long cell = blockIdx.x * 256LL + threadIdx.x;
   if (cell >= (long long)a.G * a.G * a.G) return;
   const int iz = (int)(cell % a.G);
   const long long c = cell / a.G;
-  if (a.col[c] & kIrregular) return;
-  const int nzs = a.G * a.ss;
-  const double* v = a.nodes + (size_t)c * a.ss * a.ss * nzs + iz * a.ss;
+  if ((a.col[c] & (kHasNodes | kIrregular)) != kHasNodes) return;
+  const int ss = SS > 0 ? SS : a.ss, nzs = a.G * ss;
+  const double* v = a.nodes + (size_t)c * ss * ss * nzs + iz * ss;
+  const int2* range = a.range + (size_t)c * ss * ss;
   double sum = grid[cell];
-  for (int r = 0; r < a.ss * a.ss; ++r, v += nzs)
-    for (int k = 0; k < a.ss; ++k) sum += v[k];
+  if constexpr (SS > 0) {
+#pragma unroll 1
+    for (int is = 0; is < SS; ++is, v += SS * nzs, range += SS) {
+      double node[SS][SS];
+#pragma unroll
+      for (int js = 0; js < SS; ++js) {
+        const int2 held = range[js];
+#pragma unroll
+        for (int k = 0; k < SS; ++k) {
+          const int n = iz * SS + k;
+          node[js][k] = n >= held.x && n < held.y ? v[js * nzs + k] : -0.0;
+        }
+      }
+#pragma unroll
+      for (int js = 0; js < SS; ++js)
+#pragma unroll
+        for (int k = 0; k < SS; ++k) sum += node[js][k];
+    }
+  } else {
+    for (int r = 0; r < ss * ss; ++r, v += nzs) {
+      const int2 held = range[r];
+      const int k1 = min(held.y - iz * ss, ss);
+      for (int k = max(held.x - iz * ss, 0); k < k1; ++k) sum += v[k];
+    }
+  }
   grid[cell] = sum;
 }
 
@@ -136,25 +171,30 @@ dtfe_status_t grid_by_rays(int G, unsigned ss, int lanes, double* d_grid, cudaSt
   *taken = false;
   if (!grid_takes_rays(G, ss)) return DTFE_OK;
   const size_t n = (size_t)G * ss, col_bytes = sizeof(int) * (size_t)G * G;
-  void *nodes = nullptr, *col = nullptr;
+  void *nodes = nullptr, *range = nullptr, *col = nullptr;
   if (scratch_alloc_async(&nodes, sizeof(double) * n * n * n, s) != DTFE_OK ||
+      scratch_alloc_async(&range, sizeof(int2) * n * n, s) != DTFE_OK ||
       scratch_alloc_async(&col, col_bytes, s) != DTFE_OK) {
     scratch_free_async(nodes, s);
+    scratch_free_async(range, s);
     cudaGetLastError();
     dtfe_clear_error();
     return DTFE_OK;
   }
   *taken = true;
-  const GridRays a{G, (int)ss, lanes, static_cast<double*>(nodes), static_cast<int*>(col)};
+  const GridRays a{G, (int)ss, lanes, static_cast<double*>(nodes), static_cast<int2*>(range),
+                   static_cast<int*>(col)};
   cudaError_t e = cudaMemsetAsync(col, 0, col_bytes, s);
   if (e == cudaSuccess) {
     rays(a);
-    k_grid_sum<<<(unsigned)(((long long)G * G * G + 255) / 256), 256, 0, s>>>(a, d_grid);
+    const auto sum = ss == 2 ? k_grid_sum<2> : (ss == 3 ? k_grid_sum<3> : (ss == 4 ? k_grid_sum<4> : k_grid_sum<0>));
+    sum<<<(unsigned)(((long long)G * G * G + 255) / 256), 256, 0, s>>>(a, d_grid);
     serial(a);
     count_launch(3);
     e = cudaGetLastError();
   }
   scratch_free_async(nodes, s);
+  scratch_free_async(range, s);
   scratch_free_async(col, s);
   SDTFE_CUDA(e);
   return DTFE_OK;

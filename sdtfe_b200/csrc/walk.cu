@@ -263,10 +263,9 @@ __global__ void __launch_bounds__(128) k_grid64(const GridArgs64 a, const GridRa
 __global__ void __launch_bounds__(64) k_grid_rays64(const GridArgs64 a, const GridRays r) {
   int i, j, is, js, c = 0;
   if (ray_of_grid(r, &i, &j, &is, &js)) {
-    ColumnAcc64<NodeSink> acc{{ray_nodes(r, i, j, is, js), 0, false}, a.offz, a.dzs, a.w,
-                              a.G * a.ss};
+    ColumnAcc64<NodeSink> acc{ray_nodes(r, i, j, is, js), a.offz, a.dzs, a.w, a.G * a.ss};
     const int st = grid_ray64(a, i, j, is, js, acc, &c);
-    ray_done(r, i, j, acc.out, st);
+    ray_done(r, i, j, is, js, acc.out, st);
   }
   const unsigned sum = __reduce_add_sync(0xffffffffu, (unsigned)c);
   if ((threadIdx.x & 31) == 0 && sum) atomicAdd(a.stats + kStatVisits, (unsigned long long)sum);
@@ -470,6 +469,17 @@ dtfe_status_t launch_trace64(Mesh& m, int axis, int n_rays, const double* d_x, c
 // sub-rays 0.36 against 0.49).
 static int grid_lanes64(long long n) { return n <= 8192 ? 8 : 32; }
 
+// FP64 grids whose cells outnumber the tets a thousandfold are walked a thread a
+// column even at ss > 1, once the columns fill the GPU: most of their time is
+// the nodes', which a sub-ray writes and another kernel reads again.  One thread a
+// column against sub-rays, ms: 100 points, 200^3 at ss 2 0.40 and 0.50, 400^3 2.15
+// and 3.0; 1000 points, 200^3 0.75 and 0.64, 250^3 1.01 and 1.15, 260^3 at ss 3 3.45
+// and 3.9; 8000 points, 400^3 at ss 2 4.0 and 4.3; below the line, 8000 points, 250^3
+// 1.57 and 1.25, 32k points, 400^3 5.1 and 4.3.  Mixed grids do not gain.
+static bool dense_columns64(int G, int nt) {
+  return G >= 200 && (double)G * G * G >= 1000.0 * nt;
+}
+
 dtfe_status_t launch_grid64(Mesh& m, int G, double box_len, const double center[3], unsigned ss,
                             uint64_t seed, int max_visits, double* d_grid, cudaStream_t s) {
   const AxisData& A = m.ax[DTFE_AXIS_Z];
@@ -494,14 +504,16 @@ dtfe_status_t launch_grid64(Mesh& m, int G, double box_len, const double center[
   SDTFE_CUDA(cudaMemsetAsync(m.stats, 0, sizeof(unsigned long long) * kStatCount, s));
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
   bool taken = false;
-  SDTFE_TRY(grid_by_rays(
-      G, ss, grid_lanes64((long long)G * ss * G * ss), d_grid, s, &taken,
-      [&](const GridRays& r) {
-        k_grid_rays64<<<(unsigned)((ray_warps(r) + 1) / 2), 64, 0, s>>>(a, r);
-      },
-      [&](const GridRays& r) { k_grid64<true, true><<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, r); }));
+  const unsigned blocks = grid_warps(G, a.lanes) / 4;
+  if (!dense_columns64(G, m.nt))
+    SDTFE_TRY(grid_by_rays(
+        G, ss, grid_lanes64((long long)G * ss * G * ss), d_grid, s, &taken,
+        [&](const GridRays& r) {
+          k_grid_rays64<<<(unsigned)((ray_warps(r) + 1) / 2), 64, 0, s>>>(a, r);
+        },
+        [&](const GridRays& r) { k_grid64<true, true><<<blocks, 128, 0, s>>>(a, r); }));
   if (!taken) {
-    (ss > 1 ? k_grid64<false, true> : k_grid64<false, false>)<<<grid_warps(G, a.lanes) / 4, 128, 0, s>>>(a, GridRays{});
+    (ss > 1 ? k_grid64<false, true> : k_grid64<false, false>)<<<blocks, 128, 0, s>>>(a, GridRays{});
     count_launch();
   }
   SDTFE_CUDA(cudaGetLastError());

@@ -608,7 +608,7 @@ struct ColumnAcc32 {
       const double2* f = reinterpret_cast<const double2*>(fld + t.L / 12u);
       const double2 kx = __ldg(f), yz = __ldg(f + 1);
       const double base = kx.x + kx.y * ox + yz.x * oy;
-      out.begin(i0);
+      out.begin(i0, i1);
       for (int is = i0; is < i1; ++is) {
         const double zi = z0 + dzs * is + dzs / 2.;
         out.put(is, (base + yz.y * zi) * w);
@@ -641,7 +641,7 @@ struct ColumnAcc32 {
     const double gx = C.grad[3 * (size_t)t], gy = C.grad[3 * (size_t)t + 1],
                  gz = C.grad[3 * (size_t)t + 2];
     const double fixed = A.w + gx * (r.ox - A.x) + gy * (r.oy - A.y) - gz * A.z;
-    out.begin(i0);
+    out.begin(i0, i1);
     for (int is = i0; is < i1; ++is) {
       const double zi = z0 + dzs * is + dzs / 2.;
       out.put(is, (fixed + gz * zi) * w);
@@ -1383,9 +1383,9 @@ __global__ void __launch_bounds__(64)
     k_grid_rays32(const __grid_constant__ GridArgs32 a, const GridRays r) {
   int i, j, is, js, c = 0, fb = 0;
   if (ray_of_grid(r, &i, &j, &is, &js)) {
-    auto acc = column_acc32(a, NodeSink{ray_nodes(r, i, j, is, js), 0, false});
+    auto acc = column_acc32(a, ray_nodes(r, i, j, is, js));
     const int st = grid_ray32(a, i, j, is, js, acc, &c, &fb);
-    ray_done(r, i, j, acc.out, st);
+    ray_done(r, i, j, is, js, acc.out, st);
   }
   const unsigned v = __reduce_add_sync(0xffffffffu, (unsigned)c);
   const unsigned f = __reduce_add_sync(0xffffffffu, (unsigned)fb);

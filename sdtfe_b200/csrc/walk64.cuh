@@ -426,7 +426,7 @@ struct ColumnAcc64 {
     if (i1 > i0) {
       const double4 A = load256(&r.t->v[0]), f = load256(&r.t->f);
       const double fixed = f.x + f.y * (ox - A.x) + f.z * (oy - A.y) - f.w * A.z;
-      out.begin(i0);
+      out.begin(i0, i1);
       for (int is = i0; is < i1; ++is) {
         const double zi = z0 + dzs * is + dzs / 2.;
         out.put(is, (fixed + f.w * zi) * w);
