@@ -82,7 +82,7 @@ dtfe_status_t plan(dtfe_batch_s* b) {
     SDTFE_TRY(batch_grid32(b->plan.variant, b->plan.smem, &b->grid, &b->block));
   } else {
     SDTFE_TRY(plan_batch64(maps.data(), n, &b->plan));
-    SDTFE_TRY(batch_grid64(b->plan.smem, &b->grid, &b->block));
+    SDTFE_TRY(batch_grid64(&b->plan, &b->grid, &b->block));
   }
   const size_t bytes = b->plan.jobs.size();
   if (bytes > b->d_jobs_bytes) {
@@ -118,7 +118,7 @@ dtfe_status_t enqueue(dtfe_batch_s* b, cudaStream_t s) {
       SDTFE_CUDA(cudaMemsetAsync(j.d_map, 0, sizeof(double) * (size_t)j.params.grid_dim * j.params.grid_dim, s));
   if (b->precision == DTFE_MIXED)
     return launch_batch32(b->plan, b->d_jobs, b->d_queue, b->d_loc, b->grid, s);
-  return launch_batch64(b->plan, b->d_jobs, b->d_queue, b->grid, s);
+  return launch_batch64(b->plan, b->d_jobs, b->d_queue, s);
 }
 
 dtfe_status_t launch(dtfe_batch_s* b, cudaStream_t s) {
@@ -139,8 +139,9 @@ dtfe_status_t launch(dtfe_batch_s* b, cudaStream_t s) {
     }
     SDTFE_CUDA(cudaEventRecord(b->ev0, s));
     SDTFE_CUDA(cudaGraphLaunch(b->exec, s));
-    // the graph's kernel nodes: the mixed path's tile locations, then the walk
-    count_launch(b->plan.n_jobs ? (b->precision == DTFE_MIXED ? 2 : 1) : 0);
+    // the graph's kernel nodes: the mixed path's tile locations, then the walk; the
+    // FP64 path's parts
+    count_launch(b->precision == DTFE_MIXED ? (b->plan.n_jobs ? 2 : 0) : (unsigned)b->plan.parts.size());
   } else {
     SDTFE_CUDA(cudaEventRecord(b->ev0, s));
     SDTFE_TRY(enqueue(b, s));

@@ -177,6 +177,13 @@ struct BatchPlan {
   int n_jobs = 0;
   long long total_tiles = 0;
   size_t smem = 0;            // dynamic shared memory per block
+  // FP64: a launch per block size, each over its jobs of the table
+  struct Part {
+    int block = 0, first = 0, n_jobs = 0, grid = 0;
+    long long tiles = 0;
+    size_t smem = 0;
+  };
+  std::vector<Part> parts;
   std::vector<unsigned char> jobs;  // the job table as the kernel reads it
 };
 // tiles of a whole map (the tile shape depends on precision and variant)
@@ -184,12 +191,13 @@ int map_tiles64(const MapGeom& g);
 int map_tiles32(const MapGeom& g, int variant);
 dtfe_status_t plan_batch64(const BatchMap* maps, int n, BatchPlan* plan);
 dtfe_status_t plan_batch32(const BatchMap* maps, int n, int variant, BatchPlan* plan);
-// blocks of a persistent launch: resident blocks per SM x SMs
-dtfe_status_t batch_grid64(size_t smem, int* grid, int* block);
+// blocks of a persistent launch: resident blocks per SM x SMs (FP64: into the
+// plan's parts; *grid and *block are the first one's)
+dtfe_status_t batch_grid64(BatchPlan* plan, int* grid, int* block);
 dtfe_status_t batch_grid32(int variant, size_t smem, int* grid, int* block);
 // d_jobs holds plan.jobs; d_queue is a zeroed counter
 dtfe_status_t launch_batch64(const BatchPlan& plan, const void* d_jobs, unsigned long long* d_queue,
-                             int grid, cudaStream_t s);
+                             cudaStream_t s);
 // (mixed) d_loc: room for plan.total_tiles tile locations (kLocBytes each)
 dtfe_status_t launch_batch32(const BatchPlan& plan, const void* d_jobs, unsigned long long* d_queue,
                              void* d_loc, int grid, cudaStream_t s);

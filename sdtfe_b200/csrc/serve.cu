@@ -373,8 +373,8 @@ dtfe_status_t launch_iteration(Server* S, Slot& sl, const std::vector<std::pair<
   }
   if (plans[1].n_jobs) {
     int grid = 0, block = 0;
-    SDTFE_TRY(batch_grid64(plans[1].smem, &grid, &block));
-    SDTFE_TRY(launch_batch64(plans[1], dj + b0, sl.d_queue + 1, grid, s));
+    SDTFE_TRY(batch_grid64(&plans[1], &grid, &block));
+    SDTFE_TRY(launch_batch64(plans[1], dj + b0, sl.d_queue + 1, s));
     ++S->st.iterations;
   }
   SDTFE_CUDA(cudaEventRecord(sl.ev, s));

@@ -26,7 +26,17 @@ namespace {
 // 128 registers 10.03 ms, 4 x 128 9.77, 10 x 64 of 96 9.39, 12 x 64 of 80 10.7
 // (spills in the loop).  Blocks of two warps also lose less at the end-of-tile
 // barrier than blocks of eight.
-constexpr int kBlock64 = 64, kBlocks64 = 10;
+constexpr int kBlock64 = 64;
+// A pixel's samples are one block's, and take 9 B each of its shared memory.  64
+// threads fit 65 samples badly, and with thousands an SM holds few such blocks: maps
+// of more than 64 samples walk 128 a block (131k clustered points, ms with 64 and 128:
+// 100^2 x 80 3.41 and 2.65, 64^2 x 257 4.27 and 3.68, 64^2 x 1000 14.7 and 12.1), and
+// beyond 4096, or with few pixels, 256 (with 64, 128 and 256: 24^2 x 3000 25.3, 11.4
+// and 8.9, 28^2 x 6000 63, 42.6 and 20.7; the line between 128 and 256 is near 48^2
+// pixels at 400 and at 1000 samples).
+constexpr int kFewPixels64 = 2600;
+constexpr int map_block64(int S) { return S <= 64 ? kBlock64 : (S <= 4096 ? 128 : 256); }
+constexpr int map_min_blocks64(int block) { return block == 64 ? 10 : (block == 128 ? 5 : 2); }
 
 struct MapArgs64 {
   const TriRec64* __restrict__ tri;
@@ -122,7 +132,8 @@ __device__ __forceinline__ void map_tile64(const MapArgs64& a, int tile, double*
   }
 }
 
-__global__ void __launch_bounds__(kBlock64, kBlocks64) k_map64(const MapArgs64 a) {
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, map_min_blocks64(BLOCK)) k_map64(const MapArgs64 a) {
   extern __shared__ double s_val[];  // P*S doubles, then P*S bytes of success flags
   unsigned char* s_ok = reinterpret_cast<unsigned char*>(s_val + a.TW * a.TH * a.S);
   map_tile64(a, blockIdx.x, s_val, s_ok);
@@ -152,9 +163,10 @@ __device__ __forceinline__ void claim_tile64(const BatchJob64* __restrict__ jobs
   *job = lo;
 }
 
-__global__ void __launch_bounds__(kBlock64, kBlocks64) k_batch64(const BatchJob64* __restrict__ jobs, int n_jobs,
-                                                 long long total_tiles,
-                                                 unsigned long long* __restrict__ queue) {
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, map_min_blocks64(BLOCK))
+    k_batch64(const BatchJob64* __restrict__ jobs, int n_jobs, long long total_tiles,
+              unsigned long long* __restrict__ queue) {
   extern __shared__ double s_val[];
   __shared__ MapArgs64 s_args;
   __shared__ long long s_tile[2];
@@ -296,9 +308,9 @@ MapGeom map_geometry(const Mesh& m, const dtfe_map_params_t& p) {
   return g;
 }
 
-// tile of pixels per block: TW x TH pixels x S samples <= kBlock64 threads
-static void tile_shape(int S, int* TW, int* TH) {
-  int P = kBlock64 / S;
+// tile of pixels per block: TW x TH pixels x S samples <= block threads
+static void tile_shape(int S, int block, int* TW, int* TH) {
+  int P = block / S;
   if (P < 1) P = 1;
   int lg = 31 - __builtin_clz((unsigned)P);
   int tw = 1 << ((lg + 1) / 2);
@@ -315,7 +327,7 @@ static WalkConf64 walk_conf64(const Mesh& m, int axis, double lz, double dist, u
 }
 
 // The kernel arguments of one FP64 map; *tiles_y receives its rows of tiles.
-static dtfe_status_t map_args64(Mesh& m, const MapGeom& g, double* d_map,
+static dtfe_status_t map_args64(Mesh& m, const MapGeom& g, int block, double* d_map,
                                 unsigned long long* stats, double* ray_rho, int* ray_crossed,
                                 int* ray_status, MapArgs64* out, int* tiles_y) {
   const AxisData& A = m.ax[g.axis];
@@ -326,7 +338,7 @@ static dtfe_status_t map_args64(Mesh& m, const MapGeom& g, double* d_map,
   a.map = d_map;
   a.G = g.G;
   a.S = g.S;
-  tile_shape(g.S, &a.TW, &a.TH);
+  tile_shape(g.S, block, &a.TW, &a.TH);
   a.tiles_x = (g.G + a.TW - 1) / a.TW;
   *tiles_y = (g.G + a.TH - 1) / a.TH;
   a.dxy = g.dxy;
@@ -350,13 +362,15 @@ dtfe_status_t launch_map64(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
                            double* ray_rho, int* ray_crossed, int* ray_status) {
   MapArgs64 a;
   int tiles_y = 0;
-  SDTFE_TRY(map_args64(m, g, d_map, m.stats, ray_rho, ray_crossed, ray_status, &a, &tiles_y));
+  const int block = (long long)g.G * g.G < kFewPixels64 && g.S > 64 ? 256 : map_block64(g.S);
+  SDTFE_TRY(map_args64(m, g, block, d_map, m.stats, ray_rho, ray_crossed, ray_status, &a, &tiles_y));
   const int P = a.TW * a.TH;
   int threads = P * g.S;
-  threads = threads > kBlock64 ? kBlock64 : ((threads + 31) / 32) * 32;
+  threads = threads > block ? block : ((threads + 31) / 32) * 32;
+  const auto kernel = block == 64 ? k_map64<64> : (block == 128 ? k_map64<128> : k_map64<256>);
   const size_t smem = (size_t)P * g.S * (sizeof(double) + 1);
   if (smem > 48 * 1024)
-    SDTFE_CUDA(cudaFuncSetAttribute(k_map64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SDTFE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long long blocks = (long long)a.tiles_x * tiles_y;
   const bool tile_loc = m.fp64_location == DTFE_LOCATE_TILE && a.n_tri > 0;
   if (tile_loc && a.n_tri >= (1 << 27))
@@ -372,7 +386,7 @@ dtfe_status_t launch_map64(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
     count_launch();
     a.loc = static_cast<const int2*>(loc);
   }
-  k_map64<<<(unsigned)blocks, threads, smem, s>>>(a);
+  kernel<<<(unsigned)blocks, threads, smem, s>>>(a);
   count_launch();
   const cudaError_t e = cudaGetLastError();
   if (loc) scratch_free_async(loc, s);
@@ -384,8 +398,12 @@ dtfe_status_t launch_map64(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
 
 int map_tiles64(const MapGeom& g) {
   int TW, TH;
-  tile_shape(g.S, &TW, &TH);
+  tile_shape(g.S, map_block64(g.S), &TW, &TH);
   return ((g.G + TW - 1) / TW) * ((g.G + TH - 1) / TH);
+}
+
+static auto batch_kernel64(int block) {
+  return block == 64 ? k_batch64<64> : (block == 128 ? k_batch64<128> : k_batch64<256>);
 }
 
 dtfe_status_t plan_batch64(const BatchMap* maps, int n, BatchPlan* plan) {
@@ -394,53 +412,79 @@ dtfe_status_t plan_batch64(const BatchMap* maps, int n, BatchPlan* plan) {
   plan->n_jobs = 0;
   plan->total_tiles = 0;
   plan->smem = 0;
+  plan->parts.clear();
   plan->jobs.assign(sizeof(BatchJob64) * (size_t)(n > 0 ? n : 0), 0);
-  for (int i = 0; i < n; ++i) {
-    const BatchMap& b = maps[i];
-    BatchJob64 j;
-    int tiles_y = 0;
-    SDTFE_TRY(map_args64(*b.mesh, b.g, b.d_map, b.stats, nullptr, nullptr, nullptr, &j.args, &tiles_y));
-    const long long tiles = (long long)j.args.tiles_x * tiles_y;
-    const long long cnt = b.count < 0 ? tiles - b.tile0 : b.count;
-    if (b.tile0 < 0 || cnt < 0 || b.tile0 + cnt > tiles)
-      return set_error(DTFE_ERR_INVALID, "batch map %d: tiles [%d, %lld) outside the map's %lld", i,
-                       b.tile0, b.tile0 + cnt, tiles);
-    if (cnt == 0) continue;
-    j.first = plan->total_tiles;
-    j.tile0 = b.tile0;
-    j.count = (int)cnt;
-    memcpy(plan->jobs.data() + sizeof(BatchJob64) * plan->n_jobs, &j, sizeof(j));
-    ++plan->n_jobs;
-    plan->total_tiles += cnt;
-    const size_t smem = (size_t)j.args.TW * j.args.TH * j.args.S * (sizeof(double) + 1);
-    if (smem > plan->smem) plan->smem = smem;
+  for (const int block : {256, 128, 64}) {
+    BatchPlan::Part part;
+    part.block = block;
+    part.first = plan->n_jobs;
+    for (int i = 0; i < n; ++i) {
+      const BatchMap& b = maps[i];
+      if (map_block64(b.g.S) != block) continue;
+      BatchJob64 j;
+      int tiles_y = 0;
+      SDTFE_TRY(map_args64(*b.mesh, b.g, block, b.d_map, b.stats, nullptr, nullptr, nullptr, &j.args,
+                           &tiles_y));
+      const long long tiles = (long long)j.args.tiles_x * tiles_y;
+      const long long cnt = b.count < 0 ? tiles - b.tile0 : b.count;
+      if (b.tile0 < 0 || cnt < 0 || b.tile0 + cnt > tiles)
+        return set_error(DTFE_ERR_INVALID, "batch map %d: tiles [%d, %lld) outside the map's %lld", i,
+                         b.tile0, b.tile0 + cnt, tiles);
+      if (cnt == 0) continue;
+      j.first = part.tiles;
+      j.tile0 = b.tile0;
+      j.count = (int)cnt;
+      memcpy(plan->jobs.data() + sizeof(BatchJob64) * plan->n_jobs, &j, sizeof(j));
+      ++plan->n_jobs;
+      ++part.n_jobs;
+      part.tiles += cnt;
+      const size_t smem = (size_t)j.args.TW * j.args.TH * j.args.S * (sizeof(double) + 1);
+      if (smem > part.smem) part.smem = smem;
+    }
+    plan->total_tiles += part.tiles;
+    if (part.n_jobs) plan->parts.push_back(part);
   }
   plan->jobs.resize(sizeof(BatchJob64) * plan->n_jobs);
   return DTFE_OK;
 }
 
-dtfe_status_t batch_grid64(size_t smem, int* grid, int* block) {
-  int dev = 0, sms = 0, per_sm = 0;
+dtfe_status_t batch_grid64(BatchPlan* plan, int* grid, int* block) {
+  int dev = 0, sms = 0;
   SDTFE_CUDA(cudaGetDevice(&dev));
   SDTFE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (smem > 48 * 1024)
-    SDTFE_CUDA(cudaFuncSetAttribute(k_batch64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  SDTFE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch64, kBlock64, smem));
-  if (per_sm < 1) return set_error(DTFE_ERR_UNSUPPORTED, "FP64 batch: %zu B of shared memory per block", smem);
-  *grid = per_sm * sms;
+  *grid = 0;
   *block = kBlock64;
+  for (BatchPlan::Part& part : plan->parts) {
+    const auto kernel = batch_kernel64(part.block);
+    int per_sm = 0;
+    if (part.smem > 48 * 1024)
+      SDTFE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)part.smem));
+    SDTFE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, part.block, part.smem));
+    if (per_sm < 1)
+      return set_error(DTFE_ERR_UNSUPPORTED, "FP64 batch: %zu B of shared memory per block", part.smem);
+    part.grid = per_sm * sms;
+  }
+  if (!plan->parts.empty()) {
+    *grid = plan->parts[0].grid;
+    *block = plan->parts[0].block;
+  }
   return DTFE_OK;
 }
 
 dtfe_status_t launch_batch64(const BatchPlan& plan, const void* d_jobs, unsigned long long* d_queue,
-                             int grid, cudaStream_t s) {
-  if (plan.n_jobs == 0) return DTFE_OK;
-  if (plan.smem > 48 * 1024)
-    SDTFE_CUDA(cudaFuncSetAttribute(k_batch64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
-  k_batch64<<<grid, kBlock64, plan.smem, s>>>(static_cast<const BatchJob64*>(d_jobs), plan.n_jobs,
-                                         plan.total_tiles, d_queue);
-  count_launch();
-  SDTFE_CUDA(cudaGetLastError());
+                             cudaStream_t s) {
+  const BatchJob64* jobs = static_cast<const BatchJob64*>(d_jobs);
+  bool used = false;  // the queue counter, which the caller has cleared for the first part
+  for (const BatchPlan::Part& part : plan.parts) {
+    const auto kernel = batch_kernel64(part.block);
+    if (part.smem > 48 * 1024)
+      SDTFE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)part.smem));
+    if (used) SDTFE_CUDA(cudaMemsetAsync(d_queue, 0, sizeof(unsigned long long), s));
+    used = true;
+    kernel<<<part.grid, part.block, part.smem, s>>>(jobs + part.first, part.n_jobs, part.tiles, d_queue);
+    count_launch();
+    SDTFE_CUDA(cudaGetLastError());
+  }
   return DTFE_OK;
 }
 
