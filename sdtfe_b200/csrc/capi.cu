@@ -52,13 +52,13 @@ dtfe_status_t check_params(const Mesh& m, const dtfe_map_params_t* p) {
 }
 
 // records + hull for the map's axis and precision, on the mesh stream
-dtfe_status_t prepare_axis(Mesh& m, int axis, int precision) {
+dtfe_status_t prepare_axis(Mesh& m, int axis, int precision, bool links) {
   if (!m.grad) SDTFE_TRY(mesh_gradients(&m));
   // the mixed walk reads FP64 records only when the coordinates are not floats
   const bool want64 = precision == DTFE_FP64 ||
                       (!m.fp32_exact && !(m.flags & DTFE_MESH_NO_FP64_REC));
   const bool want32 = precision == DTFE_MIXED;
-  SDTFE_TRY(mesh_records(&m, axis, want64, want32));
+  SDTFE_TRY(mesh_records(&m, axis, want64, want32, links));
   SDTFE_TRY(mesh_hull(&m, axis, nullptr, nullptr));
   return DTFE_OK;
 }
@@ -249,6 +249,7 @@ dtfe_status_t dtfe_map_device(dtfe_mesh_t h, const dtfe_map_params_t* p, double*
   const AxisData& A = m.ax[p->axis];
   const bool ready = A.hull_built && (p->precision == DTFE_FP64 ? A.rec64 != nullptr
                                                                  : A.geo32 != nullptr &&
+                                                                       (m.link || !mesh_link_bytes(m)) &&
                                                                        (m.fp32_exact || A.rec64));
   cudaStream_t s = stream ? (cudaStream_t)stream : m.stream;
   if (!ready) {

@@ -533,44 +533,84 @@ dtfe_status_t mesh_field64(Mesh* m) {
 }
 
 static bool has_links(const Mesh& m) { return m.nt <= kMaxLinkedTets; }
-static size_t link_bytes(const Mesh& m) {
+
+// device bytes of a mesh's links (0: it is too large for any)
+size_t mesh_link_bytes(const Mesh& m) {
   return has_links(m) ? kLinkRowsPerTet * sizeof(uint4) * (size_t)m.nt : 0;
 }
 
-dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32) {
+// The links, which all axes and both precisions share.  Where a walk may be running
+// on records built before, on any stream, they are not shown to it until they are
+// complete.
+static dtfe_status_t build_links(Mesh* m, bool in_use) {
+  uint4* link = nullptr;
+  const size_t rows = kLinkRowsPerTet * (size_t)m->nt;
+  SDTFE_TRY(dmalloc_async(&link, rows, m));
+  cudaError_t e = cudaSuccess;
+  if (m->nt) {
+    k_links<<<grid_for(4LL * m->nt), kBlock, 0, m->stream>>>(m->rows, m->nt, link);
+    count_launch();
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess && in_use) e = cudaStreamSynchronize(m->stream);
+  if (e != cudaSuccess) {
+    dfree_async(link, rows, m);
+    return set_error(DTFE_ERR_CUDA, "walk links: %s", cudaGetErrorString(e));
+  }
+  m->link = link;
+  return DTFE_OK;
+}
+
+static bool any_records(const Mesh& m) {
+  bool any = false;
+  for (const AxisData& A : m.ax) any = any || A.rec64 || A.geo32;
+  return any;
+}
+
+dtfe_status_t mesh_links(Mesh* m) {
+  return m->link || !has_links(*m) ? DTFE_OK : build_links(m, any_records(*m));
+}
+
+dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32, bool want_links) {
   if (axis < 0 || axis > 2) return set_error(DTFE_ERR_INVALID, "axis %d not in 0..2", axis);
   if (!m->grad) return set_error(DTFE_ERR_INVALID, "mesh_records before mesh_gradients");
   AxisData& A = m->ax[axis];
   const bool need64 = want64 && !A.rec64, need32 = want32 && !A.geo32;
-  if (!need64 && !need32) return DTFE_OK;
+  // The mixed walk has links (but for a mesh too large to have any): a map's low bits
+  // depend on them.  The FP64 walk's do not, and where there is no memory for
+  // links it takes general steps alone.
+  const bool need_links = want32 && !m->link && has_links(*m);
+  if (!need64 && !need32 && !need_links) return DTFE_OK;
   // the mixed walk's records address 4*t + F in an int: up to 2^29 - 1 tets
   if (need32 && m->nt >= (1 << 29))
     return set_error(DTFE_ERR_UNSUPPORTED, "mixed maps of %d tets (at most 2^29 - 1)", m->nt);
-  const bool links = !A.link && has_links(*m);
+  const bool in_use = any_records(*m);
   // all or nothing: a record array that exists has been built; stream-ordered
   // allocations, so that building records for one mesh does not stall the
   // device (the serving loop builds and drops them while maps run)
   dtfe_status_t st = DTFE_OK;
   if (need64) st = dmalloc_async(&A.rec64, m->nt, m);
   if (st == DTFE_OK && need32) st = dmalloc_async(&A.geo32, 4 * (size_t)m->nt, m);
-  if (st == DTFE_OK && links) st = dmalloc_async(&A.link, kLinkRowsPerTet * (size_t)m->nt, m);
-  if (st == DTFE_OK && m->nt) {
+  if (st == DTFE_OK && (need64 || need32) && m->nt) {
     k_records<<<grid_for(m->nt), kBlock, 0, m->stream>>>(m->pos, m->rows, m->grad, m->nt, axis,
                                                          need64 ? A.rec64 : nullptr,
                                                          need32 ? A.geo32 : nullptr);
     count_launch();
-    if (links) {
-      k_links<<<grid_for(4LL * m->nt), kBlock, 0, m->stream>>>(m->rows, m->nt, A.link);
-      count_launch();
-    }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
       st = set_error(DTFE_ERR_CUDA, "walk records: %s", cudaGetErrorString(e));
   }
+  if (st == DTFE_OK && (need_links || (want_links && !m->link && has_links(*m)))) {
+    st = build_links(m, in_use);
+    if (st == DTFE_ERR_NOMEM && !need_links) {
+      cudaGetLastError();
+      dtfe_clear_error();
+      st = DTFE_OK;
+    }
+  }
   if (st != DTFE_OK) {
     if (need64) dfree_async(A.rec64, m->nt, m);
     if (need32) dfree_async(A.geo32, 4 * (size_t)m->nt, m);
-    if (links) dfree_async(A.link, kLinkRowsPerTet * (size_t)m->nt, m);
     return st;
   }
   return DTFE_OK;
@@ -579,8 +619,7 @@ dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32) {
 size_t mesh_record_bytes(const Mesh& m, int axis) {
   const AxisData& A = m.ax[axis];
   const size_t nt = (size_t)m.nt;
-  return (A.geo32 ? 4 * sizeof(TetGeo32) * nt : 0) + (A.rec64 ? sizeof(TetRec64) * nt : 0) +
-         (A.link ? link_bytes(m) : 0);
+  return (A.geo32 ? 4 * sizeof(TetGeo32) * nt : 0) + (A.rec64 ? sizeof(TetRec64) * nt : 0);
 }
 
 size_t mesh_missing_record_bytes(const Mesh& m, int axis, int precision) {
@@ -588,7 +627,6 @@ size_t mesh_missing_record_bytes(const Mesh& m, int axis, int precision) {
   const size_t nt = (size_t)m.nt;
   size_t b = 0;
   if (precision == DTFE_MIXED && !A.geo32) b += 4 * sizeof(TetGeo32) * nt;
-  if (!A.link) b += link_bytes(m);
   // the mixed walk reads FP64 records only when the coordinates are not floats
   const bool want64 = precision == DTFE_FP64 ||
                       (!m.fp32_exact && !(m.flags & DTFE_MESH_NO_FP64_REC));
@@ -596,14 +634,18 @@ size_t mesh_missing_record_bytes(const Mesh& m, int axis, int precision) {
   return b;
 }
 
+// Frees the links (the caller has no map of the mesh in flight), ordered on the
+// mesh stream.
+void mesh_drop_links(Mesh* m) { dfree_async(m->link, kLinkRowsPerTet * (size_t)m->nt, m); }
+
 // Frees one axis' walk records (the caller has no map of that axis in flight),
-// ordered on the mesh stream.
+// and with the mesh's last records the links, ordered on the mesh stream.
 void mesh_drop_records(Mesh* m, int axis) {
   if (axis < 0 || axis > 2) return;
   AxisData& A = m->ax[axis];
   dfree_async(A.rec64, m->nt, m);
   dfree_async(A.geo32, 4 * (size_t)m->nt, m);
-  dfree_async(A.link, kLinkRowsPerTet * (size_t)m->nt, m);
+  if (!any_records(*m)) mesh_drop_links(m);
 }
 
 dtfe_status_t mesh_hull_mask(Mesh* m, int axis, uint32_t* host_mask_out, int* count_out) {
@@ -708,8 +750,8 @@ void mesh_free(Mesh* m) {
   for (auto& A : m->ax) {
     dfree_async(A.rec64, m->nt, m);
     dfree_async(A.geo32, 4 * (size_t)m->nt, m);
-    dfree_async(A.link, kLinkRowsPerTet * (size_t)m->nt, m);
   }
+  mesh_drop_links(m);
   dfree_async(m->fld64, m->nt, m);
   dfree_async(m->pos, m->n, m);
   dfree_async(m->rows, 2 * (size_t)m->nt, m);

@@ -55,7 +55,6 @@ struct AxisData {
   // walk records in this axis' projected frame (built on demand, per precision)
   TetRec64* rec64 = nullptr;
   TetGeo32* geo32 = nullptr;  // 4 per tet (one per entry face): the mixed walk's records
-  uint4* link = nullptr;      // 12 per tet: their links (none beyond kMaxLinkedTets)
 };
 
 struct Mesh {
@@ -70,6 +69,8 @@ struct Mesh {
   int4* rows = nullptr;     // 2 per tet: vertex ids, neighbour ids
   double* grad = nullptr;   // 3 per tet
   int* adj = nullptr;       // tets incident to each vertex
+  uint4* link = nullptr;    // 12 per tet: the links between all axes' records, or none
+                            // (beyond kMaxLinkedTets, or without the memory for them)
   double4* fld64 = nullptr; // per-tet FP64 field (k, grad) of the mixed 3-D grid (on demand)
   AxisData ax[3];
   unsigned long long* stats = nullptr;  // kStatCount counters of the last map
@@ -92,13 +93,17 @@ dtfe_status_t mesh_upload(Mesh* m, const double* particle_data, int n, const int
                           int nt, float p_mass, unsigned flags);
 dtfe_status_t mesh_density(Mesh* m);
 dtfe_status_t mesh_gradients(Mesh* m);
-dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32);
+dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32, bool want_links);
+// the links alone, for a mesh that went without
+dtfe_status_t mesh_links(Mesh* m);
 // the mixed 3-D grid's per-tet FP64 field (k_field64), built once on the mesh stream
 dtfe_status_t mesh_field64(Mesh* m);
 void mesh_drop_records(Mesh* m, int axis);
+void mesh_drop_links(Mesh* m);
 // device bytes of one axis' walk records: held now, and still to build for a
-// map of the given precision
+// map of the given precision (mesh_missing_record_bytes); of the mesh's links
 size_t mesh_record_bytes(const Mesh& m, int axis);
+size_t mesh_link_bytes(const Mesh& m);
 // returns the current device's cached, unused walk-record memory to the system
 void mesh_trim_record_pool();
 // per-call device scratch, stream-ordered on s from the walk-record pool
@@ -128,9 +133,10 @@ __host__ __device__ inline void permute3(int axis, double x, double y, double z,
 }
 
 // capi.cu: parameter checks, and the records + hull a map of (axis,
-// precision) reads, built on the mesh stream
+// precision) reads, built on the mesh stream (links false: an FP64 map does without
+// links if the mesh has none)
 dtfe_status_t check_params(const Mesh& m, const dtfe_map_params_t* p);
-dtfe_status_t prepare_axis(Mesh& m, int axis, int precision);
+dtfe_status_t prepare_axis(Mesh& m, int axis, int precision, bool links = true);
 
 // walk.cu / walk32.cu launchers
 struct MapGeom {

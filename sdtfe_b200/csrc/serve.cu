@@ -139,12 +139,35 @@ void note_use(Server* S) {
   if (S->in_use > S->peak) S->peak = S->in_use;
 }
 
-// drops idle records, least recently used first, until `need` more bytes fit
-bool make_room(Server* S, size_t need, std::pair<int, int> keep) {
-  while (S->in_use + need > S->cfg.device_budget) {
+// Records are resident by (mesh, axis); a mesh's links, which its axes share, are
+// under (mesh, kLinks) and go with its last records.
+constexpr int kLinks = 3;
+
+// Whether a mesh holds records that its owner built beside the server's: its links
+// are then the owner's too, neither dropped nor under the budget.
+bool owner_has_records(Server* S, int mesh_id, const Mesh& m) {
+  for (int a = 0; a < 3; ++a) {
+    const auto it = S->resident.find({mesh_id, a});
+    if (record_bytes(m, a) > (it == S->resident.end() ? 0 : it->second.bytes)) return true;
+  }
+  return false;
+}
+
+void count_links(Server* S, int mesh_id, const Mesh& m) {
+  Resident& r = S->resident[{mesh_id, kLinks}];
+  const size_t bytes = m.link && !owner_has_records(S, mesh_id, m) ? mesh_link_bytes(m) : 0;
+  S->in_use += bytes - r.bytes;
+  r.bytes = bytes;
+}
+
+// drops idle records, least recently used first, until need() more bytes fit
+template <class Need>
+bool make_room(Server* S, const Need& need, std::pair<int, int> keep) {
+  while (S->in_use + need() > S->cfg.device_budget) {
     auto victim = S->resident.end();
     for (auto it = S->resident.begin(); it != S->resident.end(); ++it) {
       if (it->second.refs > 0 || it->first == keep || it->second.bytes == 0) continue;
+      if (it->first.second == kLinks) continue;
       if (victim == S->resident.end() || it->second.last_use < victim->second.last_use) victim = it;
     }
     if (victim == S->resident.end()) return false;
@@ -155,6 +178,7 @@ bool make_room(Server* S, size_t need, std::pair<int, int> keep) {
     }
     S->in_use -= victim->second.bytes;
     victim->second.bytes = 0;
+    count_links(S, victim->first.first, h->m);
     ++S->st.evictions;
   }
   return true;
@@ -194,7 +218,7 @@ void release(Server* S, Request* r) {
   S->active.erase(std::remove(S->active.begin(), S->active.end(), r), S->active.end());
 }
 
-dtfe_status_t admit_one(Server* S, Request* r) {
+dtfe_status_t admit_one(Server* S, Request* r, bool links) {
   dtfe_mesh_t h = S->meshes[r->mesh_id];
   Mesh& m = h->m;
   const std::pair<int, int> key{r->mesh_id, r->p.axis};
@@ -202,10 +226,13 @@ dtfe_status_t admit_one(Server* S, Request* r) {
   {
     std::lock_guard<std::mutex> lk(h->mu);
     const size_t before = record_bytes(m, r->p.axis);
-    SDTFE_TRY(prepare_axis(m, r->p.axis, r->p.precision));
+    dtfe_status_t st = prepare_axis(m, r->p.axis, r->p.precision, links);
+    if (st == DTFE_OK && links) st = mesh_links(&m);
     const size_t after = record_bytes(m, r->p.axis);
     res.bytes += after - before;
     S->in_use += after - before;
+    count_links(S, r->mesh_id, m);
+    SDTFE_TRY(st);
     SDTFE_CUDA(cudaEventRecord(S->ev_setup, m.stream));
     SDTFE_CUDA(cudaStreamWaitEvent(S->setup, S->ev_setup, 0));
   }
@@ -245,24 +272,38 @@ bool admit(Server* S) {
   bool progress = false;
   while (!S->pending.empty() && (int)S->active.size() < S->cfg.max_active) {
     Request* r = S->pending.front();
-    const Mesh& m = S->meshes[r->mesh_id]->m;
+    dtfe_mesh_t h = S->meshes[r->mesh_id];
+    const Mesh& m = h->m;
     const std::pair<int, int> key{r->mesh_id, r->p.axis};
-    const size_t need = r->map_bytes + missing_record_bytes(m, r->p.axis, r->p.precision);
-    if (!make_room(S, need, key)) {
+    const auto bare = [&] { return r->map_bytes + missing_record_bytes(m, r->p.axis, r->p.precision); };
+    const auto whole = [&] { return bare() + (m.link ? 0 : mesh_link_bytes(m)); };
+    bool links = true, room = make_room(S, whole, key);
+    if (!room) {
       bool idle = S->active.empty();
       for (const Slot& sl : S->slot) idle = idle && !sl.busy;
       if (!idle) break;  // wait for running requests to free memory
-      // alone on the device and still too large: it can never run
+      // alone on the device and still too large: FP64 without links, if that fits
+      if (r->p.precision == DTFE_FP64) {
+        links = false;
+        {
+          std::lock_guard<std::mutex> lk(h->mu);
+          if (!owner_has_records(S, r->mesh_id, m)) mesh_drop_links(&h->m);
+          count_links(S, r->mesh_id, m);
+        }
+        room = make_room(S, bare, key);
+      }
+    }
+    if (!room) {  // it can never run
       S->pending.pop_front();
       set_error(DTFE_ERR_ADMISSION, "request %llu needs %zu bytes; the budget is %zu",
-                (unsigned long long)r->id, need, S->cfg.device_budget);
+                (unsigned long long)r->id, links ? whole() : bare(), S->cfg.device_budget);
       fail_request(S, r, DTFE_ERR_ADMISSION);
       progress = true;
       continue;
     }
     S->pending.pop_front();
     S->active.push_back(r);
-    dtfe_status_t s = admit_one(S, r);
+    dtfe_status_t s = admit_one(S, r, links);
     if (s == DTFE_ERR_NOMEM) {
       // the device had less room than the budget assumed: return the pool's
       // cached map memory, drop every idle (mesh, axis) record set and try
@@ -270,9 +311,9 @@ bool admit(Server* S) {
       release(S, r);
       cudaStreamSynchronize(S->copy);
       cudaMemPoolTrimTo(S->pool, 0);
-      make_room(S, S->cfg.device_budget + 1, key);
+      make_room(S, [&] { return S->cfg.device_budget + 1; }, key);
       S->active.push_back(r);
-      s = admit_one(S, r);
+      s = admit_one(S, r, links);
     }
     if (s != DTFE_OK) {
       release(S, r);
@@ -693,8 +734,12 @@ dtfe_status_t dtfe_server_add_mesh(dtfe_server_t S, dtfe_mesh_t mesh, int* mesh_
     r.last_use = ++S->use_clock;
     S->in_use += b;
   }
+  {
+    std::lock_guard<std::mutex> mk(mesh->mu);
+    count_links(S, id, mesh->m);
+  }
   if (S->auto_budget) SDTFE_TRY(set_auto_budget(S));  // this mesh's records are in use, not free
-  make_room(S, 0, {-1, -1});  // evict down to the budget (records of idle pairs only)
+  make_room(S, [] { return size_t(0); }, {-1, -1});  // evict down to the budget (records of idle pairs only)
   note_use(S);
   *mesh_id = id;
   return DTFE_OK;

@@ -323,7 +323,7 @@ static void tile_shape(int S, int block, int* TW, int* TH) {
 static WalkConf64 walk_conf64(const Mesh& m, int axis, double lz, double dist, uint64_t seed,
                               int max_visits) {
   const AxisData& A = m.ax[axis];
-  return WalkConf64{lz, dist, seed, max_visits, A.rec64, m.rows, A.link, A.tri_face};
+  return WalkConf64{lz, dist, seed, max_visits, A.rec64, m.rows, m.link, A.tri_face};
 }
 
 // The kernel arguments of one FP64 map; *tiles_y receives its rows of tiles.

@@ -1412,7 +1412,7 @@ MixConf mix_conf(const Mesh& m, int axis, double z0, double lz, double dist, uin
   C.rec64 = m.ax[axis].rec64;
   C.exact32 = m.fp32_exact ? 1 : 0;
   C.geo = m.ax[axis].geo32;
-  C.link = m.ax[axis].link;
+  C.link = m.link;
   C.tri_face = m.ax[axis].tri_face;
   C.rows = m.rows;
   C.pos = m.pos;
