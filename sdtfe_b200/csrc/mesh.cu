@@ -342,22 +342,26 @@ dtfe_status_t exclusive_scan(const int* in, int* out, int n, cudaStream_t s) {
   return DTFE_OK;
 }
 
-// The meshes' memory pool of each device (vertices, rows, gradients,
-// adjacency, walk records, per-call scratch): stream-ordered allocation (no
-// device-wide synchronisation when a mesh is built or destroyed, or records
-// are built or dropped, while maps run), and freed memory kept for reuse up
-// to an eighth of the device (at most 16 GB) instead of being unmapped and
-// mapped again by every mesh.
+// The memory pools of each device: stream-ordered allocation (no device-wide
+// synchronisation when a mesh is built or destroyed, or records are built or
+// dropped, while maps run), and freed memory kept for reuse instead of being
+// unmapped and mapped again.  kMeshPool: the meshes' own arrays (vertices, rows,
+// gradients, adjacency, walk records), kept up to an eighth of the device, at most
+// 16 GB.  kScratchPool: what a call or a build takes for itself, kept up to
+// kScratchKept; more goes back to the system at the next synchronisation.
+// dtfe_trim_memory gives back both.
 constexpr int kMaxPoolDevices = 64;
+constexpr size_t kScratchKept = size_t(5) << 30;
+enum PoolKind : int { kMeshPool, kScratchPool, kPools };
 std::mutex g_pool_mu;
-cudaMemPool_t g_record_pool[kMaxPoolDevices] = {};
+cudaMemPool_t g_pool[kPools][kMaxPoolDevices] = {};
 
-dtfe_status_t record_pool(cudaMemPool_t* out) {
+dtfe_status_t device_pool(PoolKind kind, cudaMemPool_t* out) {
   int dev = 0;
   SDTFE_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kMaxPoolDevices) return set_error(DTFE_ERR_UNSUPPORTED, "device %d", dev);
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  if (!g_record_pool[dev]) {
+  if (!g_pool[kind][dev]) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -366,27 +370,38 @@ dtfe_status_t record_pool(cudaMemPool_t* out) {
     SDTFE_CUDA(cudaMemPoolCreate(&pool, &props));
     size_t fr = 0, total = 0;
     SDTFE_CUDA(cudaMemGetInfo(&fr, &total));
-    uint64_t keep = std::min<uint64_t>(uint64_t(16) << 30, total / 8);
+    uint64_t keep = std::min<uint64_t>(kind == kMeshPool ? uint64_t(16) << 30 : kScratchKept, total / 8);
     SDTFE_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    g_record_pool[dev] = pool;
+    g_pool[kind][dev] = pool;
   }
-  *out = g_record_pool[dev];
+  *out = g_pool[kind][dev];
+  return DTFE_OK;
+}
+
+// What one pool keeps free may be what the other needs.
+dtfe_status_t pool_alloc(PoolKind kind, void** p, size_t bytes, cudaStream_t s) {
+  *p = nullptr;
+  cudaMemPool_t pool = nullptr;
+  SDTFE_TRY(device_pool(kind, &pool));
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    cudaMemPool_t other = nullptr;
+    SDTFE_TRY(device_pool(kind == kMeshPool ? kScratchPool : kMeshPool, &other));
+    cudaMemPoolTrimTo(other, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  }
+  SDTFE_CUDA(e);
   return DTFE_OK;
 }
 
 }  // namespace
 
-// Per-call device scratch, stream-ordered from the record pool (whose freed
-// memory is kept for reuse, so a map's or a build's scratch costs no mapping).
-// From the default pool, which unmaps what is free at every synchronisation, a
-// 64^2 map into a host array waited 430 of its 600 us for its 32 KB to be mapped;
-// compute_density of 131k points took 7.2 ms instead of 5.7.
+// Per-call device scratch.  From the default pool, which unmaps what is free at
+// every synchronisation, a 64^2 map into a host array waited for its 32 KB to be
+// mapped.
 dtfe_status_t scratch_alloc_async(void** p, size_t bytes, cudaStream_t s) {
-  *p = nullptr;
-  cudaMemPool_t pool = nullptr;
-  SDTFE_TRY(record_pool(&pool));
-  SDTFE_CUDA(cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s));
-  return DTFE_OK;
+  return pool_alloc(kScratchPool, p, bytes ? bytes : 1, s);
 }
 
 void scratch_free_async(void* p, cudaStream_t s) {
@@ -397,19 +412,18 @@ void mesh_trim_record_pool() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxPoolDevices) return;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  if (g_record_pool[dev]) cudaMemPoolTrimTo(g_record_pool[dev], 0);
+  for (auto& pools : g_pool)
+    if (pools[dev]) cudaMemPoolTrimTo(pools[dev], 0);
 }
 
 namespace {
 
-// stream-ordered allocation from the record pool, on the mesh stream
+// stream-ordered allocation from the meshes' pool, on the mesh stream
 template <class T>
 dtfe_status_t dmalloc_async(T** p, size_t count, Mesh* m) {
   *p = nullptr;
   if (count == 0) count = 1;
-  cudaMemPool_t pool = nullptr;
-  SDTFE_TRY(record_pool(&pool));
-  SDTFE_CUDA(cudaMallocFromPoolAsync((void**)p, count * sizeof(T), pool, m->stream));
+  SDTFE_TRY(pool_alloc(kMeshPool, reinterpret_cast<void**>(p), count * sizeof(T), m->stream));
   m->bytes += count * sizeof(T);
   return DTFE_OK;
 }

@@ -94,3 +94,26 @@ def test_trim_returns_the_pools_memory(sd, mesh_input):
     with sd.Mesh(pos4, tetra, 1.0) as m:  # the pool refills on the next mesh
         got, st = m.map(sd.map_params(64, 1.0, 1.0, (0.5, 0.5, 0.5), 2, 0.0, 5))
         assert st.rays == 64 * 64 * 2 and got.sum() > 0
+
+
+def test_scratch_kept_is_bounded_and_given_back(sd, mesh_input):
+    """An 8 GB device copy of a host grid goes back to the device at the next synchronisation but
+    for what may be kept; dtfe_trim_memory gives that back too."""
+    import torch
+
+    pos4, tetra = mesh_input
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    with sd.Mesh(pos4, tetra, 1.0) as m:
+        m.grid(32, 1.0, (0.5, 0.5, 0.5), 2, 4)
+        sd.trim_memory()
+        before = free()
+        m.grid(1000, 3000.0, (0.5, 0.5, 0.5), 1, 4)
+        assert before - free() <= 5 * 2**30 + 2**28
+        m.grid(256, 3.0, (0.5, 0.5, 0.5), 2, 4)
+        assert 2**30 <= before - free() <= 5 * 2**30 + 2**28  # the node values, 1 GiB, are kept
+        sd.trim_memory()
+        assert before - free() <= 2**26
