@@ -60,6 +60,9 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
+# profiles/roofline.json's entry for the present build of each walk kernel (its
+# "k_map32" is the walk that read all four vertices of a tet)
+PROFILE_OF = {"k_map32": "k_map32_apex"}
 BYTES_PER_VISIT = {"mixed": 48, "fp64": 112}  # bytes a walk step reads: one vertex, its links and the tet's field
 
 
@@ -1000,8 +1003,7 @@ def run_ours(args, pre=None):
     hbm_note = "measured" if hbm else "fallback"
     hbm = hbm or 6650.0
     kname = "k_map32" if args.precision == "mixed" else "k_map64"
-    # (the profile's key "k_map32" is the walk that read all four vertices of a tet)
-    roof = roofline({"k_map32": "k_map32_apex"}.get(kname, kname), visits, len(tetra), bpv, kern_ms, clk.get("sm_mhz") or 1965.0,
+    roof = roofline(PROFILE_OF.get(kname, kname), visits, len(tetra), bpv, kern_ms, clk.get("sm_mhz") or 1965.0,
                     torch.cuda.get_device_properties(dev).multi_processor_count, hbm, hbm_note)
     roof["kernel"] = kname
 

@@ -51,3 +51,17 @@ def test_roofline_scales_with_the_timed_launch():
     assert abs(a["frac"] - b["frac"]) < 1e-12          # twice the visits in twice the time
     assert abs(a["traffic"] - 4 * b["traffic"]) < 1e-3  # DRAM bytes per tet
     assert abs(a["peak"] - 148 * 4 * 1.965) < 1e-9     # G warp instructions/s
+
+
+def test_roofline_of_the_kernel_the_bench_times():
+    """The entry, and the bytes a visit, that the bench itself reports the mixed walk from."""
+    bench = _bench()
+    key, bpv = bench.PROFILE_OF["k_map32"], bench.BYTES_PER_VISIT["mixed"]
+    prof = json.load(open(os.path.join(ROOT, "profiles", "roofline.json")))[key]
+    assert 100 < prof["visits"] / prof["rays"] < 1000
+    assert 3.0 < prof["warp_inst"] / prof["visits"] < 5.0
+    assert bpv == 32 + 16  # the record and its links
+    r = bench.roofline(key, prof["visits"], prof["tets"], bpv, prof["duration_ms_under_ncu"], 1960.0, 148, 6545.6,
+                       "measured")
+    assert r["bound"] == "issue" and abs(r["frac"] - prof["issue_active_pct"] / 100.0) < 0.02
+    assert r["traffic"] == prof["dram_bytes"]
