@@ -133,7 +133,7 @@ __device__ __forceinline__ void map_tile64(const MapArgs64& a, int tile, double*
 }
 
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, map_min_blocks64(BLOCK)) k_map64(const MapArgs64 a) {
+__global__ void __launch_bounds__(BLOCK, map_min_blocks64(BLOCK)) k_map64(const __grid_constant__ MapArgs64 a) {
   extern __shared__ double s_val[];  // P*S doubles, then P*S bytes of success flags
   unsigned char* s_ok = reinterpret_cast<unsigned char*>(s_val + a.TW * a.TH * a.S);
   map_tile64(a, blockIdx.x, s_val, s_ok);
