@@ -85,11 +85,11 @@ __device__ __forceinline__ bool ray_of_grid(const GridRays& a, int* i, int* j, i
   *js = fj % a.ss;
   return lane < a.lanes && fi < nf && fj < nf;
 }
-inline long long ray_warps(const GridRays& a) {
-  const long long nf = (long long)a.G * a.ss;
-  const int pi = patch_rows(a.lanes), pj = patch_cols(a.lanes);
+inline long long ray_warps(long long nf, int lanes) {
+  const int pi = patch_rows(lanes), pj = patch_cols(lanes);
   return ((nf + pi - 1) / pi) * ((nf + pj - 1) / pj);
 }
+inline long long ray_warps(const GridRays& a) { return ray_warps((long long)a.G * a.ss, a.lanes); }
 
 __device__ __forceinline__ size_t ray_index(const GridRays& a, int i, int j, int is, int js) {
   return (((size_t)i * a.G + j) * a.ss + is) * a.ss + js;
@@ -147,14 +147,13 @@ __global__ void __launch_bounds__(256) k_grid_sum(const GridRays a, double* __re
   grid[cell] = sum;
 }
 
-// Which grids are walked by sub-rays: all with several a column, as long as the
-// rows of nodes (8 B times the fine grid) stay within 4 GiB - up to 406^3 cells
-// at ss = 2, 268^3 at 3, 203^3 at 4.  One thread a column is slower below and,
-// measured, still at that size (83k-point lattice, mixed / FP64, one thread a
-// column -> sub-rays): 128^3 ss 4 15.1 / 11.3 -> 3.2 / 2.4 ms, 200^3 ss 2 3.8 /
-// 2.8 -> 2.8 / 1.6, 256^3 ss 3 12.8 / 9.6 -> 6.7 / 5.3, 384^3 ss 2 8.8 / 7.0 ->
-// 6.8 / 5.6.  Batches of the rows lose that again to one tail each (384^3 in 1
-// GiB batches: 12.8 / 6.7).
+// Which grids are walked by sub-rays: all with several a column (but for dense FP64
+// grids, walk.cu), as long as the rows of nodes (8 B times the fine grid) stay within
+// 4 GiB - up to 406^3 cells at ss = 2, 268^3 at 3, 203^3 at 4.  One thread a column is
+// slower below and, measured, still at that size (83k-point lattice, mixed / FP64, one
+// thread a column -> sub-rays): 128^3 ss 4 6.9 / 10.9 -> 1.9 / 2.0 ms, 200^3 ss 2 3.0 /
+// 2.8 -> 1.3 / 1.4, 256^3 ss 3 9.2 / 7.7 -> 4.4 / 4.3, 384^3 ss 2 6.6 / 6.0 -> 4.5 / 4.4.
+// Batches of the rows lose that again to one tail each.
 constexpr size_t kNodeBytes = size_t(4) << 30;
 inline bool grid_takes_rays(int G, unsigned ss) {
   const double n = (double)G * ss;

@@ -840,7 +840,7 @@ __device__ __forceinline__ float rcp32(float x) {
 // All that can go wrong is gathered in one condition (clear), so that the
 // common step has one branch.
 //
-// What bounds it: instruction issue (73 % of the cycles of 32 warps per SM;
+// What bounds it: instruction issue (77 % of the cycles of 32 warps per SM;
 // 104 thread instructions a visit, 56 of them on the FMA and ALU pipes' FP32)
 // together with the L1's load return (30 wavefronts a warp's visit, 60 % of
 // its cycles: 48 B a lane, lanes of one warp in six to eight tets).  Records
@@ -1351,8 +1351,9 @@ __device__ __forceinline__ int grid_ray32(const GridArgs32& a, int i, int j, int
 // registers: on a mesh far larger than L2 (61.8M tets, 512^3) 9.7 ms, five
 // blocks 10.2, six 10.9, seven 12.4; on one within it (83k points) 1.85, 1.86, 1.87
 // and 2.01, and 256^3 0.567, 0.556, 0.557, 0.559.
+constexpr int kColumnBlocks = 4, kRayBlocks = 10;
 template <bool Marked>
-__global__ void __launch_bounds__(128, 4)
+__global__ void __launch_bounds__(128, kColumnBlocks)
     k_grid32(const __grid_constant__ GridArgs32 a, const GridRays r) {
   int i, j;
   bool active = grid_column(a.G, a.lanes, &i, &j);
@@ -1379,7 +1380,7 @@ __global__ void __launch_bounds__(128, 4)
 }
 
 // One thread per sub-ray, node values to the ray's row (grid_rays.cuh).
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(64, kRayBlocks)
     k_grid_rays32(const __grid_constant__ GridArgs32 a, const GridRays r) {
   int i, j, is, js, c = 0, fb = 0;
   if (ray_of_grid(r, &i, &j, &is, &js)) {
@@ -1588,13 +1589,16 @@ dtfe_status_t launch_map32(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
 // Columns or sub-rays a warp of the mixed grid walks.  A launch that leaves the
 // SMs few warps waits for each warp's longest walk, its most nodes and its
 // general steps, one lane at a time; fewer lanes a warp shorten all three while
-// all warps are still resident (16 a SM; the sub-ray kernel holds more).  Full ->
-// 16 -> 8 lanes, ms: 64^3 0.222, 0.170, 0.146; 128^3 0.337, 0.277, 0.253; 160^3
-// 0.326, 0.281, 0.377; 180^3 0.547, 0.437, 0.603; 256^3 0.703, 0.813; sub-rays at ss
-// 2 or 3: 30^3 0.323, 0.276, 0.233; 49^3 0.475, 0.398, 0.327; 82^3 0.731, 0.637,
-// 0.574; 85^3 0.426, 0.412, 0.434; 100^3 1.10, 0.82, 0.91.
-static int grid_lanes32(long long n, bool sub_rays) {
-  return n <= 148 * (sub_rays ? 182 : 128) ? 8 : (n <= 148 * 288 ? 16 : 32);
+// all warps are still resident: 16 an SM of k_grid32 and 20 of k_grid_rays32.  8,
+// 16 and 32 lanes, ms, 83k-point lattice / 20k clustered points: 128^3 0.29, 0.34,
+// 0.40 / 0.19, 0.20, 0.22; 137^3, past 8 lanes, 0.38, 0.33, 0.40 / 0.20, 0.21, 0.24;
+// 180^3 0.54, 0.37, 0.42 / 0.35, 0.28, 0.29; 206^3, past 16, 0.74, 0.60, 0.43 / 0.45,
+// 0.40, 0.33; sub-rays at 49^3, ss 3, 0.54, 0.60, 0.65 / 0.31, 0.32, 0.35; 82^3, ss 2,
+// past 8, 0.68, 0.61, 0.68 / 0.40, 0.36, 0.37; 103^3 0.86, 0.61, 0.68 / 0.52, 0.39,
+// 0.45; 110^3, past 16, 0.90, 0.75, 0.71 / 0.56, 0.45, 0.49.
+template <class Warps>
+static int grid_lanes32(long long resident, const Warps& warps) {
+  return warps(8) <= resident ? 8 : (warps(16) <= resident ? 16 : 32);
 }
 
 dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[3], unsigned ss,
@@ -1611,7 +1615,10 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
   a.n_tri = A.n_tri;
   a.G = G;
   a.ss = (int)ss;
-  a.lanes = grid_lanes32((long long)G * G, false);
+  int dev = 0, sms = 0;
+  SDTFE_CUDA(cudaGetDevice(&dev));
+  SDTFE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  a.lanes = grid_lanes32(sms * kColumnBlocks * 4, [&](int lanes) { return (long long)grid_warps(G, lanes); });
   a.loc_budget = 4 * A.n_tri + 64;
   // src/dtfe.c:668-735 and :398-404: cell and node spacing, weight 1/ss^3
   a.dxy = box_len / G;
@@ -1631,7 +1638,8 @@ dtfe_status_t launch_grid32(Mesh& m, int G, double box_len, const double center[
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
   bool taken = false;
   SDTFE_TRY(grid_by_rays(
-      G, ss, grid_lanes32((long long)G * ss * G * ss, true), d_grid, s, &taken,
+      G, ss, grid_lanes32(sms * kRayBlocks * 2, [&](int lanes) { return ray_warps((long long)G * ss, lanes); }),
+      d_grid, s, &taken,
       [&](const GridRays& r) {
         k_grid_rays32<<<(unsigned)((ray_warps(r) + 1) / 2), 64, 0, s>>>(a, r);
       },

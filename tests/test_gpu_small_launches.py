@@ -54,3 +54,14 @@ def test_grids(golden, sd, oracle, mesh, G, ss):
     assert np.array_equal(got, want)
     mixed = mesh.grid(G, 1.0, (0.5, 0.5, 0.5), ss, 3, precision=sd.DTFE_MIXED)
     assert np.all(np.abs(mixed - got) <= 1e-5 * np.abs(got))
+
+
+# the last sides whose warps of 8 and of 16 lanes are all resident (grid_lanes32), and the next
+@pytest.mark.parametrize("G,ss", [(136, 1), (137, 1), (192, 1), (193, 1), (76, 2), (77, 2), (108, 2), (109, 2)])
+def test_mixed_grids_at_the_resident_lines(sd, mesh, G, ss):
+    want = mesh.grid(G, 1.0, (0.5, 0.5, 0.5), ss, 3)
+    st64 = mesh.last_stats()
+    got = mesh.grid(G, 1.0, (0.5, 0.5, 0.5), ss, 3, precision=sd.DTFE_MIXED)
+    st32 = mesh.last_stats()
+    assert np.all(np.abs(got - want) <= 1e-5 * np.abs(want))
+    assert (st64.rays, st64.visits, list(st64.status)) == (st32.rays, st32.visits, list(st32.status))
