@@ -68,3 +68,27 @@ def test_visit_budget(golden, sd, budget):
     s = golden_set(golden, "clustered")
     status = same_walks(sd, s["pos4"], s["tetra"], s["trace_x"], s["trace_y"], budget)
     assert (status == sd.RAY_BUDGET).any()
+
+
+@pytest.mark.parametrize("what", ["flipped", "flipped half", "swapped links"])
+def test_unusable_links_against_the_oracle(golden, sd, oracle, what):
+    """The FP64 walk, which reads the same links as the mixed one: every ray ends as the oracle's, which
+    reads none, to the bit."""
+    s = golden_set(golden, "clustered")
+    tetra = s["tetra"].copy()
+    rng = np.random.default_rng(3)
+    pick = rng.random(len(tetra)) < (0.5 if what == "flipped half" else 0.03)
+    if what == "swapped links":
+        tetra[pick, 4], tetra[pick, 5] = s["tetra"][pick, 5], s["tetra"][pick, 4]
+    else:
+        for a, b in ((1, 2), (5, 6)):
+            tetra[pick, a], tetra[pick, b] = s["tetra"][pick, b], s["tetra"][pick, a]
+    xy = rng.random((3000, 2))
+    xs, ys = np.concatenate([s["trace_x"], xy[:, 0]]), np.concatenate([s["trace_y"], xy[:, 1]])
+    want = oracle.trace(oracle.prepare(s["pos4"], tetra, 1.0), xs, ys, 0.0, 1.0, 1 / 24, 5, 4000, 4000)
+    with sd.Mesh(s["pos4"], tetra, 1.0) as m:
+        p = sd.map_params(24, 1.0, 1.0, (0.5, 0.5, 0.5), 4, 0.0, 5, max_visits=4000)
+        got = m.trace(p, xs, ys, 0.0, 1.0, 1 / 24, 4000)
+    ok = want[2] == sd.RAY_OK
+    assert np.array_equal(got[2], want[2]) and np.array_equal(got[1], want[1]) and np.array_equal(got[0], want[0])
+    assert np.array_equal(got[3][ok], want[3][ok])
