@@ -1481,6 +1481,11 @@ constexpr int kDefaultVariant32 = 7;  // (128, 8): the usual winner on B200
 // left to hide spills (32,768 rays 130 us, with 64 registers 134; 128 registers
 // are no faster).
 const MapKernel32 kSparseMap32 = k_map32<128, 6, true>;
+// ... and, with full warps, its maps whose blocks are all resident at six an SM (64^2 x
+// 16 and 128^2 x 4 over 32k uniform points 0.437 -> 0.408 and 0.498 -> 0.461 ms, 150^2 x
+// 4 0.539 -> 0.494; over 131k clustered ones 2 %; past them, 180^2 x 4, 0.486 against 0.570).
+constexpr int kResidentBlocks32 = 6;
+const MapKernel32 kResidentMap32 = k_map32<128, kResidentBlocks32>;
 
 typedef void (*BatchKernel32)(const BatchTable32, unsigned long long*, const int2*);
 const BatchKernel32 kBatch32[] = {k_batch32<256, 2>, k_batch32<256, 3>, k_batch32<256, 4>,
@@ -1560,15 +1565,22 @@ dtfe_status_t launch_map32(Mesh& m, const MapGeom& g, double* d_map, cudaStream_
                            double* ray_rho, int* ray_crossed, int* ray_status) {
   const int vi = pick_variant32(m.tune32);
   const Variant32& V = kVariants32[vi];
-  const int lanes = vi == kDefaultVariant32 && !m.full_warps ? map_lanes32(g, V.block) : 32;
-  const MapKernel32 kernel = lanes < 32 ? kSparseMap32 : V.kernel;
+  const bool small = vi == kDefaultVariant32 && !m.full_warps;  // (may be)
+  const int lanes = small ? map_lanes32(g, V.block) : 32;
   MapArgs32 a;
   int tiles_y = 0;
   SDTFE_TRY(map_args32(m, g, vi, lanes, d_map, m.stats, ray_rho, ray_crossed, ray_status, &a, &tiles_y));
   const size_t smem = (size_t)a.TW * a.TH * g.S * (sizeof(double) + 1);
+  const long long blocks = (long long)a.tiles_x * tiles_y;
+  MapKernel32 kernel = lanes < 32 ? kSparseMap32 : V.kernel;
+  if (small && lanes == 32) {
+    int dev = 0, sms = 0;
+    SDTFE_CUDA(cudaGetDevice(&dev));
+    SDTFE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (blocks <= (long long)kResidentBlocks32 * sms) kernel = kResidentMap32;
+  }
   if (smem > 40 * 1024)
     SDTFE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const long long blocks = (long long)a.tiles_x * tiles_y;
   SDTFE_CUDA(cudaMemsetAsync(m.stats, 0, sizeof(unsigned long long) * kStatCount, s));
   SDTFE_CUDA(cudaEventRecord(m.ev0, s));
   void* loc = nullptr;  // each tile's shared point location

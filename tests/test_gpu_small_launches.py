@@ -65,3 +65,9 @@ def test_mixed_grids_at_the_resident_lines(sd, mesh, G, ss):
     st32 = mesh.last_stats()
     assert np.all(np.abs(got - want) <= 1e-5 * np.abs(want))
     assert (st64.rays, st64.visits, list(st64.status)) == (st32.rays, st32.visits, list(st32.status))
+
+
+# maps on either side of the blocks that are all resident at six an SM (kResidentMap32), and large samples
+@pytest.mark.parametrize("side,samples", [(182, 1), (320, 1), (337, 1), (150, 4), (180, 4), (6, 2000), (30, 128), (31, 128)])
+def test_resident_maps_equal_full_warps(sd, mesh, side, samples):
+    test_maps_equal_full_warps(sd, mesh, side, samples)
