@@ -12,8 +12,9 @@ namespace sdtfe {
 
 // a3 part 1: per-tet volume |V| in the reference's operation order
 // (src/triangulate.c:191-215), and the tets of each vertex counted.  Checked:
-// a tet with a vertex id outside [0, n) sets *err and is passed over, here and
-// by k_tet_fill.
+// a tet with a vertex id outside [0, n) sets *flags' kOutOfRange and is passed
+// over, here and by k_tet_fill.  One that lists a vertex twice sets kRepeated.
+constexpr int kOutOfRange = 1, kRepeated = 2;
 __device__ __forceinline__ bool vertices_in(const int4& v, int n) {
   return (unsigned)v.x < (unsigned)n && (unsigned)v.y < (unsigned)n && (unsigned)v.z < (unsigned)n &&
          (unsigned)v.w < (unsigned)n;
@@ -22,14 +23,16 @@ __device__ __forceinline__ bool vertices_in(const int4& v, int n) {
 template <bool Checked>
 __global__ void k_volume_count(const double4* __restrict__ pos, const int4* __restrict__ rows,
                                int nt, int n, double* __restrict__ vol, int* __restrict__ cnt,
-                               int* __restrict__ err) {
+                               int* __restrict__ flags) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   const int4 v = rows[2 * (size_t)t];
   if (Checked && !vertices_in(v, n)) {
-    atomicOr(err, 1);
+    atomicOr(flags, kOutOfRange);
     return;
   }
+  if (v.x == v.y || v.x == v.z || v.x == v.w || v.y == v.z || v.y == v.w || v.z == v.w)
+    atomicOr(flags, kRepeated);
   const double4 a = pos[v.x], b = pos[v.y], c = pos[v.z], d = pos[v.w];
   const double r0 = (a.x - d.x) * ((b.y - d.y) * (c.z - d.z) - (b.z - d.z) * (c.y - d.y));
   const double r1 = (a.y - d.y) * ((b.z - d.z) * (c.x - d.x) - (b.x - d.x) * (c.z - d.z));
@@ -92,12 +95,12 @@ __device__ inline void shell_sort(int* a, int d) {
 }
 
 // The places of K tets a lane, at list positions lane, lane + 32, ...  A tet that
-// lists the vertex several times is in the list as often: equal ids take their
-// places in list order, so that every place is taken.
+// lists the vertex several times is in the list as often: where there are such tets
+// (repeated), equal ids take their places in list order, so that every place is taken.
 template <int K>
 __device__ __forceinline__ void rank_volumes(const int* __restrict__ list, int d,
                                              const double* __restrict__ vol, int lane,
-                                             double* row) {
+                                             bool repeated, double* row) {
   unsigned id[K];
   int rank[K];
   double v[K];
@@ -107,17 +110,19 @@ __device__ __forceinline__ void rank_volumes(const int* __restrict__ list, int d
     id[k] = i < d ? (unsigned)list[i] : 0u;  // (no place is taken from d on)
     v[k] = i < d ? vol[id[k]] : 0.0;
     rank[k] = 0;
+    if (repeated) {
+      const unsigned same = __match_any_sync(0xffffffffu, i < d ? id[k] : 0xffffffffu);
+      rank[k] = __popc(same & ((1u << lane) - 1u));
+    }
   }
+  const unsigned tie = repeated ? 1u : 0u;  // an equal id of an earlier 32 comes first
 #pragma unroll
   for (int c = 0; c < K; ++c) {
     const int m = min(32, d - 32 * c);
     for (int j = 0; j < m; ++j) {
       const unsigned other = __shfl_sync(0xffffffffu, id[c], j);
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const bool earlier = c < k || (c == k && j < lane);  // in the list
-        rank[k] += other < id[k] + (unsigned)earlier;
-      }
+      for (int k = 0; k < K; ++k) rank[k] += other < (c < k ? id[k] + tie : id[k]);
     }
   }
 #pragma unroll
@@ -129,13 +134,13 @@ __device__ __forceinline__ void rank_volumes(const int* __restrict__ list, int d
 // reference's in-place scatter-add, to the bit); valid in lane 0.  The whole
 // warp calls it; row: kRankedTets doubles of shared memory, the warp's own.
 __device__ inline double volume_sum(int* __restrict__ list, int d, const double* __restrict__ vol,
-                                    double* row) {
+                                    bool repeated, double* row) {
   const int lane = (int)(threadIdx.x & 31u);
   double s = 0;
   if (d <= kRankedTets) {
-    if (d <= 32) rank_volumes<1>(list, d, vol, lane, row);
-    else if (d <= 64) rank_volumes<2>(list, d, vol, lane, row);
-    else rank_volumes<4>(list, d, vol, lane, row);
+    if (d <= 32) rank_volumes<1>(list, d, vol, lane, repeated, row);
+    else if (d <= 64) rank_volumes<2>(list, d, vol, lane, repeated, row);
+    else rank_volumes<4>(list, d, vol, lane, repeated, row);
     __syncwarp();
     if (lane == 0)
       for (int i = 0; i < d; ++i) s += row[i];

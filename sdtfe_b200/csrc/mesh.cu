@@ -59,12 +59,13 @@ __global__ void k_fp32_exact(const double4* __restrict__ pos, int n, int* __rest
 // (density.cuh).
 __global__ void __launch_bounds__(32 * kDensityWarps)
     k_density(const int* __restrict__ off, int* __restrict__ idx, const double* __restrict__ vol,
-              int n, double m4, double4* __restrict__ pos, int* __restrict__ adj) {
+              int n, double m4, const int* __restrict__ flags, double4* __restrict__ pos,
+              int* __restrict__ adj) {
   __shared__ double row[kDensityWarps][kRankedTets];
   const int w = (int)(threadIdx.x >> 5), v = blockIdx.x * kDensityWarps + w;
   if (v >= n) return;
   const int b = off[v], d = off[v + 1] - b;
-  const double s = volume_sum(idx + b, d, vol, row[w]);
+  const double s = volume_sum(idx + b, d, vol, (*flags & kRepeated) != 0, row[w]);
   if ((threadIdx.x & 31) == 0) {
     pos[v].w = m4 / s;
     adj[v] = d;
@@ -492,12 +493,13 @@ dtfe_status_t mesh_density(Mesh* m) {
   double* vol = nullptr;
   int *cnt = nullptr, *off = nullptr, *idx = nullptr;
   SDTFE_TRY(scratch_alloc_async(&vol, sizeof(double) * (nt ? nt : 1), s));
-  SDTFE_TRY(scratch_alloc_async(&cnt, sizeof(int) * (n + 1), s));
+  SDTFE_TRY(scratch_alloc_async(&cnt, sizeof(int) * ((size_t)n + 2), s));
   SDTFE_TRY(scratch_alloc_async(&off, sizeof(int) * (n + 1), s));
   SDTFE_TRY(scratch_alloc_async(&idx, sizeof(int) * (4 * (size_t)nt + 1), s));
-  SDTFE_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (n + 1), s));
+  int* const flags = cnt + n + 1;  // behind the n + 1 counts
+  SDTFE_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * ((size_t)n + 2), s));
   if (nt) {
-    k_volume_count<false><<<grid_for(nt), kBlock, 0, s>>>(m->pos, m->rows, nt, n, vol, cnt, nullptr);
+    k_volume_count<false><<<grid_for(nt), kBlock, 0, s>>>(m->pos, m->rows, nt, n, vol, cnt, flags);
     count_launch();
   }
   SDTFE_TRY(exclusive_scan(cnt, off, n, s));
@@ -508,7 +510,7 @@ dtfe_status_t mesh_density(Mesh* m) {
   if (n) {
     // p_mass*(1+DIM) is a float product in the reference (float * int)
     const double m4 = (double)(m->p_mass * 4);
-    k_density<<<grid_for(n, kDensityWarps), 32 * kDensityWarps, 0, s>>>(off, idx, vol, n, m4, m->pos, m->adj);
+    k_density<<<grid_for(n, kDensityWarps), 32 * kDensityWarps, 0, s>>>(off, idx, vol, n, m4, flags, m->pos, m->adj);
     count_launch();
   }
   cudaFreeAsync(vol, s);

@@ -56,12 +56,12 @@ inline unsigned blocks_for(long long n) { return (unsigned)((n + kBlk - 1) / kBl
 // Nothing is written when a tet was out of range.
 __global__ void __launch_bounds__(32 * kDensityWarps)
     k_na_density(const int* __restrict__ off, int* __restrict__ idx, const double* __restrict__ vol,
-                 int n, double m4, const int* __restrict__ err, double* __restrict__ rho) {
+                 int n, double m4, const int* __restrict__ flags, double* __restrict__ rho) {
   __shared__ double row[kDensityWarps][kRankedTets];
   const int w = (int)(threadIdx.x >> 5), v = blockIdx.x * kDensityWarps + w;
-  if (v >= n || *err) return;
+  if (v >= n || (*flags & kOutOfRange)) return;
   const int b = off[v];
-  const double s = volume_sum(idx + b, off[v + 1] - b, vol, row[w]);
+  const double s = volume_sum(idx + b, off[v + 1] - b, vol, (*flags & kRepeated) != 0, row[w]);
   if ((threadIdx.x & 31) == 0) rho[v] = m4 / s;
 }
 
@@ -95,7 +95,7 @@ extern "C" dtfe_status_t dtfe_density_noalloc(const double* d_particle_data, int
     return set_error(DTFE_ERR_INVALID, "NULL device pointer");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int n = n_particles, nt = n_tetra;
-  // carve the scratch: error flag | cnt (n+1) | off (n+1) | vol | idx (4 nt) | scan temp;
+  // carve the scratch: flags | cnt (n+1) | off (n+1) | vol | idx (4 nt) | scan temp;
   // the fixed part is checked first, in size_t, so that n + 1 below is an int
   const size_t o_cnt = 256;
   const size_t o_off = align256(o_cnt + sizeof(int) * ((size_t)n + 1));
@@ -117,7 +117,7 @@ extern "C" dtfe_status_t dtfe_density_noalloc(const double* d_particle_data, int
                      "the static scratch holds %zu (about 1.9M tets)",
                      n, nt, need, kNoAllocScratchBytes);
   SDTFE_TRY(scratch_base(&base));
-  int* err = reinterpret_cast<int*>(base);
+  int* flags = reinterpret_cast<int*>(base);
   double* vol = reinterpret_cast<double*>(base + o_vol);
   int* cnt = reinterpret_cast<int*>(base + o_cnt);
   int* off = reinterpret_cast<int*>(base + o_off);
@@ -127,9 +127,9 @@ extern "C" dtfe_status_t dtfe_density_noalloc(const double* d_particle_data, int
   const int4* rows = reinterpret_cast<const int4*>(d_tetra_data);
 
   // the array keeps the previous call's contents: clear what starts at zero
-  SDTFE_CUDA(cudaMemsetAsync(err, 0, o_cnt + sizeof(int) * ((size_t)n + 1), s));
+  SDTFE_CUDA(cudaMemsetAsync(flags, 0, o_cnt + sizeof(int) * ((size_t)n + 1), s));
   if (nt) {
-    k_volume_count<true><<<blocks_for(nt), kBlk, 0, s>>>(pos, rows, nt, n, vol, cnt, err);
+    k_volume_count<true><<<blocks_for(nt), kBlk, 0, s>>>(pos, rows, nt, n, vol, cnt, flags);
     count_launch();
   }
   SDTFE_CUDA(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, cnt, off, n + 1, s));
@@ -139,13 +139,13 @@ extern "C" dtfe_status_t dtfe_density_noalloc(const double* d_particle_data, int
   }
   const double m4 = (double)(p_mass * 4);  // float product, as in the reference
   k_na_density<<<(unsigned)(((long long)n + kDensityWarps - 1) / kDensityWarps), 32 * kDensityWarps, 0, s>>>(
-      off, idx, vol, n, m4, err, d_rho);
+      off, idx, vol, n, m4, flags, d_rho);
   count_launch();
   SDTFE_CUDA(cudaGetLastError());
-  int h_err = 0;
-  SDTFE_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
+  int h_flags = 0;
+  SDTFE_CUDA(cudaMemcpyAsync(&h_flags, flags, sizeof(int), cudaMemcpyDeviceToHost, s));
   SDTFE_CUDA(cudaStreamSynchronize(s));
-  if (h_err)
+  if (h_flags & kOutOfRange)
     return set_error(DTFE_ERR_MESH, "tetra_data holds a vertex id outside [0, %d)", n);
   return DTFE_OK;
 }
