@@ -347,12 +347,12 @@ dtfe_status_t exclusive_scan(const int* in, int* out, int n, cudaStream_t s) {
 // synchronisation when a mesh is built or destroyed, or records are built or
 // dropped, while maps run), and freed memory kept for reuse instead of being
 // unmapped and mapped again.  kMeshPool: the meshes' own arrays (vertices, rows,
-// gradients, adjacency, walk records), kept up to an eighth of the device, at most
-// 16 GB.  kScratchPool: what a call or a build takes for itself, kept up to
-// kScratchKept; more goes back to the system at the next synchronisation.
-// dtfe_trim_memory gives back both.
+// gradients, adjacency, walk records) and small scratch, kept up to an eighth of
+// the device, at most 16 GB.  kScratchPool: what a call or a build takes for itself
+// from kLargeScratch on, kept up to kScratchKept; more goes back to the system at
+// the next synchronisation.  dtfe_trim_memory gives back both.
 constexpr int kMaxPoolDevices = 64;
-constexpr size_t kScratchKept = size_t(5) << 30;
+constexpr size_t kScratchKept = size_t(5) << 30, kLargeScratch = size_t(32) << 20;
 enum PoolKind : int { kMeshPool, kScratchPool, kPools };
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[kPools][kMaxPoolDevices] = {};
@@ -400,9 +400,11 @@ dtfe_status_t pool_alloc(PoolKind kind, void** p, size_t bytes, cudaStream_t s) 
 
 // Per-call device scratch.  From the default pool, which unmaps what is free at
 // every synchronisation, a 64^2 map into a host array waited for its 32 KB to be
-// mapped.
+// mapped.  Small pieces come from the pool where a mesh's stream has memory of its
+// own: taken from one that all streams share, they cost a map of a few thousand
+// rays 5 to 11 us when several meshes take turns.
 dtfe_status_t scratch_alloc_async(void** p, size_t bytes, cudaStream_t s) {
-  return pool_alloc(kScratchPool, p, bytes ? bytes : 1, s);
+  return pool_alloc(bytes < kLargeScratch ? kMeshPool : kScratchPool, p, bytes ? bytes : 1, s);
 }
 
 void scratch_free_async(void* p, cudaStream_t s) {
