@@ -130,10 +130,11 @@ dtfe_status_t dtfe_mesh_create(const double *particle_data, int n_particles,
 dtfe_status_t dtfe_mesh_destroy(dtfe_mesh_t mesh);
 /* Returns to the system what the library's pools keep of the current device's
  * memory for reuse, for callers that need it elsewhere: up to an eighth of the
- * device, at most 16 GB, of destroyed meshes' memory, and up to 5 GiB of what calls
- * took for themselves (the device copies of host maps and grids, temporaries of mesh
- * builds, and up to 4 GiB of node values for a grid with supersampling > 1; more
- * than that goes back at the next synchronisation). */
+ * device, at most 16 GB, of destroyed meshes' memory and small scratch, and up to
+ * 5 GiB of the pieces of 32 MB and more that calls took for themselves (the device
+ * copies of host maps and grids, temporaries of mesh builds, and up to 4 GiB of node
+ * values for a grid with supersampling > 1; what is beyond goes back at the next
+ * synchronisation). */
 dtfe_status_t dtfe_trim_memory(void);
 dtfe_status_t dtfe_mesh_info(dtfe_mesh_t mesh, dtfe_mesh_info_t *info);
 dtfe_status_t dtfe_mesh_sync(dtfe_mesh_t mesh);
@@ -285,7 +286,8 @@ dtfe_status_t dtfe_batch_destroy(dtfe_batch_t batch);
  * iterations overlap on two streams.  Requests are admitted while a slot is
  * free and their map buffer plus any walk records they need fit the device
  * budget; records of idle (mesh, axis) pairs are evicted least recently used
- * first.  A request's map is the same alone and in any mix: every pixel is
+ * first.  An FP64 request that fits alone only without the links between its
+ * mesh's records is served without them, slower.  A request's map is the same alone and in any mix: every pixel is
  * formed by one block from its own samples, whatever else the launch holds. */
 typedef struct dtfe_server_s *dtfe_server_t;
 

@@ -22,10 +22,9 @@ namespace {
 // Threads per block of the FP64 maps and the blocks per SM their registers
 // allow (96 a thread).  The walk waits on FP64 latencies, so warps count more
 // than the few spills around its out-of-line step: 131k clustered points, 512^2
-// x 16, while the walk still picked each crossing's operands: 2 x 256 threads of
-// 128 registers 10.03 ms, 4 x 128 9.77, 10 x 64 of 96 9.39, 12 x 64 of 80 10.7
-// (spills in the loop).  Blocks of two warps also lose less at the end-of-tile
-// barrier than blocks of eight.
+// x 16: 8 x 64 threads 9.73 ms, 10 x 64 of 96 registers 8.80, 12 x 64 of 80 10.7
+// (spills in the loop), 5 x 128 8.86, 2 x 256 of 128 10.2; 32k uniform points,
+// 256^2 x 4: 0.610, 0.552, 0.626, 0.575 and 0.669.
 constexpr int kBlock64 = 64;
 // A pixel's samples are one block's, and take 9 B each of its shared memory.  64
 // threads fit 65 samples badly, and with thousands an SM holds few such blocks: maps

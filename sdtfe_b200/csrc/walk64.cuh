@@ -685,8 +685,8 @@ __device__ __forceinline__ bool entry_triangle64(const WalkConf64& W, const Ray6
 // reference computes it for that face of that tet (crossing64).
 //
 // What bounds it: latency, with the FP64 and the ALU pipe each near half of
-// their rate (56 % issue at 16 to 20 warps per SM; about 270 warp instructions
-// a visit, a third of them FP64).  All six products in the mesh's order, the
+// their rate (66 % issue at 19 warps per SM; about 250 warp instructions a visit,
+// a third of them FP64).  All six products in the mesh's order, the
 // face rule on their signs and each face's operands picked by its index took
 // 456, at 24 of 32 lanes.  131k clustered points, 512^2 x 16: 15.7 -> 8.8 ms;
 // 32k uniform points, 256^2 x 4: 0.864 -> 0.549 ms.  Measured and not kept: the
