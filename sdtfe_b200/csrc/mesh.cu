@@ -559,11 +559,17 @@ size_t mesh_link_bytes(const Mesh& m) {
 
 // The links, which all axes and both precisions share.  Where a walk may be running
 // on records built before, on any stream, they are not shown to it until they are
-// complete.
-static dtfe_status_t build_links(Mesh* m, bool in_use) {
+// complete.  Not required: a mesh whose links do not fit goes without.
+static dtfe_status_t build_links(Mesh* m, bool in_use, bool required) {
   uint4* link = nullptr;
   const size_t rows = kLinkRowsPerTet * (size_t)m->nt;
-  SDTFE_TRY(dmalloc_async(&link, rows, m));
+  const dtfe_status_t st = dmalloc_async(&link, rows, m);
+  if (st == DTFE_ERR_NOMEM && !required) {
+    cudaGetLastError();
+    dtfe_clear_error();
+    return DTFE_OK;
+  }
+  SDTFE_TRY(st);
   cudaError_t e = cudaSuccess;
   if (m->nt) {
     k_links<<<grid_for(4LL * m->nt), kBlock, 0, m->stream>>>(m->rows, m->nt, link);
@@ -585,8 +591,8 @@ static bool any_records(const Mesh& m) {
   return any;
 }
 
-dtfe_status_t mesh_links(Mesh* m) {
-  return m->link || !has_links(*m) ? DTFE_OK : build_links(m, any_records(*m));
+dtfe_status_t mesh_links(Mesh* m, bool required) {
+  return m->link || !has_links(*m) ? DTFE_OK : build_links(m, any_records(*m), required);
 }
 
 dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32, bool want_links) {
@@ -618,14 +624,8 @@ dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32, bool wan
     if (e != cudaSuccess)
       st = set_error(DTFE_ERR_CUDA, "walk records: %s", cudaGetErrorString(e));
   }
-  if (st == DTFE_OK && (need_links || (want_links && !m->link && has_links(*m)))) {
-    st = build_links(m, in_use);
-    if (st == DTFE_ERR_NOMEM && !need_links) {
-      cudaGetLastError();
-      dtfe_clear_error();
-      st = DTFE_OK;
-    }
-  }
+  if (st == DTFE_OK && (need_links || (want_links && !m->link && has_links(*m))))
+    st = build_links(m, in_use, need_links);
   if (st != DTFE_OK) {
     if (need64) dfree_async(A.rec64, m->nt, m);
     if (need32) dfree_async(A.geo32, 4 * (size_t)m->nt, m);

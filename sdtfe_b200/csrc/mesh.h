@@ -94,8 +94,8 @@ dtfe_status_t mesh_upload(Mesh* m, const double* particle_data, int n, const int
 dtfe_status_t mesh_density(Mesh* m);
 dtfe_status_t mesh_gradients(Mesh* m);
 dtfe_status_t mesh_records(Mesh* m, int axis, bool want64, bool want32, bool want_links);
-// the links alone, for a mesh that went without
-dtfe_status_t mesh_links(Mesh* m);
+// the links alone, for a mesh that went without (and may again, unless required)
+dtfe_status_t mesh_links(Mesh* m, bool required);
 // the mixed 3-D grid's per-tet FP64 field (k_field64), built once on the mesh stream
 dtfe_status_t mesh_field64(Mesh* m);
 void mesh_drop_records(Mesh* m, int axis);

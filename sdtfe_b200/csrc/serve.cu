@@ -227,7 +227,7 @@ dtfe_status_t admit_one(Server* S, Request* r, bool links) {
     std::lock_guard<std::mutex> lk(h->mu);
     const size_t before = record_bytes(m, r->p.axis);
     dtfe_status_t st = prepare_axis(m, r->p.axis, r->p.precision, links);
-    if (st == DTFE_OK && links) st = mesh_links(&m);
+    if (st == DTFE_OK && links) st = mesh_links(&m, r->p.precision == DTFE_MIXED);
     const size_t after = record_bytes(m, r->p.axis);
     res.bytes += after - before;
     S->in_use += after - before;

@@ -67,3 +67,38 @@ def test_requests_under_a_budget(golden, sd, room, held):
         # the mesh serves its owner as before
         for (axis, precision), w in zip(asked, want):
             assert np.array_equal(m.map(params(sd, axis, precision))[0], w)
+
+
+def test_served_without_links_when_the_device_is_full(sd):
+    """FP64 records without links, as the device has room for the records alone; a
+    request over them that a server's budget has links for is served all the same."""
+    import torch
+
+    from sdtfe_b200 import workloads
+
+    pos4, _ = workloads.clustered_box(n=200000, seed=7, n_clusters=6, r_max=0.05)
+    tetra = sd.triangulate(pos4)
+    nt, part = len(tetra), 64 << 20
+    p = params(sd, 0, sd.DTFE_FP64)
+    assert nt * LINKS > 3 * part  # more than is left beside the records
+    with sd.Mesh(pos4, tetra, 1.0) as alone, sd.Server() as srv:
+        want = alone.map(p)[0]
+        assert np.array_equal(srv.wait(srv.submit(srv.add_mesh(alone), p))[0], want)
+    with sd.Mesh(pos4, tetra, 1.0, flags=sd.MESH_LAZY) as m:
+        for axis in range(3):
+            m.hull(axis)
+        sd.trim_memory()
+        before, taken = m.info().device_bytes, []
+        try:
+            while torch.cuda.mem_get_info()[0] > nt * REC64 + 3 * part:
+                taken.append(torch.empty(part, dtype=torch.uint8, device="cuda"))
+            assert np.array_equal(m.map(p)[0], want)
+            assert m.info().device_bytes == before + nt * REC64
+            with sd.Server(device_budget=nt * (REC64 + LINKS) + part) as srv:
+                assert np.array_equal(srv.wait(srv.submit(srv.add_mesh(m), p))[0], want)
+            assert m.info().device_bytes == before + nt * REC64
+        finally:
+            taken.clear()
+            torch.cuda.empty_cache()
+        with sd.Server() as srv:  # room again: with its links
+            assert np.array_equal(srv.wait(srv.submit(srv.add_mesh(m), p))[0], want)
